@@ -28,6 +28,8 @@ struct XferLaunch {
     uint32_t nDescs;
     uint32_t totalChunks;
     uint32_t chunkShift;        // chunk size = 1 << chunkShift bytes
+    uint32_t warpChunks;        // 1: chunks are sized for warps (batchCopyWarp), 0: for CTAs
+    uint32_t uniformChunks;     // chunks per descriptor when all descriptors have the same number, else 0
     uint32_t pad;
     unsigned int *doneCounter;  // device word, zero between launches
     uint64_t *hostFlag;         // device-visible address of the pinned completion word
