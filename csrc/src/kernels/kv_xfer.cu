@@ -4,9 +4,9 @@
 
 namespace {
 
-template<bool kCast> __global__ void __launch_bounds__(nixl_kv::kKvThreads) kvXferKernel(const __grid_constant__ NixlKvXferParams p) {
-    nixl_kv::moveBlocks<kCast>(p, p.src_blocks, p.dst_blocks);
-    nixl_kv::signalWhenAllDone(p, p.done_counter);
+template<bool kCast, int kVec> __global__ void __launch_bounds__(nixl_kv::kKvThreads, 4) kvXferKernel(const __grid_constant__ nixl_kv::KvPlan k) {
+    nixl_kv::moveBlocks<kCast, kVec>(k, k.p.src_blocks, k.p.dst_blocks);
+    nixl_kv::signalWhenAllDone(k.p, k.p.done_counter);
 }
 
 } // namespace
@@ -18,9 +18,15 @@ extern "C" int nixl_kv_xfer_launch(const NixlKvXferParams *params, void *stream)
     if (const cudaError_t e = nixl_kv::checkShape(p); e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
-    const int grid = nixl_kv::gridFor(p, dev);
+    const nixl_kv::KvPlan k = nixl_kv::planFor(p);
+    const int grid = nixl_kv::gridFor(k, dev);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (p.cast_fp8) kvXferKernel<true><<<grid, nixl_kv::kKvThreads, 0, s>>>(p);
-    else kvXferKernel<false><<<grid, nixl_kv::kKvThreads, 0, s>>>(p);
+    if (p.cast_fp8) {
+        if (k.vec_bytes == 32) kvXferKernel<true, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+        else kvXferKernel<true, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+    } else {
+        if (k.vec_bytes == 32) kvXferKernel<false, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+        else kvXferKernel<false, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+    }
     return static_cast<int>(cudaGetLastError());
 }

@@ -17,10 +17,10 @@ constexpr size_t kScratchBytes = kCounterBytes + 2 * kTableBytes;
 // In host code this name is only a handle for cudaGetSymbolAddress; device code names it directly.
 static __device__ __align__(256) unsigned char g_kvScratch[kScratchBytes];
 
-template<bool kCast> __global__ void __launch_bounds__(nixl_kv::kKvThreads) kvXferStaticKernel(const __grid_constant__ NixlKvXferParams p) {
-    nixl_kv::moveBlocks<kCast>(p, reinterpret_cast<const int32_t *>(g_kvScratch + kCounterBytes),
-                               reinterpret_cast<const int32_t *>(g_kvScratch + kCounterBytes + kTableBytes));
-    nixl_kv::signalWhenAllDone(p, reinterpret_cast<unsigned int *>(g_kvScratch));
+template<bool kCast, int kVec> __global__ void __launch_bounds__(nixl_kv::kKvThreads, 4) kvXferStaticKernel(const __grid_constant__ nixl_kv::KvPlan k) {
+    nixl_kv::moveBlocks<kCast, kVec>(k, reinterpret_cast<const int32_t *>(g_kvScratch + kCounterBytes),
+                                     reinterpret_cast<const int32_t *>(g_kvScratch + kCounterBytes + kTableBytes));
+    nixl_kv::signalWhenAllDone(k.p, reinterpret_cast<unsigned int *>(g_kvScratch));
 }
 
 // Device address of g_kvScratch per GPU, looked up once per device with that device current.
@@ -78,8 +78,14 @@ extern "C" int nixl_kv_xfer_launch_static(const NixlKvXferParams *params, const 
     if ((e = cudaMemcpyAsync(scratch + kCounterBytes + kTableBytes, host_dst_blocks, bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return static_cast<int>(e);
 
-    const int grid = nixl_kv::gridFor(p, dev);
-    if (p.cast_fp8) kvXferStaticKernel<true><<<grid, nixl_kv::kKvThreads, 0, s>>>(p);
-    else kvXferStaticKernel<false><<<grid, nixl_kv::kKvThreads, 0, s>>>(p);
+    const nixl_kv::KvPlan k = nixl_kv::planFor(p);
+    const int grid = nixl_kv::gridFor(k, dev);
+    if (p.cast_fp8) {
+        if (k.vec_bytes == 32) kvXferStaticKernel<true, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+        else kvXferStaticKernel<true, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+    } else {
+        if (k.vec_bytes == 32) kvXferStaticKernel<false, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+        else kvXferStaticKernel<false, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
+    }
     return static_cast<int>(cudaGetLastError());
 }

@@ -116,3 +116,65 @@ def test_rejects_bad_arguments():
     with pytest.raises(TypeError):
         xfer.post(torch.zeros(4, device="cuda:0"), torch.zeros(4, device="cuda:0"))
     xfer.close()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize(
+    "tokens,heads,dst_heads,dim,src_order,dst_order,base",
+    [
+        (1, 1, 1, 8, "NHD", "NHD", 0),      # a block of one 16-byte vector
+        (3, 1, 2, 24, "NHD", "HND", 0),     # rows of 48 bytes: 16-byte vectors, a slot that is not full
+        (5, 3, 7, 96, "HND", "NHD", 0),     # nothing to merge, neither count a power of two
+        (16, 4, 4, 128, "NHD", "NHD", 0),   # a block is one run of bytes
+        (16, 4, 8, 64, "HND", "HND", 0),    # tokens merge, heads do not
+        (33, 2, 2, 64, "HND", "HND", 0),    # one run, not a multiple of a slot
+        (16, 2, 4, 128, "NHD", "NHD", 16),  # caches that start 16 bytes off a 32-byte boundary
+    ],
+)
+def test_block_shapes_and_alignments(fp8, tokens, heads, dst_heads, dim, src_order, dst_order, base):
+    n, pool, esize = 3, 21, 1 if fp8 else 2
+    cfg = nixl_agent_config(enable_prog_thread=False, backends=["NVLINK"])
+    tag = f"kvs{int(fp8)}_{tokens}_{heads}_{dst_heads}_{dim}_{src_order}{dst_order}{base}"
+    a, b = nixl_agent(tag + "_p", cfg), nixl_agent(tag + "_d", cfg)
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(tokens * 100 + heads)
+    src_size, dst_size = pool * tokens * heads * dim * 2, pool * tokens * dst_heads * dim * esize
+    pad = 512 + base
+    src_mem = torch.zeros(n * (src_size + pad) // 512 * 512 + 1024, dtype=torch.uint8, device=dev)
+    dst_mem = torch.full((n * (dst_size + pad) // 512 * 512 + 1024,), 7, dtype=torch.uint8, device=dev)
+
+    def views(mem, size, shape, dtype):
+        step = (size + pad - base) // 512 * 512
+        return [mem[base + i * step : base + i * step + size].view(dtype).view(shape) for i in range(n)]
+
+    def shape(order, h):
+        return (pool, tokens, h, dim) if order == "NHD" else (pool, h, tokens, dim)
+
+    src = views(src_mem, src_size, shape(src_order, heads), torch.bfloat16)
+    dst = views(dst_mem, dst_size, shape(dst_order, dst_heads), torch.uint8 if fp8 else torch.bfloat16)
+    for t in src:
+        t.copy_(torch.randn(t.shape, device=dev, generator=g))
+    a.register_memory(src_mem)
+    b.register_memory(dst_mem)
+    a.add_remote_agent(b.get_agent_metadata())
+    off = dst_heads - heads
+    xfer = KVTransfer(a, src, KVLayout(tokens, heads, dim, src_order), b.name, [(t.data_ptr(), dst_size, 0) for t in dst],
+                      KVLayout(tokens, dst_heads, dim, dst_order, esize), dst_head_offset=off, cast_fp8=fp8, scale=0.5 if fp8 else 1.0)
+    sb = torch.randperm(pool, device=dev, generator=g)[:19].int()
+    db = torch.randperm(pool, device=dev, generator=g)[:19].int()
+    want_mem = dst_mem.clone()
+    want = [want_mem[t.data_ptr() - dst_mem.data_ptr() :][:dst_size].view(t.dtype).view(t.shape) for t in dst]
+    for s, w in zip(src, want):
+        picked = s[sb.long()]
+        if src_order != dst_order:
+            picked = picked.transpose(1, 2)
+        if fp8:
+            picked = (picked.float() * 0.5).to(torch.float8_e4m3fn).view(torch.uint8)
+        if dst_order == "NHD":
+            w[db.long(), :, off:] = picked
+        else:
+            w[db.long(), off:] = picked
+    xfer.wait(xfer.post(sb, db))
+    torch.cuda.synchronize()
+    assert torch.equal(dst_mem, want_mem)  # and nothing outside the blocks was touched
+    xfer.close()
