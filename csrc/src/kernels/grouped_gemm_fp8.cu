@@ -291,9 +291,9 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             const long long grow = static_cast<long long>(sh.rowStart[t.g]) + local_row;
             const float *sa_row = scale_a + grow * k_steps;
             const float *sw = p.scale_w + (static_cast<long long>(t.g) * n_tiles + t.nt) * k_steps;
-            float acc[HN];
+            uint64_t acc[2][16]; // fp32 pairs
 #pragma unroll
-            for (int i = 0; i < HN; ++i) acc[i] = 0.f;
+            for (int i = 0; i < 16; ++i) acc[0][i] = acc[1][i] = 0;
             bool ok = true;
             // The scales of a step are needed by every FMA of that step, so their loads must not sit on
             // the critical path: a register ring keeps them kPrefetch steps ahead.  They are kept as
@@ -333,10 +333,8 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                     tcFenceBefore();
                     __syncwarp();
                     if (lane == 0) mbarArrive(&sh.tmemEmpty[buf]);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) acc[i] = fmaf(v0[i], s, acc[i]);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) acc[32 + i] = fmaf(v1[i], s, acc[32 + i]);
+                    fmaScale32(acc[0], v0, pack2(s, s));
+                    fmaScale32(acc[1], v1, pack2(s, s));
                     ++it;
                 }
             }
@@ -347,7 +345,10 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 const long long first_grow = static_cast<long long>(sh.rowStart[t.g]) + first_row;
                 const int rows_left = sh.rowCount[t.g] - first_row;
                 __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + first_grow * p.N + t.nt * BN + half * HN + (lane & 7) * 8;
-                storeRows64(reinterpret_cast<const float(&)[32]>(acc[0]), reinterpret_cast<const float(&)[32]>(acc[32]), out, p.N, rows_left, lane);
+                float lo[32], hi[32];
+                unpack32(acc[0], lo);
+                unpack32(acc[1], hi);
+                storeRows64(lo, hi, out, p.N, rows_left, lane);
             }
         }
     }
@@ -406,23 +407,29 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
         std::fprintf(stderr, "nixl_grouped_gemm_fp8_launch: cuTensorMapEncodeTiled failed\n");
         return cudaErrorInvalidValue;
     }
-    // Tile shape: CTA pairs with 256 x 256 tiles when rows per expert are plentiful (compact layout
-    // of a throughput dispatch), single CTAs with 128 x 128 tiles for the expert-major low-latency
-    // layout, where most tiles hold a handful of rows.
+    // Tile shape: CTA pairs with 256 x 256 tiles when the experts have more rows than one 128-row tile on average and the
+    // tiles are enough for the 74 pairs; single CTAs with 128 x 128 tiles otherwise (the expert-major low-latency layout,
+    // where most tiles hold a handful of rows, and small products, which need every SM).  Measured, single / pair, us:
+    // 32 experts, N = K = 4096: 128 rows each 118 / 122, 200 rows 212 / 162, 512 rows 477 / 310; 16 experts, 512 x 2048:
+    // 256 rows (32 pair tiles) 14.8 / 18.7, 400 rows (50) 22.8 / 19.0; 1 expert, 4096 x 7168, 512 rows (32) 27.5 / 35.1.
     int mode = p.tile_mode & 0xff;
-    if (mode == 0) mode = (p.rows_per_expert == 0 && !p.counts_flag && p.N % 256 == 0 && p.a_rows >= 256LL * p.groups) ? 2 : 1;
+    if (mode == 0)
+        mode = (p.rows_per_expert == 0 && !p.counts_flag && p.N % 256 == 0 && p.a_rows > 128LL * p.groups &&
+                static_cast<long long>(p.a_rows) * p.N >= 40LL * 256 * 256)
+            ? 2
+            : 1;
     if (mode == 3) {
         if (p.N % 256 || p.K % 512 || p.counts_flag || p.disp_flag) return cudaErrorInvalidValue;
         if ((reinterpret_cast<uintptr_t>(p.scale_a) | reinterpret_cast<uintptr_t>(p.scale_w)) & 3) return cudaErrorInvalidValue;
-        CUtensorMap mapW64;
-        if (!nixl_gemm::makeTileMap(&mapW64, p.w, static_cast<uint64_t>(p.groups) * p.N, static_cast<uint64_t>(p.K), 64)) return cudaErrorInvalidValue;
-        return nixl_gemm::launchMxPairKernel(mapA, mapW64, p, static_cast<cudaStream_t>(stream));
+        CUtensorMap mapT; // that kernel loads token rows in boxes of 32
+        if (!nixl_gemm::makeTileMap(&mapT, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 32)) return cudaErrorInvalidValue;
+        return nixl_gemm::launchMxPairKernel(mapT, mapW, p, static_cast<cudaStream_t>(stream));
     }
     if (mode == 2) {
         if (p.N % 256) return cudaErrorInvalidValue;
-        CUtensorMap mapW64; // the pair kernel loads W in 64-row boxes
-        if (!nixl_gemm::makeTileMap(&mapW64, p.w, static_cast<uint64_t>(p.groups) * p.N, static_cast<uint64_t>(p.K), 64)) return cudaErrorInvalidValue;
-        return nixl_gemm::launchPairKernel(mapA, mapW64, p, static_cast<cudaStream_t>(stream));
+        CUtensorMap mapA64; // that kernel loads A in boxes of 64 rows
+        if (!nixl_gemm::makeTileMap(&mapA64, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 64)) return cudaErrorInvalidValue;
+        return nixl_gemm::launchPairKernel(mapA64, mapW, p, static_cast<cudaStream_t>(stream));
     }
     const size_t smem = size_t(kStages) * kStageBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;

@@ -3,16 +3,15 @@
 // Same math and operand formats as grouped_gemm_fp8.cu.  Two CTAs of a cluster share one tile:
 // each loads its own 128 rows of A and 128 of the tile's 256 W rows per 128-channel step (32 KiB
 // per CTA and step: half the L2 -> shared-memory traffic per MAC of 128 x 128 tiles), the even CTA
-// issues M256 N128 K32 MMAs that read both CTAs' shared memory and write both CTAs' TMEM, and each
+// issues M256 N256 K32 MMAs that read both CTAs' shared memory and write both CTAs' TMEM, and each
 // CTA promotes and stores its own 128 rows.
 //
-// A 128-channel step is eight MMAs: four into one 128-column TMEM slot for the left half of the
-// tile's columns and four into a second slot for the right half; two steps (four slots, all of
-// TMEM) are in flight.  To make the two N = 128 instruction groups cover contiguous columns, CTA c
-// keeps W rows [64c, 64c+64) of the left half and of the right half (two 64-row TMA boxes).
+// A 128-channel step is four MMAs into two neighbouring 128-column TMEM slots; two steps (four slots,
+// all of TMEM) are in flight.  (Eight N = 128 instructions, one per slot, read A from shared memory twice and
+// were slower by an eighth.)  A tile with at most 128 rows left runs as M = 128 (tailTile).
 //
-// What bounds this kernel is not the tensor pipe (eight MMAs take 512 cycles) but the hand-offs
-// around it, so they are kept to a minimum:
+// What bounds this kernel is partly power (the SM clock falls from 1.7 to 1.45 GHz under load) and otherwise not
+// the tensor pipe (four MMAs take 512 cycles, a step about 940) but promotion and the hand-offs around it:
 //  * the issuing thread polls one barrier per step.  full[s] collects the producer's arrival (with
 //    both CTAs' byte count) and one arrival from each of the pair's sixteen promotion warps, sent
 //    when the warp has read the two slots the step will overwrite;
@@ -20,8 +19,14 @@
 //    in front of the MMAs delayed them by a few hundred cycles each;
 //  * promotion warps poll once per step too (one commit covers both slots), arrive with relaxed
 //    semantics (a cluster-scope release cost several hundred cycles per arrive) and fetch their
-//    scales behind the arrive;
+//    scales behind the arrive; they add with packed fp32 FMAs, half the instructions;
 //  * ring positions are counters, not divisions, on the single-thread roles.
+// (With W on the M side and tokens on the N side no rows are padded at all, but a token's scale then belongs to a register:
+// reading the scales from shared memory, 4 bytes per lane and FMA, made a step twice as long.)
+//
+// Measured on one B200, back to back for half a second (that is, under the power cap), before / now: 31 experts that share
+// 16384 rows unevenly, 2048 x 7168: 423 / 351 us (1.37 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 844 / 718 us
+// (1.53 PFLOP/s); one expert, 8192 rows, 4096 x 7168: 311 / 266 us (1.81 PFLOP/s).
 //
 //   warp 0      TMA producer (both CTAs; completion bytes are counted on the even CTA's barrier)
 //   warp 1      MMA issuer (even CTA only); commits are multicast to both CTAs' barriers
@@ -49,14 +54,13 @@ using nixl_gemm::kMaxGroups;
 
 constexpr int BM = 128;        // rows per CTA (256 per pair)
 constexpr int BN = 256;        // tile columns
-constexpr int BNS = 128;       // columns per half-step / TMEM slot
-constexpr int WBOX = 64;       // W rows per TMA box (per CTA and column half)
+constexpr int BNS = 128;       // columns per TMEM slot: a step's accumulator is two neighbouring slots
+constexpr int WROWS = 128;     // W rows each CTA keeps: the pair's MMA reads N = 256 rows, half from either CTA
 constexpr int BK = 128;
 constexpr int kStages = 6;
 constexpr int kThreads = 384;
 constexpr int kATileBytes = BM * BK;           // 16 KiB
-constexpr int kWBoxBytes = WBOX * BK;          // 8 KiB
-constexpr int kStageBytes = kATileBytes + 2 * kWBoxBytes; // 32 KiB per CTA
+constexpr int kStageBytes = kATileBytes + WROWS * BK; // 32 KiB per CTA
 constexpr int kSlots = 4;
 constexpr int kTmemCols = kSlots * BNS;        // 512
 constexpr int kPromoWarps = 8;
@@ -103,46 +107,37 @@ __device__ __forceinline__ void tmaLoad2dPair(void *smem_dst, const CUtensorMap 
                  "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y)
                  : "memory");
 }
-// A whole 128-channel step of the issuer as one instruction sequence: eight MMAs (four per TMEM
-// slot), the two commits, and then a non-blocking test of the next step's barrier.  Barrier
-// instructions placed in front of the MMAs delayed them by a few hundred cycles each, so the only
-// poll of a step sits behind its MMAs, where the tensor pipe still has work queued.
-__device__ __forceinline__ void issueKStep(uint32_t tmem_d0, uint32_t tmem_d1, uint64_t da, uint64_t dw0, uint64_t dw1, uint32_t idesc,
-                                           uint32_t bar_tmem_full, uint32_t bar_stage_empty, uint32_t peek_bar, uint32_t peek_par,
-                                           uint32_t &ready_next) {
-    uint64_t da2 = da;
+// A whole 128-channel step of the issuer as one instruction sequence: four MMAs, two commits, and then a
+// non-blocking test of the next step's barrier.  Barrier instructions placed in front of the MMAs
+// delayed them by a few hundred cycles each, so the only poll of a step sits behind its MMAs, where
+// the tensor pipe still has work queued.
+__device__ __forceinline__ void issueKStep(uint32_t tmem_d, uint64_t da, uint64_t dw, uint32_t idesc, uint32_t bar_tmem_full, uint32_t bar_stage_empty,
+                                           uint32_t peek_bar, uint32_t peek_par, uint32_t &ready_next) {
     asm volatile(
         "{\n"
         " .reg .pred pf, pacc, pnew;\n"
-        " setp.ne.b32 pacc, %12, 0;\n"
-        " setp.eq.b32 pnew, %12, 0;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %3, %4, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pnew;\n"
-        " add.u64 %3, %3, 2;\n add.u64 %4, %4, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %3, %4, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " add.u64 %3, %3, 2;\n add.u64 %4, %4, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %3, %4, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " add.u64 %3, %3, 2;\n add.u64 %4, %4, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %3, %4, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%2], %6, %5, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pnew;\n"
-        " add.u64 %6, %6, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%2], %6, %5, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " add.u64 %6, %6, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%2], %6, %5, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " add.u64 %6, %6, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%2], %6, %5, %7, {%13, %13, %13, %13, %13, %13, %13, %13}, pacc;\n"
-        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%8], %14;\n"
-        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%9], %14;\n"
-        " mbarrier.test_wait.parity.shared::cta.b64 pf, [%10], %11;\n"
+        " setp.ne.b32 pacc, %9, 0;\n"
+        " setp.eq.b32 pnew, %9, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %2, %3, %4, {%10, %10, %10, %10, %10, %10, %10, %10}, pnew;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %2, %3, %4, {%10, %10, %10, %10, %10, %10, %10, %10}, pacc;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %2, %3, %4, {%10, %10, %10, %10, %10, %10, %10, %10}, pacc;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%1], %2, %3, %4, {%10, %10, %10, %10, %10, %10, %10, %10}, pacc;\n"
+        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], %11;\n"
+        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%6], %11;\n"
+        " mbarrier.test_wait.parity.shared::cta.b64 pf, [%7], %8;\n"
         " selp.u32 %0, 1, 0, pf;\n"
         "}\n"
-        : "=r"(ready_next), "+r"(tmem_d0), "+r"(tmem_d1), "+l"(da), "+l"(dw0), "+l"(dw1), "+l"(da2)
+        : "=r"(ready_next), "+r"(tmem_d), "+l"(da), "+l"(dw)
         : "r"(idesc), "r"(bar_tmem_full), "r"(bar_stage_empty), "r"(peek_bar), "r"(peek_par), "r"(1u), "r"(0u), "h"(static_cast<uint16_t>(3))
         : "memory");
 }
 
-// D fp32, A and B e4m3, both K-major, M = 256 (both CTAs), N = 128.
-__device__ __forceinline__ constexpr uint32_t instrDescPair() {
-    return (1u << 4) | (static_cast<uint32_t>(BNS >> 3) << 17) | (static_cast<uint32_t>((2 * BM) >> 4) << 24);
+// D fp32, A and B e4m3, both K-major, M = m (256 or 128 rows of both CTAs together), N = 256.
+__device__ __forceinline__ constexpr uint32_t instrDescPair(int m) {
+    return (1u << 4) | (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 struct Tile {
@@ -160,6 +155,84 @@ __device__ __forceinline__ bool tileAt(const Shared &sh, int groups, int n_tiles
     out.g = lo;
     out.mt = local / n_tiles;
     out.nt = local - out.mt * n_tiles;
+    return true;
+}
+
+// A tile with at most 128 rows left runs as M = 128: 64 rows per CTA, and each CTA's TMEM lanes 0 - 63 hold their columns
+// [0, 128) of the tile, lanes 64 - 127 the same rows' columns [128, 256).  Half the MMA time, half the promotion and half the
+// A traffic of a tile whose second 128 rows would be padding.
+__device__ __forceinline__ bool tailTile(const Shared &sh, const Tile &t) { return sh.rowCount[t.g] - t.mt * (2 * BM) <= BM; }
+
+// Promotion of one tile: every step's sums leave TMEM, are scaled and added up in registers; then the tile is stored.  kTail: see
+// tailTile (64 of 128 columns per thread; a loop of its own, as conditions in the full tile's loop made the compiler spill there).
+// False when another role gave up.
+template<bool kTail>
+__device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, bool valid, const float *sw0, int k_steps, uint32_t lane_base, uint32_t full0, int lane,
+                                            uint32_t &it, uint32_t &s2, bool &rdy, __nv_bfloat16 *out, long long row_stride, int rows_left) {
+    volatile int *abort_flag = &sh.abort;
+    constexpr int kBlocks = kTail ? 2 : 4; // of 32 columns
+    const float *sw1 = kTail ? sw0 : sw0 + k_steps;
+    uint64_t acc[kBlocks][16]; // fp32 pairs: left half's 64 columns, right half's
+#pragma unroll
+    for (int j = 0; j < kBlocks; ++j)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[j][i] = 0;
+    // Scales are fetched two steps ahead and kept as loaded: multiplying them right away would make the warp
+    // wait for the loads it has just issued.  (A loop unrolled over a ring of four made the compiler spill.)
+    float a0 = valid ? __ldg(sa_row) : 0.f, w00 = __ldg(sw0), w10 = __ldg(sw1);
+    float a1 = valid && k_steps > 1 ? __ldg(sa_row + 1) : 0.f, w01 = k_steps > 1 ? __ldg(sw0 + 1) : 0.f, w11 = k_steps > 1 ? __ldg(sw1 + 1) : 0.f;
+#pragma unroll 1
+    for (int ks = 0; ks < k_steps; ++ks, ++it) {
+        const float s0 = a0 * w00, s1 = a0 * w10;
+        const uint64_t s00 = pack2(s0, s0), s11 = pack2(s1, s1);
+        a0 = a1;
+        w00 = w01;
+        w10 = w11;
+        const int nxt = ks + 2;
+        const uint32_t kp = it & 1u, sl = kp * 2u;
+        if (!rdy && !mbarWait(&sh.tmemFull[kp], (it >> 1) & 1, abort_flag)) return false;
+        tcFenceAfter();
+        float v0[32], v1[32];
+        tmemLoad32(lane_base + sl * BNS, v0);
+        tmemLoad32(lane_base + sl * BNS + 32, v1);
+        tmemLoadWait(v0);
+        tmemLoadWait(v1);
+        if constexpr (!kTail) {
+            fmaScale32(acc[0], v0, s00);
+            tmemLoad32(lane_base + (sl + 1) * BNS, v0); // second slot's loads run behind the first slot's FMAs
+            fmaScale32(acc[1], v1, s00);
+            tmemLoad32(lane_base + (sl + 1) * BNS + 32, v1);
+        }
+        // While those are in flight, look at the next step's barrier.
+        rdy = mbarTest(&sh.tmemFull[kp ^ 1u], ((it + 1) >> 1) & 1);
+        if constexpr (!kTail) {
+            tmemLoadWait(v0);
+            tmemLoadWait(v1);
+        }
+        // This step's slots are in registers: tell the step that reuses them.
+        tcFenceBefore();
+        __syncwarp();
+        if (lane == 0) mbarArriveCluster(full0 + s2 * 8u);
+        if (++s2 == kStages) s2 = 0;
+        // The scale prefetch goes behind the arrive (loads issued before it would hold it up).
+        if (nxt < k_steps) {
+            a1 = valid ? __ldg(sa_row + nxt) : 0.f;
+            w01 = __ldg(sw0 + nxt);
+            if (!kTail) w11 = __ldg(sw1 + nxt);
+        }
+        fmaScale32(acc[kBlocks - 2], v0, kTail ? s00 : s11);
+        fmaScale32(acc[kBlocks - 1], v1, kTail ? s00 : s11);
+    }
+    // Coalesced stores: see storeRows64.
+    float lo[32], hi[32];
+    unpack32(acc[0], lo);
+    unpack32(acc[1], hi);
+    storeRows64(lo, hi, out, row_stride, rows_left, lane);
+    if constexpr (!kTail) {
+        unpack32(acc[2], lo);
+        unpack32(acc[3], hi);
+        storeRows64(lo, hi, out + BNS, row_stride, rows_left, lane);
+    }
     return true;
 }
 
@@ -233,13 +306,6 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     tcFenceAfter();
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
-    // k-steps this pair executes in total (every tile has k_steps of them)
-    int my_tiles = 0;
-    {
-        const int total = sh.tilePrefix[p.groups];
-        if (pair < total) my_tiles = (total - pair + pairs - 1) / pairs;
-    }
-
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp == 0 && lane == 0) {
@@ -248,9 +314,12 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
             uint32_t it = 0;
             Tile t;
             for (int ti = pair; tileAt(sh, p.groups, n_tiles, ti, t); ti += pairs) {
-                const int row0 = sh.rowStart[t.g] + t.mt * (2 * BM) + static_cast<int>(cta) * BM;
+                const int rows_cta = tailTile(sh, t) ? BM / 2 : BM;
+                const int lo = t.mt * (2 * BM) + static_cast<int>(cta) * rows_cta;
+                const int row0 = sh.rowStart[t.g] + lo;
+                const uint32_t bytes = static_cast<uint32_t>(2 * (rows_cta + WROWS) * BK); // both CTAs' shares
                 if (p.disp_flag) {
-                    const int lo = t.mt * (2 * BM) + static_cast<int>(cta) * BM, hi = min(lo + BM, sh.rowCount[t.g]);
+                    const int hi = min(lo + rows_cta, sh.rowCount[t.g]);
                     int first = 0;
                     for (int r = 0; r < p.ranks; ++r) {
                         const int c = p.counts[static_cast<long long>(r) * p.experts_total + p.expert_base + t.g];
@@ -273,43 +342,44 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
                     }
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
-                const int wrow = t.g * p.N + t.nt * BN + static_cast<int>(cta) * WBOX;
+                const int wrow = t.g * p.N + t.nt * BN + static_cast<int>(cta) * WROWS;
                 for (int ks = 0; ks < k_steps; ++ks, ++it) {
                     const int s = it % kStages;
                     if (!mbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, abort_flag)) goto role_done;
-                    if (cta == 0) mbarExpectTx(&sh.full[s], 2 * kStageBytes); // both CTAs' shares
+                    if (cta == 0) mbarExpectTx(&sh.full[s], bytes);
                     const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
                     unsigned char *st = tiles + s * kStageBytes;
                     tmaLoad2dPair(st, &mapA, ks * BK, row0, bar);
-                    tmaLoad2dPair(st + kATileBytes, &mapW, ks * BK, wrow, bar);               // columns [64c, 64c+64) of the left half
-                    tmaLoad2dPair(st + kATileBytes + kWBoxBytes, &mapW, ks * BK, wrow + BNS, bar); // and of the right half
+                    if (rows_cta == BM) tmaLoad2dPair(st + kATileBytes / 2, &mapA, ks * BK, row0 + BM / 2, bar);
+                    tmaLoad2dPair(st + kATileBytes, &mapW, ks * BK, wrow, bar);
                 }
             }
         } else if (warp == 1 && lane == 0 && cta == 0) {
             // ------------------------------------------------------------ MMA issuer (even CTA)
             // One poll per eight MMAs: full[s] completes when both CTAs' bytes have landed and all
             // promotion warps of the pair have read the step's two TMEM slots.
-            const uint32_t ksteps_total = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(k_steps);
             uint32_t s = 0, full_par = 0, sl = 0; // ring positions as counters: no divisions on this thread
             uint32_t ready = 0;
             const uint32_t full_bar0 = smemU32(&sh.full[0]), empty_bar0 = smemU32(&sh.empty[0]), tfull_bar0 = smemU32(&sh.tmemFull[0]);
             const uint64_t desc0 = smemDesc(smemU32(tiles));
-            for (uint32_t it = 0; it < ksteps_total; ++it) {
-                if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) goto role_done;
-                tcFenceAfter();
-                uint32_t ns = s + 1, nfull_par = full_par;
-                if (ns == kStages) {
-                    ns = 0;
-                    nfull_par ^= 1u;
+            Tile t;
+            for (int ti = pair; tileAt(sh, p.groups, n_tiles, ti, t); ti += pairs) {
+                const uint32_t idesc = instrDescPair(tailTile(sh, t) ? BM : 2 * BM);
+                for (int ks = 0; ks < k_steps; ++ks) {
+                    if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) goto role_done;
+                    tcFenceAfter();
+                    uint32_t ns = s + 1, nfull_par = full_par;
+                    if (ns == kStages) {
+                        ns = 0;
+                        nfull_par ^= 1u;
+                    }
+                    const uint64_t da = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
+                    const uint64_t dw = da + static_cast<uint64_t>(kATileBytes >> 4);
+                    issueKStep(tmem + sl * BNS, da, dw, idesc, tfull_bar0 + (sl >> 1) * 8u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
+                    sl ^= 2u;
+                    s = ns;
+                    full_par = nfull_par;
                 }
-                const uint64_t da = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
-                const uint64_t dw0 = da + static_cast<uint64_t>(kATileBytes >> 4);
-                const uint64_t dw1 = da + static_cast<uint64_t>((kATileBytes + kWBoxBytes) >> 4);
-                issueKStep(tmem + sl * BNS, tmem + (sl + 1) * BNS, da, dw0, dw1, instrDescPair(), tfull_bar0 + (sl >> 1) * 8u, empty_bar0 + s * 8u,
-                           full_bar0 + ns * 8u, nfull_par, ready);
-                sl ^= 2u;
-                s = ns;
-                full_par = nfull_par;
             }
         }
     role_done:;
@@ -318,7 +388,6 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
         // ---------------------------------------------------------------- promotion + epilogue
         const int q = warp & 3;
         const int part = (warp - 4) >> 2; // which 64 of a slot's 128 columns
-        const int row_in_tile = q * 32 + lane;
         const uint32_t full0 = mapToCta(smemU32(&sh.full[0]), 0);
         const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16) + part * 64;
         uint32_t it = 0;      // step counter, same numbering as the issuer's
@@ -328,80 +397,20 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
         bool rdy = false;
         bool ok = true;
         for (int ti = pair; ok && tileAt(sh, p.groups, n_tiles, ti, t); ti += pairs) {
-            const int local_row = t.mt * (2 * BM) + static_cast<int>(cta) * BM + row_in_tile;
+            const bool tail = tailTile(sh, t);
+            // Full tile: one row, 64 columns of either half.  Tail: one of 64 rows, 64 columns of half q / 2.
+            const int first_row = t.mt * (2 * BM) + (tail ? static_cast<int>(cta) * (BM / 2) + (q & 1) * 32 : static_cast<int>(cta) * BM + q * 32);
+            const int local_row = first_row + lane;
             const bool valid = local_row < sh.rowCount[t.g];
             const long long grow = static_cast<long long>(sh.rowStart[t.g]) + local_row;
             const float *sa_row = p.scale_a + grow * k_steps;
-            const float *sw0 = p.scale_w + (static_cast<long long>(t.g) * n_blocks + t.nt * 2) * k_steps;
-            const float *sw1 = sw0 + k_steps;
-            float acc[2 * 64];
-#pragma unroll
-            for (int i = 0; i < 2 * 64; ++i) acc[i] = 0.f;
-            // Scales are fetched kPrefetch steps ahead and kept as loaded: multiplying them right away
-            // would make the warp wait for the loads it has just issued.
-            constexpr int kPrefetch = 4;
-            float ring_a[kPrefetch], ring_w0[kPrefetch], ring_w1[kPrefetch];
-#pragma unroll
-            for (int i = 0; i < kPrefetch; ++i) {
-                ring_a[i] = (i < k_steps && valid) ? __ldg(sa_row + i) : 0.f;
-                ring_w0[i] = i < k_steps ? __ldg(sw0 + i) : 0.f;
-                ring_w1[i] = i < k_steps ? __ldg(sw1 + i) : 0.f;
-            }
-            for (int ks0 = 0; ks0 < k_steps && ok; ks0 += kPrefetch) {
-#pragma unroll
-                for (int i = 0; i < kPrefetch; ++i, ++it) {
-                    const int ks = ks0 + i;
-                    if (ks >= k_steps) break;
-                    const float s0 = ring_a[i] * ring_w0[i], s1 = ring_a[i] * ring_w1[i];
-                    const int nxt = ks + kPrefetch;
-                    const uint32_t kp = it & 1u, sl = kp * 2u;
-                    if (!rdy && !mbarWait(&sh.tmemFull[kp], (it >> 1) & 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tcFenceAfter();
-                    float v0[32], v1[32];
-                    tmemLoad32(lane_base + sl * BNS, v0);
-                    tmemLoad32(lane_base + sl * BNS + 32, v1);
-                    tmemLoadWait(v0);
-                    tmemLoadWait(v1);
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[e] = fmaf(v0[e], s0, acc[e]);
-                    tmemLoad32(lane_base + (sl + 1) * BNS, v0); // second slot's loads run behind the first slot's FMAs
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[32 + e] = fmaf(v1[e], s0, acc[32 + e]);
-                    tmemLoad32(lane_base + (sl + 1) * BNS + 32, v1);
-                    // While those are in flight, look at the next step's barrier.
-                    rdy = mbarTest(&sh.tmemFull[kp ^ 1u], ((it + 1) >> 1) & 1);
-                    tmemLoadWait(v0);
-                    tmemLoadWait(v1);
-                    // Both slots of this step are in registers: tell the step that reuses them.
-                    tcFenceBefore();
-                    __syncwarp();
-                    if (lane == 0) mbarArriveCluster(full0 + s2 * 8u);
-                    if (++s2 == kStages) s2 = 0;
-                    // The scale prefetch goes behind the arrive (loads issued before it would hold it up).
-                    if (nxt < k_steps) {
-                        ring_a[i] = valid ? __ldg(sa_row + nxt) : 0.f;
-                        ring_w0[i] = __ldg(sw0 + nxt);
-                        ring_w1[i] = __ldg(sw1 + nxt);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[64 + e] = fmaf(v0[e], s1, acc[64 + e]);
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) acc[96 + e] = fmaf(v1[e], s1, acc[96 + e]);
-                }
-            }
-            if (!ok) break;
-            {
-                // Coalesced stores: see storeRows64.  acc[h * 64 ..] are this row's 64 columns of half h.
-                const int first_row = t.mt * (2 * BM) + static_cast<int>(cta) * BM + q * 32 + (lane & ~7);
-                const long long first_grow = static_cast<long long>(sh.rowStart[t.g]) + first_row;
-                const int rows_left = sh.rowCount[t.g] - first_row;
-                __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + first_grow * p.N + t.nt * BN + part * 64 + (lane & 7) * 8;
-                storeRows64(reinterpret_cast<const float(&)[32]>(acc[0]), reinterpret_cast<const float(&)[32]>(acc[32]), out, p.N, rows_left, lane);
-                storeRows64(reinterpret_cast<const float(&)[32]>(acc[64]), reinterpret_cast<const float(&)[32]>(acc[96]), out + BNS, p.N, rows_left, lane);
-            }
+            const float *sw0 = p.scale_w + (static_cast<long long>(t.g) * n_blocks + t.nt * 2 + (tail ? q >> 1 : 0)) * k_steps;
+            const int row8 = first_row + (lane & ~7);
+            const int rows_left = sh.rowCount[t.g] - row8;
+            __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + (static_cast<long long>(sh.rowStart[t.g]) + row8) * p.N + t.nt * BN +
+                (tail ? (q >> 1) * BNS : 0) + part * 64 + (lane & 7) * 8;
+            ok = tail ? promoteTile<true>(sh, sa_row, valid, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left)
+                      : promoteTile<false>(sh, sa_row, valid, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left);
         }
     }
 

@@ -11,18 +11,32 @@
 // scale factors ride along with the MMA: a whole K loop accumulates in TMEM and the epilogue runs
 // once per tile.
 //
+// The roles of the operands are swapped: W is the MMA's M side (256 weight rows per pair, 128 per CTA) and the tokens
+// are its N side.  N may be any multiple of 32, so an expert's rows are split into equal tiles of at most 256 tokens,
+// rounded up to 32, and almost nothing is computed, loaded or kept in TMEM for padding; with the tokens on the M side every
+// expert's last tile cost 256 rows.  The accumulator is transposed (a lane is a column of D, a TMEM column a token), which
+// the epilogue undoes with shuffles between neighbouring lanes (storeCols32).
+//
 // Scale factors reach the tensor core through TMEM.  For four steps at a time ("chunk") the
-// epilogue warps, idle during the main loop, build in shared memory the 512-byte layout the
-// hardware wants (byte (r % 32) * 16 + (r / 32) * 4 + step for row r: for A one 32-bit word per row
-// straight from the scale tensor, for W the block's word repeated for all 128 columns), the issuing
-// thread copies it to TMEM with tcgen05.cp (32x128b.warpx4) and selects the step's byte with the
-// scale-factor-id fields of the instruction descriptor.  Shared-memory chunk buffers form a ring of
-// four, TMEM scale columns are double-buffered by chunk parity.
+// epilogue warps, idle during the main loop, build in shared memory the 512-byte layouts the
+// hardware wants (byte (r % 32) * 16 + (r / 32) * 4 + step for row r: for the tokens one 32-bit word per row
+// straight from the scale tensor, for W the block's word repeated for all 128 rows), the issuing
+// thread copies them to TMEM with tcgen05.cp (32x128b.warpx4) and selects the step's byte with the
+// scale-factor-id fields of the instruction descriptor.  The copies run in the MMAs' pipe, and each run of them is a
+// bubble there; up to eight chunks (4096 channels) are therefore copied at once.  Both the shared-memory buffers and
+// the TMEM scale columns are double-buffered by such groups.
 //
 //   warp 0      TMA producer (both CTAs; bytes counted on the even CTA's barrier)
-//   warp 1      MMA issuer (even CTA): tcgen05.cp of scale chunks, eight M256 N128 K32 MMAs per step
-//   warp 2      TMEM allocator (512 columns: 256 accumulator, 32 scale factors)
+//   warps 1, 3  MMA issuers (even CTA): tcgen05.cp of scale groups, four M256 K32 MMAs per step
+//   warp 2      TMEM allocator (512 columns: 256 accumulator, 192 scale factors)
 //   warps 4-11  scale staging during the main loop, then the epilogue (TMEM -> bf16 -> global)
+//
+// Bound by power: the SM clock is 1.55 GHz at the first launch and 1.25 to 1.4 GHz after half a second; a full step takes
+// 697 cycles of which the MMAs need 512.  What is left is mostly the traffic into shared memory (64 of 128 bytes per cycle
+// at full rate, beside the operands' reads).  Measured on one B200 back to back for half a second, before (tokens on the
+// M side, eight N = 128 MMAs per step, scale copies every 512 channels) / now: 31 experts that share 16384 rows unevenly,
+// 2048 x 7168: 335 / 278 us (1.73 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 659 / 573 us (1.92 PFLOP/s); one
+// expert, 8192 rows, 4096 x 7168: 239 / 209 us (2.30 PFLOP/s); 32 experts, 1024 rows, 2048 x 7168: 130 / 97 us.
 //
 // TMA loads read this GPU's memory only and carry no cluster multicast.  Every wait is bounded.
 #include <cuda.h>
@@ -38,30 +52,32 @@ using namespace nixl_tc;
 using nixl_gemm::GEMM_ERR_TIMEOUT;
 using nixl_gemm::kMaxGroups;
 
-constexpr int BM = 128;        // rows per CTA (256 per pair)
-constexpr int BN = 256;        // tile columns
-constexpr int BNS = 128;       // columns per instruction group / accumulator half
-constexpr int WBOX = 64;       // W rows per TMA box (per CTA and column half)
+constexpr int BW = 128;        // W rows per CTA (256 per pair): the MMA's M side
+constexpr int BT = 256;        // tokens per tile at most: its N side, half of them from either CTA
+constexpr int TBOX = 32;       // token rows per TMA box
 constexpr int BK = 128;
 constexpr int kStages = 6;
 constexpr int kThreads = 384;
-constexpr int kATileBytes = BM * BK;
-constexpr int kWBoxBytes = WBOX * BK;
-constexpr int kStageBytes = kATileBytes + 2 * kWBoxBytes; // 32 KiB per CTA
+constexpr int kWTileBytes = BW * BK;
+constexpr int kTBoxBytes = TBOX * BK;
+constexpr int kStageBytes = kWTileBytes + BT / 2 * BK; // 32 KiB per CTA
 constexpr int kChunkSteps = 4;                 // steps whose scale bytes share one 32-bit word
-constexpr int kSfRing = 4;                     // chunk buffers in shared memory
+constexpr int kGroupChunks = 8;                // chunks copied to TMEM in one go
 constexpr int kSfAtomBytes = 512;              // 128 rows x 4 steps
-constexpr int kSfBufBytes = 3 * kSfAtomBytes;  // A, W left half, W right half
+constexpr int kSfChunkBytes = 3 * kSfAtomBytes;  // tokens 0 .. 127, tokens 128 .. 255, W
+constexpr int kSfBufBytes = kGroupChunks * kSfChunkBytes;
 constexpr int kTmemCols = 512;
-constexpr int kAccCols = 2 * BNS;              // accumulator: columns [0, 256)
-constexpr int kSfTmemStride = 16;              // scale columns of a chunk parity: [256 + 16 p, ...): A +0, W left +4, W right +8
+constexpr int kAccCols = BT;                   // accumulator: columns [0, 256)
+constexpr int kSfTmemChunk = 12;               // scale columns of a chunk: tokens +0 .. +7, W +8 .. +11
+constexpr int kSfTmemStride = kGroupChunks * kSfTmemChunk; // of a group; group g uses [256 + 96 (g % 2), ...)
 constexpr int kPromoWarps = 8;
+static_assert(kAccCols + 2 * kSfTmemStride <= kTmemCols, "accumulator and scale columns share TMEM");
 
 struct Shared {
     uint64_t full[kStages];      // even CTA: both CTAs' operand bytes of a stage have landed
     uint64_t empty[kStages];     // per CTA: the MMAs that read the stage are done
-    uint64_t sfFull[kSfRing];    // even CTA: both CTAs have staged the chunk's scale layouts (16 warp arrivals)
-    uint64_t sfEmpty[kSfRing];   // per CTA: the chunk buffer has been copied to TMEM
+    uint64_t sfFull[2];          // even CTA: both CTAs have staged the group's scale layouts (16 warp arrivals)
+    uint64_t sfEmpty[2];         // per CTA: the group's buffer has been copied to TMEM
     uint64_t tmemFull;           // per CTA: a tile's accumulator is complete
     uint64_t tmemEmpty;          // even CTA: all 16 epilogue warps have read the accumulator
     uint32_t tmemBase;
@@ -70,6 +86,7 @@ struct Shared {
     int tilePrefix[kMaxGroups + 1];
     int rowStart[kMaxGroups];
     int rowCount[kMaxGroups];
+    int tileRows[kMaxGroups]; // tokens per tile of the group, a multiple of 32
 };
 
 __device__ __forceinline__ uint32_t clusterCtaRank() {
@@ -122,46 +139,34 @@ __device__ __forceinline__ uint64_t sfDesc(uint32_t smem_addr) {
 __device__ __forceinline__ void tmemCpPair(uint32_t tmem_dst, uint64_t desc) {
     asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_dst), "l"(desc) : "memory");
 }
-// D fp32, A and B e4m3 K-major, M = 256 (both CTAs), N = 128, scale factors E8M0, scale-factor id `sf` for A and B.
-__device__ __forceinline__ uint32_t instrDescMx(uint32_t sf) {
-    return (sf << 4) | (static_cast<uint32_t>(BNS >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>((2 * BM) >> 4) << 24) | (sf << 29);
+// D fp32, A and B e4m3 K-major, M = 256 (both CTAs), N = n, scale factors E8M0, scale-factor id `sf` for A and B.
+__device__ __forceinline__ uint32_t instrDescMx(uint32_t sf, uint32_t n) {
+    return (sf << 4) | ((n >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>((2 * BW) >> 4) << 24) | (sf << 29);
 }
 
-// One 128-channel step: eight block-scaled MMAs (four per accumulator half) and the commit that frees
-// the stage.  The non-blocking test of the next step's barrier sits between the two groups of
-// MMAs: its latency then runs while the second group is being issued, and its result is read last.
-__device__ __forceinline__ void issueKStepMx(uint32_t tmem_d0, uint32_t tmem_d1, uint64_t da, uint64_t dw0, uint64_t dw1, uint32_t idesc, uint32_t tsfa,
-                                             uint32_t tsfb0, uint32_t tsfb1, uint32_t accumulate, uint32_t bar_stage_empty, uint32_t peek_bar,
-                                             uint32_t peek_par, uint32_t &ready_next, uint32_t peek2_bar, uint32_t peek2_par, uint32_t &ready2) {
-    uint64_t da2 = da;
+// One 128-channel step: four block-scaled MMAs and the commit that frees the stage.  The non-blocking
+// test of the next step's barrier sits between the MMAs: its latency then runs while the others are
+// being issued, and its result is read last.
+__device__ __forceinline__ void issueKStepMx(uint32_t tmem_d, uint64_t dw, uint64_t dt, uint32_t idesc, uint32_t tsfw, uint32_t tsft, uint32_t accumulate,
+                                             uint32_t bar_stage_empty, uint32_t peek_bar, uint32_t peek_par, uint32_t &ready_next) {
     asm volatile(
         "{\n"
-        " .reg .pred pf, pf2, pacc, pfirst;\n"
-        " setp.ne.b32 pacc, %16, 0;\n"
-        " setp.ne.b32 pfirst, %12, 0;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%2], %4, %5, %8, [%9], [%10], pfirst;\n"
-        " add.u64 %4, %4, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%2], %4, %5, %8, [%9], [%10], pacc;\n"
-        " add.u64 %4, %4, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%2], %4, %5, %8, [%9], [%10], pacc;\n"
-        " add.u64 %4, %4, 2;\n add.u64 %5, %5, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%2], %4, %5, %8, [%9], [%10], pacc;\n"
-        " mbarrier.test_wait.parity.shared::cta.b64 pf, [%14], %15;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%3], %7, %6, %8, [%9], [%11], pfirst;\n"
-        " add.u64 %7, %7, 2;\n add.u64 %6, %6, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%3], %7, %6, %8, [%9], [%11], pacc;\n"
-        " mbarrier.test_wait.parity.shared::cta.b64 pf2, [%18], %19;\n"
-        " add.u64 %7, %7, 2;\n add.u64 %6, %6, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%3], %7, %6, %8, [%9], [%11], pacc;\n"
-        " add.u64 %7, %7, 2;\n add.u64 %6, %6, 2;\n"
-        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%3], %7, %6, %8, [%9], [%11], pacc;\n"
-        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%13], %17;\n"
+        " .reg .pred pf, pacc, pfirst;\n"
+        " setp.ne.b32 pacc, %11, 0;\n"
+        " setp.ne.b32 pfirst, %7, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%1], %2, %3, %4, [%5], [%6], pfirst;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%1], %2, %3, %4, [%5], [%6], pacc;\n"
+        " mbarrier.test_wait.parity.shared::cta.b64 pf, [%9], %10;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%1], %2, %3, %4, [%5], [%6], pacc;\n"
+        " add.u64 %2, %2, 2;\n add.u64 %3, %3, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%1], %2, %3, %4, [%5], [%6], pacc;\n"
+        " tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%8], %12;\n"
         " selp.u32 %0, 1, 0, pf;\n"
-        " selp.u32 %1, 1, 0, pf2;\n"
         "}\n"
-        : "=r"(ready_next), "=r"(ready2), "+r"(tmem_d0), "+r"(tmem_d1), "+l"(da), "+l"(dw0), "+l"(dw1), "+l"(da2)
-        : "r"(idesc), "r"(tsfa), "r"(tsfb0), "r"(tsfb1), "r"(accumulate), "r"(bar_stage_empty), "r"(peek_bar), "r"(peek_par), "r"(1u),
-          "h"(static_cast<uint16_t>(3)), "r"(peek2_bar), "r"(peek2_par)
+        : "=r"(ready_next), "+r"(tmem_d), "+l"(dw), "+l"(dt)
+        : "r"(idesc), "r"(tsfw), "r"(tsft), "r"(accumulate), "r"(bar_stage_empty), "r"(peek_bar), "r"(peek_par), "r"(1u), "h"(static_cast<uint16_t>(3))
         : "memory");
 }
 
@@ -184,14 +189,15 @@ __device__ __forceinline__ bool tileAt(const Shared &sh, int groups, int n_tiles
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
-    unsigned char *sf_ring = tiles + kStages * kStageBytes; // kSfRing buffers of {A, W left, W right} layouts
-    Shared &sh = *reinterpret_cast<Shared *>(sf_ring + kSfRing * kSfBufBytes);
+    unsigned char *sf_ring = tiles + kStages * kStageBytes; // two buffers of kGroupChunks chunks' layouts
+    Shared &sh = *reinterpret_cast<Shared *>(sf_ring + 2 * kSfBufBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = p.N / BN, k_steps = p.K / BK;
+    const int n_tiles = p.N / (2 * BW), k_steps = p.K / BK;
     const int chunks = k_steps / kChunkSteps; // K is a multiple of 512
+    const int sf_groups = (chunks + kGroupChunks - 1) / kGroupChunks; // per tile
     const uint32_t cta = clusterCtaRank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
@@ -200,7 +206,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
             mbarInit(&sh.full[s], 1);
             mbarInit(&sh.empty[s], 1);
         }
-        for (int b = 0; b < kSfRing; ++b) {
+        for (int b = 0; b < 2; ++b) {
             mbarInit(&sh.sfFull[b], 2 * kPromoWarps);
             mbarInit(&sh.sfEmpty[b], 1);
         }
@@ -211,10 +217,12 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
         int run = 0;
         for (int g = 0; g < p.groups; ++g) {
             const int c = p.row_count[g];
+            const int tiles_g = (c + BT - 1) / BT; // equal tiles, rounded up to the MMA's granularity
             sh.tilePrefix[g] = run;
             sh.rowStart[g] = p.row_start[g];
             sh.rowCount[g] = c;
-            run += ((c + 2 * BM - 1) / (2 * BM)) * n_tiles;
+            sh.tileRows[g] = tiles_g > 0 ? ((c + tiles_g - 1) / tiles_g + 31) & ~31 : 32;
+            run += tiles_g * n_tiles;
         }
         sh.tilePrefix[p.groups] = run;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -241,17 +249,19 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
         uint32_t it = 0;
         Tile t;
         for (int ti = pair; tileAt(sh, p.groups, n_tiles, ti, t); ti += pairs) {
-            const int row0 = sh.rowStart[t.g] + t.mt * (2 * BM) + static_cast<int>(cta) * BM;
-            const int wrow = t.g * p.N + t.nt * BN + static_cast<int>(cta) * WBOX;
+            const int half = sh.tileRows[t.g] / 2; // tokens of this CTA
+            const int row0 = sh.rowStart[t.g] + t.mt * (2 * half) + static_cast<int>(cta) * half;
+            const int wrow = t.g * p.N + t.nt * (2 * BW) + static_cast<int>(cta) * BW;
+            const int boxes = (half + TBOX - 1) / TBOX;
+            const uint32_t bytes = static_cast<uint32_t>(2 * (kWTileBytes + boxes * kTBoxBytes)); // both CTAs' shares
             for (int ks = 0; ks < k_steps; ++ks, ++it) {
                 const int s = it % kStages;
                 if (!mbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, abort_flag)) goto producer_done;
-                if (cta == 0) mbarExpectTx(&sh.full[s], 2 * kStageBytes);
+                if (cta == 0) mbarExpectTx(&sh.full[s], bytes);
                 const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
                 unsigned char *st = tiles + s * kStageBytes;
-                tmaLoad2dPair(st, &mapA, ks * BK, row0, bar);
-                tmaLoad2dPair(st + kATileBytes, &mapW, ks * BK, wrow, bar);
-                tmaLoad2dPair(st + kATileBytes + kWBoxBytes, &mapW, ks * BK, wrow + BNS, bar);
+                tmaLoad2dPair(st, &mapW, ks * BK, wrow, bar);
+                for (int b = 0; b < boxes; ++b) tmaLoad2dPair(st + kWTileBytes + b * kTBoxBytes, &mapT, ks * BK, row0 + b * TBOX, bar);
             }
         }
     producer_done:;
@@ -268,14 +278,20 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
         const uint64_t desc0 = smemDesc(smemU32(tiles));
         const uint32_t sf_smem0 = smemU32(sf_ring);
         const uint32_t total_chunks = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(chunks);
+        uint32_t known_tile = 0xffffffffu, n_tokens = 32;
         for (uint32_t cc = me; cc < total_chunks; cc += 2) {
             const uint32_t tile = cc / static_cast<uint32_t>(chunks), c = cc - tile * static_cast<uint32_t>(chunks);
             const uint32_t it0 = cc * kChunkSteps;
             uint32_t s = it0 % kStages, full_par = (it0 / kStages) & 1u;
-            const uint32_t b = cc % kSfRing;
+            const uint32_t gg = tile * static_cast<uint32_t>(sf_groups) + c / kGroupChunks, b = gg & 1u; // scale group
+            if (tile != known_tile) {
+                Tile t;
+                if (tileAt(sh, p.groups, n_tiles, pair + static_cast<int>(tile) * pairs, t)) n_tokens = static_cast<uint32_t>(sh.tileRows[t.g]);
+                known_tile = tile;
+            }
             // Everything this chunk depends on, before asking for the turn.
             if (c == 0 && !mbarWait(&sh.tmemEmpty, (tile & 1u) ^ 1u, abort_flag)) goto issuer_done; // accumulator drained by the previous epilogue
-            if (!mbarWait(&sh.sfFull[b], (cc / kSfRing) & 1u, abort_flag)) goto issuer_done;
+            if (c % kGroupChunks == 0 && !mbarWait(&sh.sfFull[b], (gg >> 1) & 1u, abort_flag)) goto issuer_done;
             if (!mbarWait(&sh.full[s], full_par, abort_flag)) goto issuer_done;
             {
                 const long long t0 = clock64();
@@ -288,12 +304,18 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
                 }
             }
             tcFenceAfter();
-            const uint32_t src = sf_smem0 + b * kSfBufBytes;
-            const uint32_t sfc = tmem + kAccCols + (cc & 1u) * kSfTmemStride;
-            tmemCpPair(sfc, sfDesc(src));
-            tmemCpPair(sfc + 4, sfDesc(src + kSfAtomBytes));
-            tmemCpPair(sfc + 8, sfDesc(src + 2 * kSfAtomBytes));
-            tcCommitPair(sfempty_bar0 + b * 8u); // the buffer may be refilled once the copies have read it
+            const uint32_t sf_base = tmem + kAccCols + b * kSfTmemStride;
+            if (c % kGroupChunks == 0) {
+                const uint32_t here = min(static_cast<uint32_t>(kGroupChunks), static_cast<uint32_t>(chunks) - c);
+                for (uint32_t i = 0; i < here; ++i) {
+                    const uint32_t src = sf_smem0 + b * kSfBufBytes + i * kSfChunkBytes, dst = sf_base + i * kSfTmemChunk;
+                    tmemCpPair(dst, sfDesc(src));
+                    if (n_tokens > 128) tmemCpPair(dst + 4, sfDesc(src + kSfAtomBytes));
+                    tmemCpPair(dst + 8, sfDesc(src + 2 * kSfAtomBytes));
+                }
+                tcCommitPair(sfempty_bar0 + b * 8u); // the buffer may be refilled once the copies have read it
+            }
+            const uint32_t sfc = sf_base + (c % kGroupChunks) * kSfTmemChunk;
             uint32_t ready = 1; // the first step's barrier was waited for above
 #pragma unroll
             for (uint32_t sub = 0; sub < kChunkSteps; ++sub) {
@@ -304,12 +326,9 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
                     ns = 0;
                     nfull_par ^= 1u;
                 }
-                const uint64_t da = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
-                const uint64_t dw0 = da + static_cast<uint64_t>(kATileBytes >> 4);
-                const uint64_t dw1 = da + static_cast<uint64_t>((kATileBytes + kWBoxBytes) >> 4);
-                uint32_t unused = 0;
-                issueKStepMx(tmem, tmem + BNS, da, dw0, dw1, instrDescMx(sub), sfc, sfc + 4, sfc + 8, (c | sub) ? 1u : 0u, empty_bar0 + s * 8u,
-                             full_bar0 + ns * 8u, nfull_par, ready, full_bar0 + ns * 8u, nfull_par, unused);
+                const uint64_t dw = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
+                const uint64_t dt = dw + static_cast<uint64_t>(kWTileBytes >> 4);
+                issueKStepMx(tmem, dw, dt, instrDescMx(sub, n_tokens), sfc + 8, sfc, (c | sub) ? 1u : 0u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
                 s = ns;
                 full_par = nfull_par;
             }
@@ -327,93 +346,83 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     } else if (warp >= 4) {
         // ---------------------------------------------------------------- scale staging, then the epilogue
         const int q = warp & 3;
-        const int part = (warp - 4) >> 2; // 0: stages A's layout, 1: stages W's two layouts; epilogue: 64-column part of each half
-        const int row_in_tile = q * 32 + lane;
+        const int part = (warp - 4) >> 2; // epilogue: which half of the tile's tokens
+        const int row = (warp - 4) * 32 + lane; // staging: token of the tile
         const uint32_t sffull0 = mapToCta(smemU32(&sh.sfFull[0]), 0);
         const uint32_t tempty = mapToCta(smemU32(&sh.tmemEmpty), 0);
-        const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16) + part * 64;
+        const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
         const uint32_t *sa32 = reinterpret_cast<const uint32_t *>(p.scale_a);
         const uint32_t *sw32 = reinterpret_cast<const uint32_t *>(p.scale_w);
         const int n_blocks = p.N / 128;
-        // Rows and scale words of a tile, as this thread sees them.
-        struct TileView {
-            Tile t;
-            bool valid;
-            long long grow;
-        };
-        auto view = [&](int ti, TileView &v) -> bool {
-            if (!tileAt(sh, p.groups, n_tiles, ti, v.t)) return false;
-            const int local_row = v.t.mt * (2 * BM) + static_cast<int>(cta) * BM + row_in_tile;
-            v.valid = local_row < sh.rowCount[v.t.g];
-            v.grow = static_cast<long long>(sh.rowStart[v.t.g]) + local_row;
-            return true;
-        };
-        // Builds chunk c of a tile in ring buffer gcc % kSfRing once the issuer has copied that buffer's previous content out.
-        auto stage = [&](const TileView &v, int c, uint32_t gcc) -> bool {
-            const uint32_t b = gcc % kSfRing;
-            if (!mbarWait(&sh.sfEmpty[b], ((gcc / kSfRing) & 1u) ^ 1u, abort_flag)) return false;
+        // Builds the layouts of scale group sg of a tile in buffer gcc % 2 once the issuer has copied that buffer's previous content out.
+        auto stage = [&](const Tile &t, int sg, uint32_t gcc) -> bool {
+            const uint32_t b = gcc & 1u;
+            if (!mbarWait(&sh.sfEmpty[b], ((gcc >> 1) & 1u) ^ 1u, abort_flag)) return false;
             uint32_t *buf = reinterpret_cast<uint32_t *>(sf_ring + b * kSfBufBytes);
-            if (part == 0) {
-                // Row r of this CTA's half: word (r % 32) * 4 + r / 32 (rows beyond the expert get exponent 127 = 1.0).
-                buf[lane * 4 + q] = v.valid ? __ldg(sa32 + v.grow * chunks + c) : 0x7f7f7f7fu;
-            } else {
-                const long long blk = (static_cast<long long>(v.t.g) * n_blocks + v.t.nt * 2) * chunks + c;
-                buf[128 + row_in_tile] = __ldg(sw32 + blk);
-                buf[256 + row_in_tile] = __ldg(sw32 + blk + chunks);
+            const int c0 = sg * kGroupChunks, here = min(kGroupChunks, chunks - c0);
+            const int local = t.mt * sh.tileRows[t.g] + row;
+            const bool valid = row < sh.tileRows[t.g] && local < sh.rowCount[t.g];
+            const uint32_t *sa = sa32 + (static_cast<long long>(sh.rowStart[t.g]) + (valid ? local : 0)) * chunks + c0;
+            const uint32_t *sw = sw32 + (static_cast<long long>(t.g) * n_blocks + t.nt * 2 + static_cast<int>(cta)) * chunks + c0;
+#pragma unroll
+            for (int i = 0; i < kGroupChunks; ++i) {
+                if (i >= here) break;
+                uint32_t *layout = buf + i * (kSfChunkBytes / 4);
+                // Token r: word (r % 32) * 4 + r / 32 of its 128 tokens' layout (rows beyond the expert get exponent 127 = 1.0).
+                layout[part * 128 + lane * 4 + q] = valid ? __ldg(sa + i) : 0x7f7f7f7fu;
+                if (part == 0) layout[256 + row] = __ldg(sw + i);
             }
             asm volatile("fence.proxy.async;" ::: "memory"); // these generic-proxy writes are read by tcgen05.cp
             __syncwarp();
             if (lane == 0) mbarArriveClusterRelease(sffull0 + b * 8u);
             return true;
         };
-        // Staging runs ahead of the issuer by up to the ring's depth, across tile boundaries: the first
-        // chunks of the next tile are built before this tile's epilogue, so the issuer finds them
-        // waiting when the accumulator is free again.
-        const int ahead = chunks < kSfRing ? chunks : kSfRing;
-        TileView cur, nxt;
+        // Staging runs ahead of the issuer by up to two groups, across tile boundaries: the first groups of the next
+        // tile are built before this tile's epilogue, so the issuer finds them waiting when the accumulator is free again.
+        const int ahead = sf_groups < 2 ? sf_groups : 2;
+        Tile cur, nxt;
         int ti = pair;
-        bool have = view(ti, cur);
-        uint32_t cc_base = 0;
+        bool have = tileAt(sh, p.groups, n_tiles, ti, cur);
+        uint32_t g_base = 0;
         bool ok = true;
         if (have)
-            for (int c = 0; c < ahead && ok; ++c) ok = stage(cur, c, cc_base + c);
+            for (int c = 0; c < ahead && ok; ++c) ok = stage(cur, c, g_base + c);
         for (int tile = 0; have && ok; ++tile) {
-            for (int c = ahead; c < chunks && ok; ++c) ok = stage(cur, c, cc_base + c);
-            const bool have_next = view(ti + pairs, nxt);
+            for (int c = ahead; c < sf_groups && ok; ++c) ok = stage(cur, c, g_base + c);
+            const bool have_next = tileAt(sh, p.groups, n_tiles, ti + pairs, nxt);
             if (have_next)
-                for (int c = 0; c < ahead && ok; ++c) ok = stage(nxt, c, cc_base + chunks + c);
+                for (int c = 0; c < ahead && ok; ++c) ok = stage(nxt, c, g_base + sf_groups + c);
             if (!ok) break;
-            const Tile &t = cur.t;
-            // Epilogue: the tile's accumulator, two halves of 128 columns, this warp's 64 columns of each.
-            // All four TMEM loads first, then the accumulator goes back to the issuer at once; conversion
-            // and stores follow while the next tile's main loop is already running.
+            const Tile &t = cur;
+            // Epilogue: this warp's 32 columns of D (TMEM lanes) for its half of the tokens (TMEM columns), up to
+            // four blocks of 32.  All TMEM loads first, then the accumulator goes back to the issuer at once;
+            // conversion and stores follow while the next tile's main loop is already running.
             if (!mbarWait(&sh.tmemFull, static_cast<uint32_t>(tile) & 1u, abort_flag)) break;
             tcFenceAfter();
-            float v0[32], v1[32], v2[32], v3[32];
-            tmemLoad32(lane_base, v0);
-            tmemLoad32(lane_base + 32, v1);
-            tmemLoad32(lane_base + BNS, v2);
-            tmemLoad32(lane_base + BNS + 32, v3);
-            tmemLoadWait(v0);
-            tmemLoadWait(v1);
-            tmemLoadWait(v2);
-            tmemLoadWait(v3);
+            const int rows_t = sh.tileRows[t.g];
+            const int half = (rows_t / 2 + 31) & ~31;
+            const int first = part * half, mine = min(half, rows_t - first); // tokens of this warp (a multiple of 32, may be <= 0)
+            float v[4][32];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j * 32 < mine) tmemLoad32(lane_base + first + j * 32, v[j]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j * 32 < mine) tmemLoadWait(v[j]);
             tcFenceBefore();
             __syncwarp();
             if (lane == 0) mbarArriveCluster(tempty);
-            // A thread holds 64 consecutive columns of its own row: eight 16-byte pieces per half.  Eight
-            // lanes exchange pieces (8 x 8 transpose by three butterfly steps) so that every store
-            // instruction writes whole 128-byte runs: lane 8g + c then holds piece c of rows 8g .. 8g + 7.
-            const int first_row = t.mt * (2 * BM) + static_cast<int>(cta) * BM + q * 32 + (lane & ~7); // tile-local row of this lane group
-            const long long first_grow = static_cast<long long>(sh.rowStart[t.g]) + first_row;
-            const int rows_left = sh.rowCount[t.g] - first_row; // rows of the group that belong to the expert
-            __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + first_grow * p.N + t.nt * BN + part * 64 + (lane & 7) * 8;
-            storeRows64(v0, v1, out, p.N, rows_left, lane);
-            storeRows64(v2, v3, out + BNS, p.N, rows_left, lane);
+            const int local = t.mt * rows_t + first;
+            const int left = min(mine, sh.rowCount[t.g] - local);
+            __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + (static_cast<long long>(sh.rowStart[t.g]) + local) * p.N + t.nt * (2 * BW) +
+                static_cast<int>(cta) * BW + q * 32;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (j * 32 < left) storeCols32(v[j], out + static_cast<long long>(j * 32) * p.N, p.N, left - j * 32, lane);
             cur = nxt;
             have = have_next;
             ti += pairs;
-            cc_base += static_cast<uint32_t>(chunks);
+            g_base += static_cast<uint32_t>(sf_groups);
         }
     }
 
@@ -429,8 +438,8 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
 
 } // namespace
 
-cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
-    const size_t smem = size_t(kStages) * kStageBytes + size_t(kSfRing) * kSfBufBytes + sizeof(Shared) + 1024;
+cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
+    const size_t smem = size_t(kStages) * kStageBytes + size_t(2) * kSfBufBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     static bool attr_done[64] = {};
@@ -462,8 +471,8 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapA, const CUtenso
     }
     int pairs = (dev >= 0 && dev < 64) ? max_pairs[dev] : sms / 2;
     if (p.grid > 0 && p.grid / 2 < pairs) pairs = p.grid / 2 > 0 ? p.grid / 2 : 1;
-    const long long max_tiles = (static_cast<long long>(p.a_rows + 2 * BM - 1) / (2 * BM) + p.groups) * (p.N / BN);
+    const long long max_tiles = (static_cast<long long>(p.a_rows + BT - 1) / BT + p.groups) * (p.N / (2 * BW));
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapA, mapW, p);
+    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapW, p);
 }

@@ -125,6 +125,22 @@ __device__ __forceinline__ uint64_t ldAcquireSys(const uint64_t *p) {
     return v;
 }
 
+// Packed fp32 pairs (two FMAs per instruction, each half rounded as fmaf rounds).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+// acc[i] = v[i] * s + acc[i] for 32 values; s2 = pack2(s, s).
+__device__ __forceinline__ void fmaScale32(uint64_t (&acc)[16], const float (&v)[32], uint64_t s2) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i]) : "l"(pack2(v[2 * i], v[2 * i + 1])), "l"(s2));
+}
+__device__ __forceinline__ void unpack32(const uint64_t (&acc)[16], float (&v)[32]) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * i]), "=f"(v[2 * i + 1]) : "l"(acc[i]));
+}
+
 // Epilogue store of a 32-row x 64-column bf16 block held one row per lane (64 fp32 per thread).
 // Written row by row, every store instruction would touch 32 different 128-byte lines with 16
 // bytes each.  Instead eight lanes exchange their 16-byte pieces (an 8 x 8 transpose in three
@@ -160,6 +176,37 @@ __device__ __forceinline__ void storeRows64(const float (&lo)[32], const float (
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         if (i < rows_left) *reinterpret_cast<uint4 *>(out + static_cast<long long>(i) * row_stride) = piece[i];
+}
+
+// Writes 32 tokens x 32 columns of D: this lane holds column `lane` of 32 consecutive tokens (v[i]: token i).  Three
+// exchanges with neighbouring lanes (1, 2, 4 away) turn that into eight consecutive columns of four tokens per lane
+// (token 8m + lane % 8, columns lane / 8 * 8 ..), so that a store instruction writes whole 64-byte runs.
+// `out`: this block's first token and column, tokens_left: how many of the 32 may be written.
+__device__ __forceinline__ void storeCols32(const float (&v)[32], __nv_bfloat16 *out, long long row_stride, int tokens_left, int lane) {
+    uint32_t w[16];
+    const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) { // w[j]: columns (lane & ~1, lane | 1) of token 2j + b0
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        const uint32_t own = *reinterpret_cast<const uint32_t *>(&h);
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+        w[j] = b0 ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
+    }
+    uint2 x[8]; // x[i]: four columns of token 4i + 2 b1 + b0
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, b1 ? w[2 * i] : w[2 * i + 1], 2);
+        x[i] = b1 ? make_uint2(got, w[2 * i + 1]) : make_uint2(w[2 * i], got);
+    }
+    out += (lane >> 3) * 8;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        const uint2 give = b2 ? x[2 * m] : x[2 * m + 1];
+        const uint32_t gx = __shfl_xor_sync(0xffffffffu, give.x, 4), gy = __shfl_xor_sync(0xffffffffu, give.y, 4);
+        const uint4 o = b2 ? make_uint4(gx, gy, x[2 * m + 1].x, x[2 * m + 1].y) : make_uint4(x[2 * m].x, x[2 * m].y, gx, gy);
+        const int token = 8 * m + (lane & 7);
+        if (token < tokens_left) *reinterpret_cast<uint4 *>(out + token * row_stride) = o;
+    }
 }
 
 } // namespace nixl_tc
