@@ -112,9 +112,9 @@ typedef struct NixlEpGroupRecord {
 
 typedef struct NixlEpScratch { /* device memory private to the rank; zero before first use */
     int32_t *cnt;      /* [E] */
-    int32_t *fill;     /* [E] */
+    int32_t *fill;     /* [E] (not used by these kernels) */
     int32_t *sent;     /* [E] */
-    uint32_t *barrier; /* [4] */
+    uint32_t *barrier; /* [4] grid barrier (two words), CTAs that have left a dispatch */
     int32_t *status;   /* [1] bit0: a peer timed out, bit1: grid barrier timed out, bit2: capacity exceeded */
     int32_t *mask;     /* [R] non-zero: rank excluded */
 } NixlEpScratch;
@@ -164,7 +164,7 @@ typedef struct NixlEpCombineParams {
      * "outputs ready" and every home rank loads its tokens' rows straight from the expert ranks
      * and reduces them, so no row is written twice.  send_row comes from the dispatch. */
     int32_t pull;
-    const int32_t *send_row;    /* [T][K] */
+    const int32_t *send_row;    /* [T][K]; also used by a group of one rank, whatever the mode */
     /* Push mode only: rows cross NVLink in a logarithmic 10-bit format (9-bit magnitude code on a
      * per-128-channel grid plus sign; 0.66 of the bf16 bytes) and are decoded inside the reduction.
      * Needs H % 512 == 0. */

@@ -686,7 +686,7 @@ class Buffer:
         p.pull = int(pull)
         p.max_tokens = self.max_tokens
         p.use_logfmt = int(use_logfmt)
-        p.send_row = handle.send_row.data_ptr() if pull else None
+        p.send_row = handle.send_row.data_ptr() if handle.send_row is not None else None
         p.x = x.data_ptr()
         p.recv_info = handle.src_info.data_ptr()
         p.recv_count, p.expert_offsets = handle.recv_count.data_ptr(), handle.expert_offsets.data_ptr()
