@@ -1000,7 +1000,7 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         b.launch.totalChunks = static_cast<uint32_t>(chunks);
         b.launch.chunkShift = shift;
         b.launch.warpChunks = warp_chunks ? 1 : 0;
-        b.launch.uniformChunks = static_cast<uint32_t>(per);
+        b.launch.uniformChunks = b.uniformChunks;
         b.flag = c->flags.acquire();
         if (!b.flag) return fail(NIXL_ERR_BACKEND);
         b.launch.hostFlag = b.flag; // UVA: the pinned allocation's host address is device-visible
@@ -1018,19 +1018,22 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         // A device table for batches too long for the launch parameters, and for any batch of
         // several descriptors that may go through the proxy (a proxy command has room for one).
         if (!inline_ok || (b.proxyEligible && n > 1)) {
-            const size_t tbytes = n * sizeof(XferDesc), sbytes = (n + 1) * sizeof(uint32_t);
-            const size_t toff = 0, soff = (tbytes + 15) & ~size_t(15);
-            b.table = c->arena->alloc(soff + sbytes);
+            // One upload for both arrays; the starts stay behind when no kernel will search them.
+            const size_t tbytes = n * sizeof(XferDesc), sbytes = b.uniformChunks && copyPath_ == CopyPath::VECTOR ? 0 : (n + 1) * sizeof(uint32_t);
+            const size_t soff = (tbytes + 15) & ~size_t(15);
+            b.table = c->arena->alloc(soff + (n + 1) * sizeof(uint32_t));
             if (!b.table) return fail(NIXL_ERR_BACKEND);
             DeviceScope ds(b.device);
             char *base = static_cast<char *>(b.table);
-            // Pageable source: the runtime copies it out before returning, so the vectors may die.
-            bool ok = cudaOk(cudaMemcpyAsync(base + toff, b.descs.data(), tbytes, cudaMemcpyHostToDevice, c->prepStream), "table upload");
-            ok = ok && cudaOk(cudaMemcpyAsync(base + soff, starts.data(), sbytes, cudaMemcpyHostToDevice, c->prepStream), "table upload");
+            std::vector<char> image(soff + sbytes);
+            std::memcpy(image.data(), b.descs.data(), tbytes);
+            if (sbytes) std::memcpy(image.data() + soff, starts.data(), sbytes);
+            // Pageable source: the runtime copies it out before returning, so the vector may die.
+            bool ok = cudaOk(cudaMemcpyAsync(base, image.data(), image.size(), cudaMemcpyHostToDevice, c->prepStream), "table upload");
             ok = ok && cudaOk(cudaEventCreateWithFlags(&b.uploaded, cudaEventDisableTiming), "cudaEventCreate");
             ok = ok && cudaOk(cudaEventRecord(b.uploaded, c->prepStream), "cudaEventRecord");
             if (!ok) return fail(NIXL_ERR_BACKEND);
-            b.tableDev = reinterpret_cast<const XferDesc *>(base + toff);
+            b.tableDev = reinterpret_cast<const XferDesc *>(base);
             b.startsDev = reinterpret_cast<const uint32_t *>(base + soff);
             if (!inline_ok) {
                 b.launch.table = b.tableDev;

@@ -38,6 +38,24 @@ def _up(x: int, a: int = _ALIGN) -> int:
     return (x + a - 1) // a * a
 
 
+def _raw_stream(device: torch.device) -> int:
+    """The current stream's ``cudaStream_t`` of a device (torch's own accessor skips the Stream object: 0.2 us instead of 2)."""
+    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if get is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return get(device.index if device.index is not None else torch.cuda.current_device())
+
+
+def _launch_on(device: torch.device, fn, ref, stream, what: str) -> None:
+    """Calls a launcher with ``device`` current; entering the device context costs as much as half a launch, so only when needed."""
+    if device.index is None or torch.cuda.current_device() == device.index:
+        rc = fn(ref, stream)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(ref, stream)
+    _lib.check(rc, what)
+
+
 class _Layout(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int64) for n in (
         "off_counts", "off_counts_flag", "off_disp_flag", "off_recv_x", "off_recv_scales", "off_recv_info", "off_comb_x", "off_comb_flag", "off_comb_in",
@@ -206,6 +224,9 @@ class Buffer:
         with torch.cuda.device(self.device):
             self._gemm_status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._comb_params = _CombineParams()
+        # Parameter blocks that stay the same for the life of the buffer: built once, not per call.
+        self._layouts = (self._make_layout(0), self._make_layout(1))
+        self._scratch_ptrs = self._make_scratch()
         lib = _lib.lib()
         self._dispatch_fn = lib.nixl_ep_dispatch_launch
         self._dispatch_fn.argtypes = [ctypes.POINTER(_DispatchParams), ctypes.c_void_p]
@@ -399,18 +420,27 @@ class Buffer:
     # ------------------------------------------------------------------ internals
 
     def _layout(self, parity: int) -> _Layout:
+        return self._layouts[parity]
+
+    def _make_layout(self, parity: int) -> _Layout:
         lay = _Layout()
         for name, off in self._lay.items():
             setattr(lay, name, off + parity * self._half)
         return lay
 
     def _scratch(self) -> _Scratch:
+        return self._scratch_ptrs
+
+    def _make_scratch(self) -> _Scratch:
         E = self.num_experts
         s = _Scratch()
         base = self._cnt.data_ptr()
         s.cnt, s.fill, s.sent = base, base + 4 * E, base + 8 * E
         s.barrier, s.status, s.mask = self._bar.data_ptr(), self._status.data_ptr(), self.mask.data_ptr()
         return s
+
+    def _stream(self) -> ctypes.c_void_p:
+        return ctypes.c_void_p(_raw_stream(self.device))
 
     def _region(self, parity: int, name: str, nbytes: int) -> torch.Tensor:
         start = self._lay[name] + parity * self._half
@@ -495,9 +525,13 @@ class Buffer:
             elif use_fp8:
                 scales = self._region(parity, "off_recv_scales", rows * (H // 128) * 4).view(torch.float32).view(rows, H // 128)
             src_info = self._region(parity, "off_recv_info", rows * 8).view(torch.int32).view(rows, 2)
-            slot = (p, recv_count, layout_range, expert_offsets, recv_x, scales, src_info, send_row)
+            packed = None
+            if rows_per_expert:  # what the low-latency entry point returns
+                n = El * rows_per_expert
+                packed = (recv_x[:n].view(El, rows_per_expert, H), scales[:n].view(El, rows_per_expert, -1) if scales is not None else None)
+            slot = (p, recv_count, layout_range, expert_offsets, recv_x, scales, src_info, send_row, packed)
             self._disp_cache[key] = slot
-        p, recv_count, layout_range, expert_offsets, recv_x, scales, src_info, send_row = slot
+        p, recv_count, layout_range, expert_offsets, recv_x, scales, src_info, send_row, _ = slot
 
         p.x, p.topk_idx, p.T = x.data_ptr(), topk_idx.data_ptr(), T
         p.topk_weights = topk_weights.data_ptr() if topk_weights is not None else None
@@ -506,13 +540,12 @@ class Buffer:
         p.peers = self._peers_view
         p.epoch = epoch
         p.grid = grid or self._num_sms
-        stream_ptr = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        stream_ptr = self._stream()
         fn, ref = self._dispatch_fn, ctypes.byref(p)
 
         def launch(phases: int) -> None:
             p.phases = phases
-            with torch.cuda.device(self.device):
-                _lib.check(fn(ref, stream_ptr), "nixl_ep_dispatch_launch")
+            _launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_dispatch_launch")
 
         launch(phases_now)
         hook = (lambda: launch(2)) if hook_later else None
@@ -585,12 +618,13 @@ class Buffer:
         rpe = self.num_ranks * self.max_tokens
         recv_x, scales, handle, hook, keep = self._dispatch(x, topk_idx, use_fp8, round_scale, rpe, 1 if return_recv_hook else 3, return_recv_hook,
                                                             use_ue8m0=use_ue8m0)
-        El = self.local_experts
-        packed = recv_x[: El * rpe].view(El, rpe, self.hidden)
+        packed, packed_scales = self._disp_cache[(handle.parity, bool(use_fp8), rpe, bool(use_ue8m0))][-1]
+        packed = packed.view(packed.shape)  # views of the caller's own (an autograd function marks what it returns)
         event = EventOverlap(self._record() if async_finish else None)
         self._keep = keep
         if use_fp8:
-            return (packed, scales[: El * rpe].view(El, rpe, -1)), handle.recv_count, handle, event, hook
+            packed_scales = packed_scales.view(packed_scales.shape)
+            return (packed, packed_scales), handle.recv_count, handle, event, hook
         return packed, handle.recv_count, handle, event, hook
 
     def low_latency_combine(
@@ -664,30 +698,31 @@ class Buffer:
         if topk_weights.dtype != torch.float32 or not topk_weights.is_contiguous():
             raise TypeError("topk_weights must be contiguous float32")
         T, K = topk_idx.shape
-        with torch.cuda.device(self.device):
-            if out is None:
-                out = torch.empty(T, self.hidden, dtype=torch.bfloat16, device=self.device)
+        if out is None:
+            out = torch.empty(T, self.hidden, dtype=torch.bfloat16, device=self.device)
         rows = self.ll_rows if handle.rows_per_expert else self.compact_rows
-        staged = self._region(handle.parity, "off_comb_in", rows * self.hidden * 2).view(torch.bfloat16).view(rows, self.hidden)
+        x_ptr = x.data_ptr()
+        staged_ptr = self.buffer.data_ptr() + self._layouts[handle.parity].off_comb_in
         if pull is None and handle.has_group_records and not use_logfmt and self.combine_pull is None:
             pull = 2  # the expert ranks know which rows belong to one token: one row per (token, rank) comes back
         if pull is None:
             # Unless told otherwise: pull when the caller wrote its outputs into the exposed buffer
             # (nothing to copy), push when they live elsewhere (staging them first costs more than it saves).
-            pull = self.combine_pull if self.combine_pull is not None else x.data_ptr() == staged.data_ptr()
+            pull = self.combine_pull if self.combine_pull is not None else x_ptr == staged_ptr
         if pull == 2 and not handle.has_group_records:
             raise ValueError("rank-reduced combine needs a dispatch that was given topk_weights")
         if pull == 1 or pull is True:
             if x.shape[0] > rows:
                 raise ValueError("combine input has more rows than the buffer holds")
-            if x.data_ptr() != staged.data_ptr():
+            if x_ptr != staged_ptr:
+                staged = self._region(handle.parity, "off_comb_in", rows * self.hidden * 2).view(torch.bfloat16).view(rows, self.hidden)
                 staged[: x.shape[0]].copy_(x)  # callers that write into get_next_combine_buffer() skip this copy
         p = self._comb_params
         p.pull = int(pull)
         p.max_tokens = self.max_tokens
         p.use_logfmt = int(use_logfmt)
         p.send_row = handle.send_row.data_ptr() if handle.send_row is not None else None
-        p.x = x.data_ptr()
+        p.x = x_ptr
         p.recv_info = handle.src_info.data_ptr()
         p.recv_count, p.expert_offsets = handle.recv_count.data_ptr(), handle.expert_offsets.data_ptr()
         p.topk_idx, p.topk_weights, p.out = topk_idx.data_ptr(), topk_weights.data_ptr(), out.data_ptr()
@@ -697,13 +732,12 @@ class Buffer:
         p.lay = self._layout(handle.parity)
         p.epoch, p.timeout_ns = handle.epoch, self.timeout_ns
         p.scr = self._scratch()
-        stream_ptr = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
+        stream_ptr = self._stream()
         fn, ref = self._combine_fn, ctypes.byref(p)
 
         def launch(phases: int) -> None:
             p.phases = phases
-            with torch.cuda.device(self.device):
-                _lib.check(fn(ref, stream_ptr), "nixl_ep_combine_launch")
+            _launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_combine_launch")
 
         launch(phases_now)
         self._keep_c = (x, topk_idx, topk_weights, out, p)
