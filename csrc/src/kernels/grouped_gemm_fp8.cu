@@ -5,8 +5,8 @@
 //   W: e4m3, one fp32 scale per 128 x 128 block
 //
 // sm_100a only.  One persistent CTA per SM, 384 threads, warp-specialised:
-//   warp 0  TMA producer   cp.async.bulk.tensor (2-D, 128-byte swizzle) of a 128x128 A tile and a
-//                          128x128 W tile per 128-channel step into a 5-stage shared-memory ring
+//   warp 0  TMA producer   cp.async.bulk.tensor (2-D, 128-byte swizzle) of an A tile of 32, 64 or 128 rows and a
+//                          128x128 W tile per 128-channel step into a shared-memory ring of 10, 8 or 6 stages
 //   warp 1  MMA issuer     4 x tcgen05.mma.kind::f8f6f4 (M128 N128 K32) per step into one of four
 //                          TMEM accumulators (128 lanes x 128 fp32 columns each: all 512 columns).
 //                          It polls one barrier per step, with a non-blocking test issued behind
@@ -44,10 +44,11 @@ namespace {
 using namespace nixl_tc;
 
 constexpr int BM = 128, BN = 128, BK = 128; // tile; BK is also the scale granularity
-constexpr int kStages = 5;
+constexpr int kRingBytes = 200 * 1024;
+constexpr int kMaxStages = 10;
 constexpr int kThreads = 384;              // 4 role warps + 8 promotion warps
 constexpr int kTileBytes = BM * BK;         // 16 KiB (fp8)
-constexpr int kStageBytes = 2 * kTileBytes; // A + W
+constexpr int kTailBytes = kTileBytes - 32 * BK; // an MMA reads 128 A rows, also of a last stage that has room for 32
 constexpr int kAccBufs = 4;                 // TMEM accumulators in flight (4 x 128 columns = all of TMEM)
 constexpr int kTmemCols = kAccBufs * BN;
 
@@ -56,12 +57,13 @@ using nixl_gemm::GEMM_ERR_TIMEOUT;
 using nixl_gemm::kMaxGroups;
 
 struct Shared {
-    uint64_t full[kStages];
-    uint64_t empty[kStages];
+    uint64_t full[kMaxStages];
+    uint64_t empty[kMaxStages];
     uint64_t tmemFull[kAccBufs];
     uint64_t tmemEmpty[kAccBufs];
     uint32_t tmemBase;
     int abort;
+    int aRows;                      // A rows a stage has room for: 32, 64 or 128
     int tilePrefix[kMaxGroups + 1]; // tiles before group g
     int rowStart[kMaxGroups];
     int rowCount[kMaxGroups];
@@ -100,6 +102,11 @@ __device__ __forceinline__ void issueStep(uint32_t tmem_d, uint64_t da, uint64_t
         : "memory");
 }
 
+// Rows of the one TMA box that fetches A for a tile with `rows` rows.  One box, not several small ones: each TMA
+// instruction of a step costs its issuing thread more than the rows it may save (32 experts, 32 rows each, 2048 x 7168: one
+// box of 32 92 us, two of 16 101 us).
+__device__ __forceinline__ int aBoxRows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : BM; }
+
 struct Tile {
     int g, mt, nt;
 };
@@ -119,15 +126,16 @@ __device__ __forceinline__ bool tileAt(const Shared &sh, int groups, int n_tiles
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA32, const __grid_constant__ CUtensorMap mapA64,
+                  const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
-    Shared &sh = *reinterpret_cast<Shared *>(tiles + kStages * kStageBytes);
+    Shared &sh = *reinterpret_cast<Shared *>(tiles + kRingBytes + kTailBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = p.N / BN, k_steps = p.K / BK;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kMaxStages; ++s) {
             mbarInit(&sh.full[s], 2); // producer (with the byte count) + slot watcher
             mbarInit(&sh.empty[s], 1);
         }
@@ -137,7 +145,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         }
         sh.abort = 0;
         // Tile table: group g owns ceil(count/BM) x n_tiles tiles.
-        int run = 0;
+        int run = 0, most = 0;
         if (p.counts_flag) {
             // Overlapped with the dispatch: wait for everybody's counts, then derive the rows.
             for (int r = 0; r < p.ranks; ++r) {
@@ -161,6 +169,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 sh.tilePrefix[g] = run;
                 sh.rowStart[g] = p.rows_per_expert > 0 ? g * p.rows_per_expert : next;
                 sh.rowCount[g] = c;
+                most = max(most, c);
                 next += c;
                 run += ((c + BM - 1) / BM) * n_tiles;
             }
@@ -170,10 +179,12 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 sh.tilePrefix[g] = run;
                 sh.rowStart[g] = p.row_start[g];
                 sh.rowCount[g] = c;
+                most = max(most, c);
                 run += ((c + BM - 1) / BM) * n_tiles;
             }
         }
         sh.tilePrefix[p.groups] = run;
+        sh.aRows = aBoxRows(most);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
@@ -185,10 +196,16 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     tcFenceAfter();
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
+    // A stage holds the W tile and as many A rows as the fullest expert has: with few rows per expert (a decode step) the kernel
+    // is bound by the W bytes it keeps in flight, and the room that 128 A rows took goes to more stages.  Measured on one
+    // B200 before (128 A rows, 5 stages) / now: 32 experts, N = K = 4096, 32 rows each 112 / 98 us (5.6 TB/s), 64 rows 114 / 107,
+    // 128 rows 118 / 115.5; 2048 x 7168, 32 rows 110 / 91 us, 64 rows 110 / 99.
+    const uint32_t stage_bytes = static_cast<uint32_t>(kTileBytes + sh.aRows * BK);
+    const uint32_t stages = min(static_cast<uint32_t>(kMaxStages), kRingBytes / stage_bytes);
 
     if (warp == 0 && lane == 0) {
         // ---------------------------------------------------------------- TMA producer
-        uint32_t it = 0; // k-steps issued so far (ring position)
+        uint32_t s = 0, empty_par = 1; // ring position
         Tile t;
         for (int ti = blockIdx.x; tileAt(sh, p.groups, n_tiles, ti, t); ti += gridDim.x) {
             const int row0 = sh.rowStart[t.g] + t.mt * BM;
@@ -218,12 +235,19 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 }
                 asm volatile("fence.proxy.async;" ::: "memory"); // peers' generic-proxy stores before our async-proxy reads
             }
-            for (int ks = 0; ks < k_steps; ++ks, ++it) {
-                const int s = it % kStages;
-                if (!mbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, abort_flag)) goto producer_done;
-                mbarExpectTx(&sh.full[s], kStageBytes);
-                tmaLoad2d(tiles + s * kStageBytes, &mapA, ks * BK, row0, &sh.full[s]);
-                tmaLoad2d(tiles + s * kStageBytes + kTileBytes, &mapW, ks * BK, t.g * p.N + t.nt * BN, &sh.full[s]);
+            const int box = aBoxRows(sh.rowCount[t.g] - t.mt * BM);
+            const CUtensorMap *map = box == 32 ? &mapA32 : box == 64 ? &mapA64 : &mapA;
+            const uint32_t bytes = static_cast<uint32_t>(kTileBytes + box * BK);
+            for (int ks = 0; ks < k_steps; ++ks) {
+                if (!mbarWait(&sh.empty[s], empty_par, abort_flag)) goto producer_done;
+                mbarExpectTx(&sh.full[s], bytes);
+                unsigned char *st = tiles + s * stage_bytes;
+                tmaLoad2d(st, &mapW, ks * BK, t.g * p.N + t.nt * BN, &sh.full[s]);
+                tmaLoad2d(st + kTileBytes, map, ks * BK, row0, &sh.full[s]);
+                if (++s == stages) {
+                    s = 0;
+                    empty_par ^= 1u;
+                }
             }
         }
     producer_done:;
@@ -245,13 +269,13 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) goto mma_done;
             tcFenceAfter();
             uint32_t ns = s + 1, nfull_par = full_par;
-            if (ns == kStages) {
+            if (ns == stages) {
                 ns = 0;
                 nfull_par ^= 1u;
             }
             // Advancing 32 bytes along K inside the swizzle atom = +2 in the 16-byte address field (done in issueStep).
-            const uint64_t da = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
-            const uint64_t dw = da + static_cast<uint64_t>(kTileBytes >> 4);
+            const uint64_t dw = desc0 + static_cast<uint64_t>((s * stage_bytes) >> 4);
+            const uint64_t da = dw + static_cast<uint64_t>(kTileBytes >> 4);
             issueStep(tmem + buf * BN, da, dw, instrDesc(), tfull_bar0 + buf * 8u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
             buf = (buf + 1) & (kAccBufs - 1);
             s = ns;
@@ -274,7 +298,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             mbarArrive(&sh.full[s]);
             buf = (buf + 1) & (kAccBufs - 1);
             if (buf == 0) e_par ^= 1u;
-            if (++s == kStages) s = 0;
+            if (++s == stages) s = 0;
         }
     } else if (warp >= 4) {
         // ---------------------------------------------------------------- promotion + epilogue
@@ -288,6 +312,15 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         for (int ti = blockIdx.x; tileAt(sh, p.groups, n_tiles, ti, t); ti += gridDim.x) {
             const int local_row = t.mt * BM + row_in_tile;
             const bool valid = local_row < sh.rowCount[t.g];
+            if (t.mt * BM + q * 32 >= sh.rowCount[t.g]) { // this warp's 32 rows are padding: it only hands accumulators back
+                bool alive = true;
+                for (int ks = 0; ks < k_steps && alive; ++ks, ++it) {
+                    alive = mbarWait(&sh.tmemFull[it % kAccBufs], (it / kAccBufs) & 1, abort_flag);
+                    if (alive && lane == 0) mbarArrive(&sh.tmemEmpty[it % kAccBufs]);
+                }
+                if (!alive) break;
+                continue;
+            }
             const long long grow = static_cast<long long>(sh.rowStart[t.g]) + local_row;
             const float *sa_row = scale_a + grow * k_steps;
             const float *sw = p.scale_w + (static_cast<long long>(t.g) * n_tiles + t.nt) * k_steps;
@@ -401,16 +434,16 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
         return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.d)) & 15) return cudaErrorInvalidValue;
     if ((p.disp_flag || p.counts_flag) && (!p.counts || p.ranks <= 0)) return cudaErrorInvalidValue;
-    CUtensorMap mapA, mapW;
-    if (!nixl_gemm::makeTileMap(&mapA, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K)) ||
-        !nixl_gemm::makeTileMap(&mapW, p.w, static_cast<uint64_t>(p.groups) * p.N, static_cast<uint64_t>(p.K))) {
+    const uint64_t a_rows = static_cast<uint64_t>(p.a_rows), k_bytes = static_cast<uint64_t>(p.K);
+    CUtensorMap mapW, mapA, mapA32, mapA64; // A in boxes of 128, 32 and 64 rows
+    if (!nixl_gemm::makeTileMap(&mapW, p.w, static_cast<uint64_t>(p.groups) * p.N, k_bytes) || !nixl_gemm::makeTileMap(&mapA64, p.a, a_rows, k_bytes, 64)) {
         std::fprintf(stderr, "nixl_grouped_gemm_fp8_launch: cuTensorMapEncodeTiled failed\n");
         return cudaErrorInvalidValue;
     }
     // Tile shape: CTA pairs with 256 x 256 tiles when the experts have more rows than one 128-row tile on average and the
     // tiles are enough for the 74 pairs; single CTAs with 128 x 128 tiles otherwise (the expert-major low-latency layout,
     // where most tiles hold a handful of rows, and small products, which need every SM).  Measured, single / pair, us:
-    // 32 experts, N = K = 4096: 128 rows each 118 / 122, 200 rows 212 / 162, 512 rows 477 / 310; 16 experts, 512 x 2048:
+    // 32 experts, N = K = 4096: 128 rows each 116 / 122, 200 rows 210 / 162, 512 rows 477 / 310; 16 experts, 512 x 2048:
     // 256 rows (32 pair tiles) 14.8 / 18.7, 400 rows (50) 22.8 / 19.0; 1 expert, 4096 x 7168, 512 rows (32) 27.5 / 35.1.
     int mode = p.tile_mode & 0xff;
     if (mode == 0)
@@ -421,17 +454,16 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
     if (mode == 3) {
         if (p.N % 256 || p.K % 512 || p.counts_flag || p.disp_flag) return cudaErrorInvalidValue;
         if ((reinterpret_cast<uintptr_t>(p.scale_a) | reinterpret_cast<uintptr_t>(p.scale_w)) & 3) return cudaErrorInvalidValue;
-        CUtensorMap mapT; // that kernel loads token rows in boxes of 32
-        if (!nixl_gemm::makeTileMap(&mapT, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 32)) return cudaErrorInvalidValue;
-        return nixl_gemm::launchMxPairKernel(mapT, mapW, p, static_cast<cudaStream_t>(stream));
+        if (!nixl_gemm::makeTileMap(&mapA, p.a, a_rows, k_bytes) || !nixl_gemm::makeTileMap(&mapA32, p.a, a_rows, k_bytes, 32)) return cudaErrorInvalidValue;
+        return nixl_gemm::launchMxPairKernel(mapA, mapA32, mapA64, mapW, p, static_cast<cudaStream_t>(stream));
     }
     if (mode == 2) {
         if (p.N % 256) return cudaErrorInvalidValue;
-        CUtensorMap mapA64; // that kernel loads A in boxes of 64 rows
-        if (!nixl_gemm::makeTileMap(&mapA64, p.a, static_cast<uint64_t>(p.a_rows), static_cast<uint64_t>(p.K), 64)) return cudaErrorInvalidValue;
-        return nixl_gemm::launchPairKernel(mapA64, mapW, p, static_cast<cudaStream_t>(stream));
+        if (!nixl_gemm::makeTileMap(&mapA, p.a, a_rows, k_bytes)) return cudaErrorInvalidValue;
+        return nixl_gemm::launchPairKernel(mapA, mapA64, mapW, p, static_cast<cudaStream_t>(stream));
     }
-    const size_t smem = size_t(kStages) * kStageBytes + sizeof(Shared) + 1024;
+    if (!nixl_gemm::makeTileMap(&mapA, p.a, a_rows, k_bytes) || !nixl_gemm::makeTileMap(&mapA32, p.a, a_rows, k_bytes, 32)) return cudaErrorInvalidValue;
+    const size_t smem = size_t(kRingBytes) + kTailBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     {
@@ -448,6 +480,6 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
     // Upper bound of tiles (row counts live on the device): never launch more CTAs than that.
     const long long max_tiles = (static_cast<long long>(p.a_rows + BM - 1) / BM + p.groups) * (p.N / BN);
     if (grid > max_tiles) grid = static_cast<int>(max_tiles);
-    groupedGemmKernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mapA, mapW, p);
+    groupedGemmKernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mapA, mapA32, mapA64, mapW, p);
     return cudaGetLastError();
 }

@@ -25,8 +25,8 @@
 // reading the scales from shared memory, 4 bytes per lane and FMA, made a step twice as long.)
 //
 // Measured on one B200, back to back for half a second (that is, under the power cap), before / now: 31 experts that share
-// 16384 rows unevenly, 2048 x 7168: 423 / 351 us (1.37 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 844 / 718 us
-// (1.53 PFLOP/s); one expert, 8192 rows, 4096 x 7168: 311 / 266 us (1.81 PFLOP/s).
+// 16384 rows unevenly, 2048 x 7168: 423 / 349 us (1.38 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 844 / 713 us
+// (1.54 PFLOP/s); one expert, 8192 rows, 4096 x 7168: 311 / 262 us (1.84 PFLOP/s).
 //
 //   warp 0      TMA producer (both CTAs; completion bytes are counted on the even CTA's barrier)
 //   warp 1      MMA issuer (even CTA only); commits are multicast to both CTAs' barriers
@@ -237,7 +237,7 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA64, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
     Shared &sh = *reinterpret_cast<Shared *>(tiles + kStages * kStageBytes);
@@ -349,8 +349,7 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
                     if (cta == 0) mbarExpectTx(&sh.full[s], bytes);
                     const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
                     unsigned char *st = tiles + s * kStageBytes;
-                    tmaLoad2dPair(st, &mapA, ks * BK, row0, bar);
-                    if (rows_cta == BM) tmaLoad2dPair(st + kATileBytes / 2, &mapA, ks * BK, row0 + BM / 2, bar);
+                    tmaLoad2dPair(st, rows_cta == BM ? &mapA : &mapA64, ks * BK, row0, bar);
                     tmaLoad2dPair(st + kATileBytes, &mapW, ks * BK, wrow, bar);
                 }
             }
@@ -428,7 +427,7 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
 
 } // namespace
 
-cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
+cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapA64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
     const size_t smem = size_t(kStages) * kStageBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -465,5 +464,5 @@ cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorM
     const long long max_tiles = (static_cast<long long>(p.a_rows + 2 * BM - 1) / (2 * BM) + p.groups) * (p.N / BN);
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-    return cudaLaunchKernelEx(&cfg, groupedGemmPairKernel, mapA, mapW, p);
+    return cudaLaunchKernelEx(&cfg, groupedGemmPairKernel, mapA, mapA64, mapW, p);
 }

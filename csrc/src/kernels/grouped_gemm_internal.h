@@ -16,13 +16,13 @@ constexpr int kMaxGroups = 512;
 bool makeTileMap(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k, uint32_t box_rows = 128);
 
 // 256 x 256 tiles computed by CTA pairs (tcgen05 cta_group::2).  Same contract as the
-// single-CTA kernel; N must be a multiple of 256.  mapA: boxes of 64 rows, mapW: of 128.
-cudaError_t launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
+// single-CTA kernel; N must be a multiple of 256.  The maps of A have boxes of 128 and 64 rows, that of W 128.
+cudaError_t launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapA64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
 
 // Tiles of 256 columns x up to 256 tokens with power-of-two block scales applied by the tensor core (kind::mxf8f6f4.block_scale):
 // p.scale_a / p.scale_w point at exponent bytes (uint8 [a_rows][K/128] and [groups][N/128][K/128]);
-// K must be a multiple of 512, N of 256; no dispatch overlap.  mapT (tokens): boxes of 32 rows, mapW: of 128.
-cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
+// K must be a multiple of 512, N of 256; no dispatch overlap.  The maps of the tokens have boxes of 128, 32 and 64 rows.
+cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
 
 } // namespace nixl_gemm
 

@@ -35,8 +35,8 @@
 // 697 cycles of which the MMAs need 512.  What is left is mostly the traffic into shared memory (64 of 128 bytes per cycle
 // at full rate, beside the operands' reads).  Measured on one B200 back to back for half a second, before (tokens on the
 // M side, eight N = 128 MMAs per step, scale copies every 512 channels) / now: 31 experts that share 16384 rows unevenly,
-// 2048 x 7168: 335 / 278 us (1.73 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 659 / 573 us (1.92 PFLOP/s); one
-// expert, 8192 rows, 4096 x 7168: 239 / 209 us (2.30 PFLOP/s); 32 experts, 1024 rows, 2048 x 7168: 130 / 97 us.
+// 2048 x 7168: 335 / 277 us (1.74 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 659 / 562 us (1.96 PFLOP/s); one
+// expert, 8192 rows, 4096 x 7168: 239 / 200 us (2.41 PFLOP/s); 32 experts, 1024 rows, 2048 x 7168: 130 / 97 us.
 //
 // TMA loads read this GPU's memory only and carry no cluster multicast.  Every wait is bounded.
 #include <cuda.h>
@@ -54,12 +54,10 @@ using nixl_gemm::kMaxGroups;
 
 constexpr int BW = 128;        // W rows per CTA (256 per pair): the MMA's M side
 constexpr int BT = 256;        // tokens per tile at most: its N side, half of them from either CTA
-constexpr int TBOX = 32;       // token rows per TMA box
 constexpr int BK = 128;
 constexpr int kStages = 6;
 constexpr int kThreads = 384;
 constexpr int kWTileBytes = BW * BK;
-constexpr int kTBoxBytes = TBOX * BK;
 constexpr int kStageBytes = kWTileBytes + BT / 2 * BK; // 32 KiB per CTA
 constexpr int kChunkSteps = 4;                 // steps whose scale bytes share one 32-bit word
 constexpr int kGroupChunks = 8;                // chunks copied to TMEM in one go
@@ -189,7 +187,8 @@ __device__ __forceinline__ bool tileAt(const Shared &sh, int groups, int n_tiles
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_constant__ CUtensorMap mapT32, const __grid_constant__ CUtensorMap mapT64,
+                        const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
     unsigned char *sf_ring = tiles + kStages * kStageBytes; // two buffers of kGroupChunks chunks' layouts
@@ -252,8 +251,10 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
             const int half = sh.tileRows[t.g] / 2; // tokens of this CTA
             const int row0 = sh.rowStart[t.g] + t.mt * (2 * half) + static_cast<int>(cta) * half;
             const int wrow = t.g * p.N + t.nt * (2 * BW) + static_cast<int>(cta) * BW;
-            const int boxes = (half + TBOX - 1) / TBOX;
-            const uint32_t bytes = static_cast<uint32_t>(2 * (kWTileBytes + boxes * kTBoxBytes)); // both CTAs' shares
+            // One TMA box of 32, 64 or 128 token rows: an instruction more per step costs more than the rows it would save.
+            const int box = half <= 32 ? 32 : half <= 64 ? 64 : BT / 2;
+            const CUtensorMap *map = box == 32 ? &mapT32 : box == 64 ? &mapT64 : &mapT;
+            const uint32_t bytes = static_cast<uint32_t>(2 * (kWTileBytes + box * BK)); // both CTAs' shares
             for (int ks = 0; ks < k_steps; ++ks, ++it) {
                 const int s = it % kStages;
                 if (!mbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, abort_flag)) goto producer_done;
@@ -261,7 +262,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
                 const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
                 unsigned char *st = tiles + s * kStageBytes;
                 tmaLoad2dPair(st, &mapW, ks * BK, wrow, bar);
-                for (int b = 0; b < boxes; ++b) tmaLoad2dPair(st + kWTileBytes + b * kTBoxBytes, &mapT, ks * BK, row0 + b * TBOX, bar);
+                tmaLoad2dPair(st + kWTileBytes, map, ks * BK, row0, bar);
             }
         }
     producer_done:;
@@ -438,7 +439,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
 
 } // namespace
 
-cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
+cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
     const size_t smem = size_t(kStages) * kStageBytes + size_t(2) * kSfBufBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -474,5 +475,5 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtenso
     const long long max_tiles = (static_cast<long long>(p.a_rows + BT - 1) / BT + p.groups) * (p.N / (2 * BW));
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapW, p);
+    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapT32, mapT64, mapW, p);
 }

@@ -82,3 +82,14 @@ def test_either_side_of_the_tile_shape_rule(groups, rows, N):
     grouped_gemm_fp8(a, sa, w, sw, rs, rc, out=out)
     torch.cuda.synchronize()
     _check(out, a, sa, w, sw, rs, rc, K)
+
+
+@pytest.mark.parametrize("counts", [[1, 32], [33, 7, 0], [64, 64, 64], [65, 1], [128, 32, 33], [129, 31, 256]])  # the fullest expert sets the stages
+@pytest.mark.parametrize("N,K", [(128, 128), (384, 1664)])
+def test_single_cta_tiles(counts, N, K):
+    a, sa, w, sw, rs, rc = _inputs(counts, N, K, 4)
+    out = torch.full((a.shape[0], N), 5.0, dtype=torch.bfloat16, device=a.device)
+    grouped_gemm_fp8(a, sa, w, sw, rs, rc, out=out, tile_mode=1)
+    torch.cuda.synchronize()
+    assert int(out._nixl_status.item()) == 0
+    _check(out, a, sa, w, sw, rs, rc, K)
