@@ -184,10 +184,12 @@ __device__ __forceinline__ uint4 quantGroup(const uint4 &lo, const uint4 &hi, bo
 // through its own flags.
 // Measured on one B200, one rank, 32 experts, top-8, before / now: 4096 tokens x 7168 bf16 131 / 113 us (528 MB, 4.7 TB/s; the
 // rows written, 470 MB, are the bound), fp8 97 / 73 us, 4096 x 4096 fp8 74 / 47 us (3.6 TB/s); 128 tokens x 7168 fp8, low-latency
-// layout 21.6 / 13.4 us; 1 token 20.5 / 11.9 us.
+// layout 21.6 / 13.4 us (8.4 with fixed places); 1 token 20.5 / 11.9 us (7.8).
 constexpr int kBatch = 32;  // tokens whose rows are looked up together, and reported as sent together
 constexpr int kSlices = 2;  // slices of a token in flight per warp: 2 KiB
 constexpr int kDispatchCtas = 4; // per SM, with many tokens
+
+__host__ __device__ __forceinline__ bool placesAreFixed(const NixlEpDispatchParams &p) { return p.R == 1 && p.rows_per_expert > 0 && p.phases == 3; }
 
 template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpDispatchParams &p, const int *rows, const unsigned char *dests, char *const *peer_sh,
                                                                    long long t0, int n_tokens, int parts) {
@@ -305,6 +307,10 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         peer_sh[tid] = peerBase(p.peers, tid);
         masked[tid] = ldVolatile(p.scr.mask + tid);
     }
+    // One rank, low-latency layout, send and receive in one launch: a row's place is known without anybody's counts (expert e
+    // starts at e * rows_per_expert, the CTA's share at what its atomic returned), so nothing is waited for; the last CTA
+    // out publishes the counts.  13.4 -> 8.4 us for 128 tokens x 7168, 11.9 -> 7.8 us for one token.
+    const bool fixed = placesAreFixed(p);
     const long long t_first = static_cast<long long>(p.T) * blockIdx.x / gridDim.x, t_end = static_cast<long long>(p.T) * (blockIdx.x + 1) / gridDim.x;
 
     if (p.phases & 1) {
@@ -316,7 +322,13 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             if (e >= 0 && e < p.E && masked[static_cast<int>(e) / El] == 0) atomicAdd(mine + e, 1);
         }
         __syncthreads();
-        for (int e = tid; e < p.E; e += kThreads) place[e] = mine[e] ? atomicAdd(p.scr.cnt + e, mine[e]) : 0;
+        for (int e = tid; e < p.E; e += kThreads) {
+            place[e] = mine[e] ? atomicAdd(p.scr.cnt + e, mine[e]) : 0;
+            if (fixed) ebase[e] = e * p.rows_per_expert;
+        }
+        if (fixed) __syncthreads();
+    }
+    if ((p.phases & 1) && !fixed) {
         gridBarrier(p.scr.barrier, p.scr.status, p.timeout_ns);
         for (int e = tid; e < p.E; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
         __syncthreads();
@@ -337,69 +349,71 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         }
     }
 
+    const bool alone = p.R == 1;
     // 3. wait for everybody's counts (every CTA looks for itself: 8 flags, no grid barrier needed)
     //    A group of one rank has them already: its own, from the grid barrier (or from the send phase's launch).
-    const uint64_t *cflag = reinterpret_cast<const uint64_t *>(self + p.lay.off_counts_flag);
-    const bool alone = p.R == 1;
-    if (tid < p.R) {
-        if (masked[tid] == 0 && peer_sh[tid] != nullptr) {
-            if (!alone && !waitFlag(cflag + tid, p.epoch, p.timeout_ns)) {
+    if (!fixed) {
+        const uint64_t *cflag = reinterpret_cast<const uint64_t *>(self + p.lay.off_counts_flag);
+        if (tid < p.R) {
+            if (masked[tid] == 0 && peer_sh[tid] != nullptr) {
+                if (!alone && !waitFlag(cflag + tid, p.epoch, p.timeout_ns)) {
+                    atomicExch(p.scr.mask + tid, 1);
+                    atomicOr(p.scr.status, ST_PEER_TIMEOUT);
+                }
+            } else if (peer_sh[tid] == nullptr) {
                 atomicExch(p.scr.mask + tid, 1);
-                atomicOr(p.scr.status, ST_PEER_TIMEOUT);
             }
-        } else if (peer_sh[tid] == nullptr) {
-            atomicExch(p.scr.mask + tid, 1);
+            if (!alone) masked[tid] = ldVolatile(p.scr.mask + tid);
         }
-        if (!alone) masked[tid] = ldVolatile(p.scr.mask + tid);
-    }
-    __syncthreads();
-
-    // 4. placement tables.  counts[r][e] is the local copy of the all-gather.
-    const int *counts = reinterpret_cast<const int *>(self + p.lay.off_counts);
-    const bool own = alone && (p.phases & 1); // the counts are in shared memory
-    for (int e = tid; e < p.E; e += kThreads) {
-        int b = 0, all = 0;
-        for (int r = 0; r < p.R; ++r) {
-            const int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e); // (loads of all ranks in flight together)
-            if (masked[r] != 0) continue;
-            if (r < p.rank) b += c;
-            all += c;
-        }
-        if (p.phases & 1) place[e] += b;
-        ebase[e] = all; // totals first, turned into per-rank prefixes below
-    }
-    __syncthreads();
-    if (p.rows_per_expert > 0) {
-        for (int e = tid; e < p.E; e += kThreads)
-            if (ebase[e] > p.rows_per_expert) atomicOr(p.scr.status, ST_CAPACITY);
         __syncthreads();
-        for (int e = tid; e < p.E; e += kThreads) ebase[e] = (e % El) * p.rows_per_expert;
-    } else if (tid < p.R) {
-        // exclusive prefix over the local experts of destination rank `tid`
-        int run = 0;
-        for (int le = 0; le < El; ++le) {
-            const int c = ebase[tid * El + le];
-            ebase[tid * El + le] = run;
-            run += c;
-        }
-        if (run > p.cap) atomicOr(p.scr.status, ST_CAPACITY);
-    }
-    __syncthreads();
 
-    // Receiver-side bookkeeping is known as soon as the counts are: CTA 0 publishes it.
-    if (blockIdx.x == 0 && (p.phases & 6)) {
-        for (int le = tid; le < El; le += kThreads) {
-            const int e = p.rank * El + le;
-            int all = 0;
+        // 4. placement tables.  counts[r][e] is the local copy of the all-gather.
+        const int *counts = reinterpret_cast<const int *>(self + p.lay.off_counts);
+        const bool own = alone && (p.phases & 1); // the counts are in shared memory
+        for (int e = tid; e < p.E; e += kThreads) {
+            int b = 0, all = 0;
             for (int r = 0; r < p.R; ++r) {
-                int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e);
-                if (masked[r] != 0) c = 0;
-                p.layout_range[static_cast<long long>(le) * p.R + r] = (static_cast<long long>(all) << 32) | static_cast<unsigned>(c);
+                const int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e); // (loads of all ranks in flight together)
+                if (masked[r] != 0) continue;
+                if (r < p.rank) b += c;
                 all += c;
             }
-            p.recv_count[le] = all;
-            p.expert_offsets[le] = ebase[e];
-            if (le == El - 1) p.expert_offsets[El] = ebase[e] + (p.rows_per_expert > 0 ? p.rows_per_expert : all);
+            if (p.phases & 1) place[e] += b;
+            ebase[e] = all; // totals first, turned into per-rank prefixes below
+        }
+        __syncthreads();
+        if (p.rows_per_expert > 0) {
+            for (int e = tid; e < p.E; e += kThreads)
+                if (ebase[e] > p.rows_per_expert) atomicOr(p.scr.status, ST_CAPACITY);
+            __syncthreads();
+            for (int e = tid; e < p.E; e += kThreads) ebase[e] = (e % El) * p.rows_per_expert;
+        } else if (tid < p.R) {
+            // exclusive prefix over the local experts of destination rank `tid`
+            int run = 0;
+            for (int le = 0; le < El; ++le) {
+                const int c = ebase[tid * El + le];
+                ebase[tid * El + le] = run;
+                run += c;
+            }
+            if (run > p.cap) atomicOr(p.scr.status, ST_CAPACITY);
+        }
+        __syncthreads();
+
+        // Receiver-side bookkeeping is known as soon as the counts are: CTA 0 publishes it.
+        if (blockIdx.x == 0 && (p.phases & 6)) {
+            for (int le = tid; le < El; le += kThreads) {
+                const int e = p.rank * El + le;
+                int all = 0;
+                for (int r = 0; r < p.R; ++r) {
+                    int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e);
+                    if (masked[r] != 0) c = 0;
+                    p.layout_range[static_cast<long long>(le) * p.R + r] = (static_cast<long long>(all) << 32) | static_cast<unsigned>(c);
+                    all += c;
+                }
+                p.recv_count[le] = all;
+                p.expert_offsets[le] = ebase[e];
+                if (le == El - 1) p.expert_offsets[El] = ebase[e] + (p.rows_per_expert > 0 ? p.rows_per_expert : all);
+            }
         }
     }
 
@@ -432,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             else dispatchTokens<false>(p, rows, dests, peer_sh, tb, n, parts);
             __syncthreads(); // all stores of the batch issued (and its tables free for the next one)
             // Count the batch's rows as sent.  Whoever completes an expert's rows raises that expert's arrival flag at its rank.
-            for (int e = tid; e < p.E; e += kThreads) {
+            for (int e = tid; e < p.E && !fixed; e += kThreads) {
                 const int c = mine[e];
                 if (c == 0) continue;
                 // One operation releases this CTA's rows and acquires the other CTAs'.
@@ -466,6 +480,25 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             if (last) p.scr.barrier[2] = 0;
         }
         __syncthreads();
+        if (last && fixed) {
+            __threadfence(); // the other CTAs' counts
+            int *counts = reinterpret_cast<int *>(self + p.lay.off_counts);
+            uint64_t *dflag = reinterpret_cast<uint64_t *>(self + p.lay.off_disp_flag);
+            for (int e = tid; e < p.E; e += kThreads) {
+                const int c = ldVolatile(p.scr.cnt + e);
+                if (c > p.rows_per_expert) atomicOr(p.scr.status, ST_CAPACITY);
+                counts[e] = c;
+                p.recv_count[e] = c;
+                p.layout_range[e] = static_cast<unsigned>(c);
+                p.expert_offsets[e] = ebase[e];
+                if (e == p.E - 1) p.expert_offsets[p.E] = ebase[e] + p.rows_per_expert;
+                dflag[e] = p.epoch; // (every reader is a later launch)
+            }
+            if (tid == 0) {
+                reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
+                *reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag) = p.epoch;
+            }
+        }
         if (last)
             for (int e = tid; e < p.E; e += kThreads) {
                 p.scr.cnt[e] = 0;
@@ -1062,8 +1095,42 @@ __device__ __forceinline__ void localRows(int n, const uint4 *const (&src)[NR], 
     }
 }
 
+// The same for rows in the logarithmic format: each row is coded and decoded in registers, as it would be on its way out
+// and in, so the result is what the coded path gives.  Slices of 512 channels, 16 per lane.
 template <int NR>
-__global__ void __launch_bounds__(kThreads, NR <= 8 ? 3 : 2) epCombineLocal(const __grid_constant__ NixlEpCombineParams p, int parts) {
+__device__ __forceinline__ void localRowsCoded(int n, const uint4 *const (&src)[NR], const float (&w)[NR], uint4 *dst, int slices, int first, int step, int lane) {
+    for (int b = first; b < slices; b += step) {
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        const int at = b * 64 + lane * 2;
+        uint4 lo = ldNc(src[0] + at), hi = ldNc(src[0] + at + 1);
+#pragma unroll
+        for (int k = 0; k < NR; ++k) {
+            if (k >= n) break;
+            uint4 nlo = lo, nhi = hi;
+            if (k + 1 < NR && k + 1 < n) { // the next row's loads fly while this one is coded
+                nlo = ldNc(src[k + 1 < NR ? k + 1 : k] + at);
+                nhi = ldNc(src[k + 1 < NR ? k + 1 : k] + at + 1);
+            }
+            uint32_t code[5];
+            uint2 meta;
+            logfmtEncode16(lo, hi, code, meta);
+            logfmtDecodeAdd16(code, meta, w[k], acc);
+            lo = nlo;
+            hi = nhi;
+        }
+        uint4 o[2];
+        __nv_bfloat162 *oh = reinterpret_cast<__nv_bfloat162 *>(o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) oh[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+        stPeer16(dst + at, o[0]);
+        stPeer16(dst + at + 1, o[1]);
+    }
+}
+
+template <int NR, bool kCoded>
+__global__ void __launch_bounds__(kThreads, NR <= 8 && !kCoded ? 3 : 2) epCombineLocal(const __grid_constant__ NixlEpCombineParams p, int parts) {
     const int lane = threadIdx.x & 31;
     const int vecs = p.H / 8;
     const char *self = peerBase(p.peers, p.rank);
@@ -1101,7 +1168,9 @@ __global__ void __launch_bounds__(kThreads, NR <= 8 ? 3 : 2) epCombineLocal(cons
             src[k] = reinterpret_cast<const uint4 *>(x + static_cast<long long>(__shfl_sync(0xffffffffu, row, from)) * p.H);
             w[k] = __shfl_sync(0xffffffffu, weight, from);
         }
-        localRows<NR>(n, src, w, reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(p.out) + t * p.H), vecs, part * 32 + lane, 32 * parts);
+        uint4 *dst = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(p.out) + t * p.H);
+        if (!kCoded || n == 0) localRows<NR>(n, src, w, dst, vecs, part * 32 + lane, 32 * parts);
+        else localRowsCoded<NR>(n, src, w, dst, p.H / 512, part, parts, lane);
     }
 }
 
@@ -1189,10 +1258,14 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        // (CTAs without a token would only add to the barrier and the exit count; the ranks' counts are spread over CTAs.)
         if (p.T >= 4 * sms) requested = kDispatchCtas * sms;
+        else if (p.T < sms) requested = p.T > p.R ? p.T : p.R;
     }
     const int grid = coopGrid(reinterpret_cast<const void *>(epDispatchKernel), requested, smem);
     void *args[] = {const_cast<NixlEpDispatchParams *>(params)};
+    if (placesAreFixed(p)) // no CTA waits for another
+        return cudaLaunchKernel(reinterpret_cast<const void *>(epDispatchKernel), dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(epDispatchKernel), dim3(grid), dim3(kThreads), args, smem,
                                        static_cast<cudaStream_t>(stream));
 }
@@ -1207,19 +1280,28 @@ extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *s
         p.E / p.R > kMaxRanks * 8 || p.rank < 0 || p.rank >= p.R)
         return cudaErrorInvalidValue;
     void *args[] = {const_cast<NixlEpCombineParams *>(params)};
-    if (p.R == 1 && !p.use_logfmt && p.x && p.topk_weights && p.out && (p.pull == 2 || p.send_row)) {
+    if (p.R == 1 && p.x && p.topk_weights && p.out && (p.pull == 2 || p.send_row)) {
         if (!(p.phases & 1) || p.T <= 0) return cudaSuccess; // all of it happens in the send phase
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        // Three CTAs per SM; parts so that every warp has about four items, or as many as a token has slices of 512 bytes.
+        // Three CTAs per SM; parts so that every warp has about four items, or as many as a token has slices (512 bytes; coded
+        // rows 512 channels, whose coding is a long chain of arithmetic per warp).
         const int ctas = p.grid > 0 ? (p.pull == 2 ? 2 : 1) * p.grid : 3 * sms;
-        int parts = 1;
-        while (parts < 16 && 2 * parts * 256 <= p.H && static_cast<long long>(p.T) * parts < 4LL * ctas * (kThreads / 32)) parts <<= 1;
+        const long long items = 4LL * ctas * (kThreads / 32);
+        const int most = p.use_logfmt ? p.H / 512 : p.H / 256;
+        int parts = static_cast<int>(items / p.T < 16 ? items / p.T : 16);
+        parts = parts < 1 ? 1 : parts > most ? (most > 0 ? most : 1) : parts;
         const long long want = static_cast<long long>(p.T) * parts;
         const int grid = static_cast<int>(want < ctas ? want : ctas);
-        if (p.K <= 8) epCombineLocal<8><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p, parts);
-        else epCombineLocal<kMaxTopk><<<grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(p, parts);
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        if (p.K <= 8) {
+            if (p.use_logfmt) epCombineLocal<8, true><<<grid, kThreads, 0, st>>>(p, parts);
+            else epCombineLocal<8, false><<<grid, kThreads, 0, st>>>(p, parts);
+        } else {
+            if (p.use_logfmt) epCombineLocal<kMaxTopk, true><<<grid, kThreads, 0, st>>>(p, parts);
+            else epCombineLocal<kMaxTopk, false><<<grid, kThreads, 0, st>>>(p, parts);
+        }
         return cudaGetLastError();
     }
     if (p.pull == 2) {
