@@ -104,6 +104,23 @@ bool allocationRange(uintptr_t ptr, uintptr_t &base, size_t &size) {
     return true;
 }
 
+// Device address of host memory that is pinned from end to end already, 0 otherwise.  Looked at every 2 MiB, so that a
+// range that merely starts and ends in pinned memory is not taken for one.
+uintptr_t pinnedRange(uintptr_t addr, size_t len) {
+    uintptr_t first = 0;
+    for (size_t off = 0;; off = std::min(off + (size_t(2) << 20), len - 1)) {
+        cudaPointerAttributes attr{};
+        if (cudaPointerGetAttributes(&attr, reinterpret_cast<void *>(addr + off)) != cudaSuccess || attr.type != cudaMemoryTypeHost || !attr.devicePointer) {
+            cudaGetLastError();
+            return 0;
+        }
+        const uintptr_t dp = reinterpret_cast<uintptr_t>(attr.devicePointer);
+        if (off == 0) first = dp;
+        else if (dp != first + off) return 0;
+        if (off == len - 1) return first;
+    }
+}
+
 // UUID of a local GPU, looked up once per ordinal.
 struct GpuUuid {
     unsigned char b[16];
@@ -561,9 +578,15 @@ nixl_status_t Engine::registerMem(const nixlBlobDesc &mem, const nixl_mem_t &nix
         if (cuda_ && pinDram_) {
             const int dev = primaryDevice_.load() >= 0 ? primaryDevice_.load() : 0;
             DeviceScope ds(dev);
-            cudaError_t e = cudaHostRegister(reinterpret_cast<void *>(mem.addr), mem.len, cudaHostRegisterPortable | cudaHostRegisterMapped);
+            // Memory that its owner allocated pinned (cudaHostAlloc, torch's pin_memory) cannot be registered again, and need not be.
+            md->devVisible = pinnedRange(mem.addr, mem.len);
+            md->pinnedByOwner = md->devVisible != 0;
+            const cudaError_t e = md->devVisible ? cudaErrorHostMemoryAlreadyRegistered
+                                                 : cudaHostRegister(reinterpret_cast<void *>(mem.addr), mem.len, cudaHostRegisterPortable | cudaHostRegisterMapped);
             if (e == cudaSuccess) md->pinnedByUs = true;
-            if (e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered) {
+            if (md->devVisible) {
+                // found above
+            } else if (e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered) {
                 cudaGetLastError();
                 void *dp = nullptr;
                 if (cudaHostGetDevicePointer(&dp, reinterpret_cast<void *>(mem.addr), 0) == cudaSuccess)
@@ -897,7 +920,11 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
             continue;
         }
         if (!cuda_) return fail(NIXL_ERR_NOT_SUPPORTED);
-        if (lvis && rvis) { // the copy kernel can see both ends
+        // Host memory that its owner pinned: the copy engines move a long descriptor at 53 - 56 GB/s, the kernel at 50, but a copy
+        // per descriptor costs 4 to 5 us.  Measured, kernel / copies: 256 x 4 KiB 31 / 990 us, 16 x 64 KiB 31 / 85 us, 16 x 1 MiB
+        // 340 / 378 us; 16 x 4 MiB 1.34 / 1.29 ms; a single 64 KiB 8.5 / 13 us, a single 256 KiB 20 / 17 us.
+        const bool by_copy = l->pinnedByOwner && len >= (local.descCount() == 1 ? size_t(128) << 10 : size_t(4) << 20);
+        if (lvis && rvis && !by_copy) { // the copy kernel can see both ends
             int dev;
             if (l->mem == VRAM_SEG) dev = l->device;
             else dev = r->sameProcess ? r->ownerDevice : r->mapDevice;
@@ -926,7 +953,7 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
             else list.push_back({d, klass});
             continue;
         }
-        // One end is pageable host memory: let the runtime stage it.
+        // One end is pageable host memory, which the runtime stages, or a long piece of pinned memory.
         if (l->mem == DRAM_SEG && rvis) {
             const int dev = r->sameProcess ? r->ownerDevice : r->mapDevice;
             if (operation == NIXL_WRITE) req->asyncCopies.push_back({reinterpret_cast<void *>(rvis), reinterpret_cast<void *>(laddr), len, dev});

@@ -76,9 +76,10 @@ class KVBlockTransfer:
         for b in blocks:
             if not 0 <= b < per_tensor:
                 raise IndexError(f"block {b} outside 0..{per_tensor - 1}")
-        if not len(blocks) or self.tensors * per_tensor > 0x7FFFFFFF:
+        if self.tensors * len(blocks) <= 48 or self.tensors * per_tensor > 0x7FFFFFFF:
             return [t * per_tensor + int(b) for t in range(self.tensors) for b in blocks]
-        # tensor-major, as an array: 64 tensors x 32 blocks take 10 us this way, 100 us as a Python list (and as much again to convert it)
+        # tensor-major, as an array: 64 tensors x 32 blocks take 6 us this way, 100 us as a Python list and half as much again to
+        # convert it; up to some 48 entries the list is the cheaper one (2 x 1: 20 against 22.5 us per request)
         first = np.arange(self.tensors, dtype=np.int32) * per_tensor
         return (first[:, None] + np.array([int(b) for b in blocks], dtype=np.int32)).reshape(-1)
 

@@ -84,3 +84,48 @@ def test_either_side_of_the_request_size_rule():
         size = (16 << 20) + extra // 4
         at = [i * (size + 256) for i in range(4)]
         _move(f"cpr{extra}", [size] * 4, at, at[::-1], {})
+
+
+@pytest.mark.parametrize("op", ["WRITE", "READ"])
+@pytest.mark.parametrize("pinned", [True, False])
+@pytest.mark.parametrize(
+    "lens",
+    [[4096], [(128 << 10) - 1], [128 << 10], [1, 63, 4097, 70000], [(4 << 20) - 1, 4 << 20, 5, (4 << 20) + 3], [333] * 300],
+)
+def test_host_memory_either_side_of_the_copy_engine_rule(op, pinned, lens):
+    """Host memory pinned by its owner (short pieces by the kernel, long or single ones by copies) or by the registration."""
+    tag = f"cph{op}{int(pinned)}{len(lens)}_{lens[0]}"
+    cfg = nixl_agent_config(enable_prog_thread=False, backends=["NVLINK"])
+    a, b = nixl_agent(f"{tag}_a", cfg), nixl_agent(f"{tag}_b", cfg)
+    lens = np.asarray(lens, dtype=np.int64)
+    at = [np.array(_place(lens, [o] * len(lens))) for o in (3, 16)]
+    size = [int((x + lens).max()) + 64 for x in at]
+    host = torch.randint(0, 256, (size[0],), dtype=torch.uint8)
+    host = host.pin_memory() if pinned else host
+    dev = torch.randint(0, 256, (size[1],), dtype=torch.uint8, device="cuda:0")
+    want_h, want_d = host.numpy().copy(), dev.cpu().numpy()
+    for n, h, d in zip(lens, *at):
+        if op == "WRITE":
+            want_d[d : d + n] = want_h[h : h + n]
+        else:
+            want_h[h : h + n] = want_d[d : d + n]
+    ra, rb = a.register_memory(host), b.register_memory(dev)
+    a.add_remote_agent(b.get_agent_metadata())
+    ends = [a.get_xfer_descs(np.stack([t.data_ptr() + x, lens, np.zeros_like(lens)], axis=1).astype(np.uint64), m) for t, x, m in ((host, at[0], "DRAM"), (dev, at[1], "VRAM"))]
+    h = a.initialize_xfer(op, ends[0], ends[1], b.name, b"there")
+    for _ in range(2):
+        state = a.transfer(h)
+        while state == "PROC":
+            state = a.check_xfer_state(h)
+        assert state == "DONE"
+    torch.cuda.synchronize()
+    assert np.array_equal(host.numpy(), want_h) and np.array_equal(dev.cpu().numpy(), want_d)
+    seen = 0
+    for _ in range(100000):
+        seen += len(b.get_new_notifs().get(a.name, []))
+        if seen == 2:
+            break
+    assert seen == 2  # every post delivers its message
+    a.release_xfer_handle(h)
+    a.deregister_memory(ra)
+    b.deregister_memory(rb)
