@@ -36,8 +36,7 @@ struct FastDiv {
     __device__ __forceinline__ uint32_t quot(uint32_t n) const { return (__umulhi(n, m) + n) >> s; }
 };
 inline FastDiv fastDiv(uint32_t d) {
-    uint32_t s = 0;
-    while ((uint64_t(1) << s) < d) ++s;
+    const uint32_t s = d > 1 ? 32 - __builtin_clz(d - 1) : 0; // ceil(log2 d)
     return {d, static_cast<uint32_t>((((uint64_t(1) << s) - d) << 32) / d + 1), s};
 }
 
@@ -250,16 +249,25 @@ __device__ __forceinline__ void signalWhenAllDone(const NixlKvXferParams &p, uns
     }
 }
 
-// Grid for a request: `wanted` (0 = four CTAs per SM of the current device, what is resident at once), never more than there are steps.
+// Grid for a request: `wanted`, or by default four CTAs per SM of the current device, what is resident at once, and twice as
+// many when every warp has sixteen steps or more (the second half then starts staggered: 72 tensors x 195 blocks of 16 KiB
+// 78.9 us against 83.6, 72 x 164 of 24 KiB 100 against 107; 48 x 61 of 16 KiB, five steps per warp, 20.6 against 18.7).
+// Never more than there are steps for: CTAs without any would only lengthen the completion count.
 inline int gridFor(const KvPlan &k, int device) {
+    static int sm_count[64] = {}; // per device, looked up once (this is the post path)
     int grid = k.p.grid;
-    if (grid <= 0) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        grid = sms * 4;
-    }
     const long long want = (k.slots + kSlots - 1) / kSlots;
-    return grid > want ? static_cast<int>(want) : grid;
+    if (grid <= 0) {
+        int sms = device >= 0 && device < 64 ? sm_count[device] : 0;
+        if (sms <= 0) {
+            if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
+            if (device >= 0 && device < 64) sm_count[device] = sms;
+        }
+        grid = sms * 4;
+        if (want >= 16LL * grid * (kKvThreads / 32)) grid *= 2;
+    }
+    const long long most = (want + kKvThreads / 32 - 1) / (kKvThreads / 32);
+    return grid > most ? static_cast<int>(most) : grid;
 }
 
 // Shape and alignment checks common to both entry points; cudaSuccess when the request is well formed.

@@ -28,6 +28,19 @@ class _Params(ctypes.Structure):
     ]
 
 
+_fn = None
+
+
+def _launcher():
+    global _fn
+    if _fn is None:
+        fn = _lib.lib().nixl_grouped_gemm_fp8_launch
+        fn.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p]
+        fn.restype = ctypes.c_int
+        _fn = fn
+    return _fn
+
+
 def quantize_weights(w: torch.Tensor):
     """bf16/fp32 ``[G, N, K]`` -> (e4m3 ``[G, N, K]``, fp32 scales ``[G, N/128, K/128]``), 128x128 blocks."""
     G, N, K = w.shape
@@ -88,22 +101,17 @@ def grouped_gemm_mxfp8(a: torch.Tensor, scale_a: torch.Tensor, w: torch.Tensor, 
         if not t.is_contiguous():
             raise ValueError("inputs must be contiguous")
     dev = a.device
-    with torch.cuda.device(dev):
-        if out is None:
-            out = torch.empty(rows, N, dtype=torch.bfloat16, device=dev)
-        if status is None:
-            status = torch.zeros(1, dtype=torch.int32, device=dev)
+    if out is None:
+        out = torch.empty(rows, N, dtype=torch.bfloat16, device=dev)
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
     p = _Params()
     p.a, p.scale_a, p.w, p.scale_w, p.d = a.data_ptr(), scale_a.data_ptr(), w.data_ptr(), scale_w.data_ptr(), out.data_ptr()
     p.row_start, p.row_count = row_start.data_ptr(), row_count.data_ptr()
     p.groups, p.N, p.K, p.a_rows, p.grid = G, N, K, rows, grid
     p.tile_mode = 3
     p.status = status.data_ptr()
-    fn = _lib.lib().nixl_grouped_gemm_fp8_launch
-    fn.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p]
-    fn.restype = ctypes.c_int
-    with torch.cuda.device(dev):
-        _lib.check(fn(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)), "nixl_grouped_gemm_fp8_launch (block-scaled)")
+    _lib.launch_on(dev, _launcher(), ctypes.byref(p), _lib.raw_stream(dev), "nixl_grouped_gemm_fp8_launch (block-scaled)")
     out._nixl_status = status
     return out
 
@@ -149,11 +157,10 @@ def grouped_gemm_fp8(
     if row_start.dtype != torch.int32 or row_count.dtype != torch.int32:
         raise TypeError("row_start / row_count must be int32")
     dev = a.device
-    with torch.cuda.device(dev):
-        if out is None:
-            out = torch.empty(rows, N, dtype=torch.bfloat16, device=dev)
-        if status is None:
-            status = torch.zeros(1, dtype=torch.int32, device=dev)
+    if out is None:
+        out = torch.empty(rows, N, dtype=torch.bfloat16, device=dev)
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
     p = _Params()
     p.a, p.scale_a, p.w, p.scale_w, p.d = a.data_ptr(), scale_a.data_ptr(), w.data_ptr(), scale_w.data_ptr(), out.data_ptr()
     p.row_start, p.row_count = row_start.data_ptr(), row_count.data_ptr()
@@ -172,11 +179,7 @@ def grouped_gemm_fp8(
             # The dispatch runs on another stream right now: the kernel derives the row ranges itself.
             p.counts_flag = base + lay.off_counts_flag
             p.rows_per_expert = rows_per_expert
-    fn = _lib.lib().nixl_grouped_gemm_fp8_launch
-    fn.argtypes = [ctypes.POINTER(_Params), ctypes.c_void_p]
-    fn.restype = ctypes.c_int
-    with torch.cuda.device(dev):
-        _lib.check(fn(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)), "nixl_grouped_gemm_fp8_launch")
+    _lib.launch_on(dev, _launcher(), ctypes.byref(p), _lib.raw_stream(dev), "nixl_grouped_gemm_fp8_launch")
     out._nixl_status = status  # keeps the status word alive with the result
     return out
 

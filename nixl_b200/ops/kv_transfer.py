@@ -171,9 +171,8 @@ class KVTransfer:
         p.n_pairs = src_blocks.numel()
         p.done_signal, p.done_value = done_signal_ptr, done_value
         p.host_seq = self._seq
-        s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        with torch.cuda.device(self.device):
-            _lib.check(self._launch(ctypes.byref(p), ctypes.c_void_p(s.cuda_stream)), "nixl_kv_xfer_launch")
+        s = ctypes.c_void_p(stream.cuda_stream) if stream is not None else _lib.raw_stream(self.device)
+        _lib.launch_on(self.device, self._launch, ctypes.byref(p), s, "nixl_kv_xfer_launch")
         return self._seq
 
     def done(self, ticket: int) -> bool:

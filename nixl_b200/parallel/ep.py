@@ -38,24 +38,6 @@ def _up(x: int, a: int = _ALIGN) -> int:
     return (x + a - 1) // a * a
 
 
-def _raw_stream(device: torch.device) -> int:
-    """The current stream's ``cudaStream_t`` of a device (torch's own accessor skips the Stream object: 0.2 us instead of 2)."""
-    get = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if get is None:
-        return torch.cuda.current_stream(device).cuda_stream
-    return get(device.index if device.index is not None else torch.cuda.current_device())
-
-
-def _launch_on(device: torch.device, fn, ref, stream, what: str) -> None:
-    """Calls a launcher with ``device`` current; entering the device context costs as much as half a launch, so only when needed."""
-    if device.index is None or torch.cuda.current_device() == device.index:
-        rc = fn(ref, stream)
-    else:
-        with torch.cuda.device(device):
-            rc = fn(ref, stream)
-    _lib.check(rc, what)
-
-
 class _Layout(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int64) for n in (
         "off_counts", "off_counts_flag", "off_disp_flag", "off_recv_x", "off_recv_scales", "off_recv_info", "off_comb_x", "off_comb_flag", "off_comb_in",
@@ -439,9 +421,6 @@ class Buffer:
         s.barrier, s.status, s.mask = self._bar.data_ptr(), self._status.data_ptr(), self.mask.data_ptr()
         return s
 
-    def _stream(self) -> ctypes.c_void_p:
-        return ctypes.c_void_p(_raw_stream(self.device))
-
     def _region(self, parity: int, name: str, nbytes: int) -> torch.Tensor:
         start = self._lay[name] + parity * self._half
         return self.buffer[start : start + nbytes]
@@ -540,12 +519,12 @@ class Buffer:
         p.peers = self._peers_view
         p.epoch = epoch
         p.grid = grid or self._num_sms
-        stream_ptr = self._stream()
+        stream_ptr = _lib.raw_stream(self.device)
         fn, ref = self._dispatch_fn, ctypes.byref(p)
 
         def launch(phases: int) -> None:
             p.phases = phases
-            _launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_dispatch_launch")
+            _lib.launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_dispatch_launch")
 
         launch(phases_now)
         hook = (lambda: launch(2)) if hook_later else None
@@ -732,12 +711,12 @@ class Buffer:
         p.lay = self._layout(handle.parity)
         p.epoch, p.timeout_ns = handle.epoch, self.timeout_ns
         p.scr = self._scratch()
-        stream_ptr = self._stream()
+        stream_ptr = _lib.raw_stream(self.device)
         fn, ref = self._combine_fn, ctypes.byref(p)
 
         def launch(phases: int) -> None:
             p.phases = phases
-            _launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_combine_launch")
+            _lib.launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_combine_launch")
 
         launch(phases_now)
         self._keep_c = (x, topk_idx, topk_weights, out, p)
