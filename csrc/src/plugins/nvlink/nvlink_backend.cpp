@@ -922,8 +922,8 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         if (!cuda_) return fail(NIXL_ERR_NOT_SUPPORTED);
         // Host memory that its owner pinned: the copy engines move a long descriptor at 53 - 56 GB/s, the kernel at 50, but a copy
         // per descriptor costs 4 to 5 us.  Measured, kernel / copies: 256 x 4 KiB 31 / 990 us, 16 x 64 KiB 31 / 85 us, 16 x 1 MiB
-        // 340 / 378 us; 16 x 4 MiB 1.34 / 1.29 ms; a single 64 KiB 8.5 / 13 us, a single 256 KiB 20 / 17 us.
-        const bool by_copy = l->pinnedByOwner && len >= (local.descCount() == 1 ? size_t(128) << 10 : size_t(4) << 20);
+        // 340 / 378 us; 16 x 4 MiB 1.34 / 1.29 ms; a single 64 KiB 8.5 / 13 us, a single 100 KB 14.4 / 13.5, a single 256 KiB 20 / 17.
+        const bool by_copy = l->pinnedByOwner && len > (local.descCount() == 1 ? size_t(64) << 10 : size_t(4) << 20);
         if (lvis && rvis && !by_copy) { // the copy kernel can see both ends
             int dev;
             if (l->mem == VRAM_SEG) dev = l->device;

@@ -90,7 +90,7 @@ def test_either_side_of_the_request_size_rule():
 @pytest.mark.parametrize("pinned", [True, False])
 @pytest.mark.parametrize(
     "lens",
-    [[4096], [(128 << 10) - 1], [128 << 10], [1, 63, 4097, 70000], [(4 << 20) - 1, 4 << 20, 5, (4 << 20) + 3], [333] * 300],
+    [[4096], [64 << 10], [(64 << 10) + 1], [1, 63, 4097, 70000], [(4 << 20) - 1, 4 << 20, 5, (4 << 20) + 3], [333] * 300],
 )
 def test_host_memory_either_side_of_the_copy_engine_rule(op, pinned, lens):
     """Host memory pinned by its owner (short pieces by the kernel, long or single ones by copies) or by the registration."""
