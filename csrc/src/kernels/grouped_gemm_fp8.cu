@@ -55,6 +55,8 @@ constexpr int kTmemCols = kAccBufs * BN;
 using nixl_gemm::GEMM_ERR_ARRIVAL;
 using nixl_gemm::GEMM_ERR_TIMEOUT;
 using nixl_gemm::kMaxGroups;
+using nixl_gemm::ldScale;
+using nixl_gemm::waitArrivals;
 
 struct Shared {
     uint64_t full[kMaxStages];
@@ -210,29 +212,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         for (int ti = blockIdx.x; tileAt(sh, p.groups, n_tiles, ti, t); ti += gridDim.x) {
             const int row0 = sh.rowStart[t.g] + t.mt * BM;
             if (p.disp_flag) {
-                // Rows of an expert are ordered by source rank: wait for the sources whose rows
-                // intersect this tile.
-                const int lo = t.mt * BM, hi = min(lo + BM, sh.rowCount[t.g]);
-                int first = 0;
-                for (int r = 0; r < p.ranks; ++r) {
-                    const int c = p.counts[static_cast<long long>(r) * p.experts_total + p.expert_base + t.g];
-                    if (c > 0 && first < hi && first + c > lo) {
-                        const uint64_t *flag = p.disp_flag + static_cast<long long>(t.g) * p.ranks + r;
-                        uint64_t t0 = 0;
-                        unsigned spins = 0;
-                        while (ldAcquireSys(flag) < p.epoch) {
-                            if ((++spins & 63u) == 0) {
-                                const uint64_t now = nowNs();
-                                if (t0 == 0) t0 = now;
-                                else if (now - t0 > p.timeout_ns) {
-                                    atomicOr(p.status, GEMM_ERR_ARRIVAL); // compute on what is there; the host sees the bit
-                                    break;
-                                }
-                            }
-                        }
-                    }
-                    first += c;
-                }
+                waitArrivals(p, t.g, t.mt * BM, min(t.mt * BM + BM, sh.rowCount[t.g]));
                 asm volatile("fence.proxy.async;" ::: "memory"); // peers' generic-proxy stores before our async-proxy reads
             }
             const int box = aBoxRows(sh.rowCount[t.g] - t.mt * BM);
@@ -321,6 +301,8 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 if (!alive) break;
                 continue;
             }
+            const bool fresh = p.disp_flag != nullptr; // the scales travel with the rows
+            if (fresh) waitArrivals(p, t.g, t.mt * BM + q * 32, min(t.mt * BM + q * 32 + 32, sh.rowCount[t.g]));
             const long long grow = static_cast<long long>(sh.rowStart[t.g]) + local_row;
             const float *sa_row = scale_a + grow * k_steps;
             const float *sw = p.scale_w + (static_cast<long long>(t.g) * n_tiles + t.nt) * k_steps;
@@ -335,7 +317,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             float ring_a[kPrefetch], ring_w[kPrefetch];
 #pragma unroll
             for (int j = 0; j < kPrefetch; ++j) {
-                ring_a[j] = (j < k_steps && valid) ? __ldg(sa_row + j) : 0.f;
+                ring_a[j] = (j < k_steps && valid) ? ldScale(sa_row + j, fresh) : 0.f;
                 ring_w[j] = j < k_steps ? __ldg(sw + j) : 0.f;
             }
             for (int ks0 = 0; ks0 < k_steps && ok; ks0 += kPrefetch) {
@@ -347,7 +329,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                     const float s = ring_a[j] * ring_w[j];
                     const int nxt = ks + kPrefetch;
                     if (nxt < k_steps) {
-                        ring_a[j] = valid ? __ldg(sa_row + nxt) : 0.f;
+                        ring_a[j] = valid ? ldScale(sa_row + nxt, fresh) : 0.f;
                         ring_w[j] = __ldg(sw + nxt);
                     }
                     if (!mbarWait(&sh.tmemFull[buf], (it / kAccBufs) & 1, abort_flag)) {

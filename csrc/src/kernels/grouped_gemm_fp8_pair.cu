@@ -51,6 +51,8 @@ using namespace nixl_tc;
 using nixl_gemm::GEMM_ERR_ARRIVAL;
 using nixl_gemm::GEMM_ERR_TIMEOUT;
 using nixl_gemm::kMaxGroups;
+using nixl_gemm::ldScale;
+using nixl_gemm::waitArrivals;
 
 constexpr int BM = 128;        // rows per CTA (256 per pair)
 constexpr int BN = 256;        // tile columns
@@ -167,7 +169,7 @@ __device__ __forceinline__ bool tailTile(const Shared &sh, const Tile &t) { retu
 // tailTile (64 of 128 columns per thread; a loop of its own, as conditions in the full tile's loop made the compiler spill there).
 // False when another role gave up.
 template<bool kTail>
-__device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, bool valid, const float *sw0, int k_steps, uint32_t lane_base, uint32_t full0, int lane,
+__device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, bool valid, bool fresh, const float *sw0, int k_steps, uint32_t lane_base, uint32_t full0, int lane,
                                             uint32_t &it, uint32_t &s2, bool &rdy, __nv_bfloat16 *out, long long row_stride, int rows_left) {
     volatile int *abort_flag = &sh.abort;
     constexpr int kBlocks = kTail ? 2 : 4; // of 32 columns
@@ -179,8 +181,8 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
         for (int i = 0; i < 16; ++i) acc[j][i] = 0;
     // Scales are fetched two steps ahead and kept as loaded: multiplying them right away would make the warp
     // wait for the loads it has just issued.  (A loop unrolled over a ring of four made the compiler spill.)
-    float a0 = valid ? __ldg(sa_row) : 0.f, w00 = __ldg(sw0), w10 = __ldg(sw1);
-    float a1 = valid && k_steps > 1 ? __ldg(sa_row + 1) : 0.f, w01 = k_steps > 1 ? __ldg(sw0 + 1) : 0.f, w11 = k_steps > 1 ? __ldg(sw1 + 1) : 0.f;
+    float a0 = valid ? ldScale(sa_row, fresh) : 0.f, w00 = __ldg(sw0), w10 = __ldg(sw1);
+    float a1 = valid && k_steps > 1 ? ldScale(sa_row + 1, fresh) : 0.f, w01 = k_steps > 1 ? __ldg(sw0 + 1) : 0.f, w11 = k_steps > 1 ? __ldg(sw1 + 1) : 0.f;
 #pragma unroll 1
     for (int ks = 0; ks < k_steps; ++ks, ++it) {
         const float s0 = a0 * w00, s1 = a0 * w10;
@@ -216,7 +218,7 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
         if (++s2 == kStages) s2 = 0;
         // The scale prefetch goes behind the arrive (loads issued before it would hold it up).
         if (nxt < k_steps) {
-            a1 = valid ? __ldg(sa_row + nxt) : 0.f;
+            a1 = valid ? ldScale(sa_row + nxt, fresh) : 0.f;
             w01 = __ldg(sw0 + nxt);
             if (!kTail) w11 = __ldg(sw1 + nxt);
         }
@@ -319,28 +321,8 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
                 const int row0 = sh.rowStart[t.g] + lo;
                 const uint32_t bytes = static_cast<uint32_t>(2 * (rows_cta + WROWS) * BK); // both CTAs' shares
                 if (p.disp_flag) {
-                    const int hi = min(lo + rows_cta, sh.rowCount[t.g]);
-                    int first = 0;
-                    for (int r = 0; r < p.ranks; ++r) {
-                        const int c = p.counts[static_cast<long long>(r) * p.experts_total + p.expert_base + t.g];
-                        if (c > 0 && first < hi && first + c > lo) {
-                            const uint64_t *flag = p.disp_flag + static_cast<long long>(t.g) * p.ranks + r;
-                            uint64_t t0 = 0;
-                            unsigned spins = 0;
-                            while (ldAcquireSys(flag) < p.epoch) {
-                                if ((++spins & 63u) == 0) {
-                                    const uint64_t now = nowNs();
-                                    if (t0 == 0) t0 = now;
-                                    else if (now - t0 > p.timeout_ns) {
-                                        atomicOr(p.status, GEMM_ERR_ARRIVAL);
-                                        break;
-                                    }
-                                }
-                            }
-                        }
-                        first += c;
-                    }
-                    asm volatile("fence.proxy.async;" ::: "memory");
+                    waitArrivals(p, t.g, lo, min(lo + rows_cta, sh.rowCount[t.g]));
+                    asm volatile("fence.proxy.async;" ::: "memory"); // peers' generic-proxy stores before our async-proxy reads
                 }
                 const int wrow = t.g * p.N + t.nt * BN + static_cast<int>(cta) * WROWS;
                 for (int ks = 0; ks < k_steps; ++ks, ++it) {
@@ -401,6 +383,8 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
             const int first_row = t.mt * (2 * BM) + (tail ? static_cast<int>(cta) * (BM / 2) + (q & 1) * 32 : static_cast<int>(cta) * BM + q * 32);
             const int local_row = first_row + lane;
             const bool valid = local_row < sh.rowCount[t.g];
+            const bool fresh = p.disp_flag != nullptr; // the scales travel with the rows
+            if (fresh) waitArrivals(p, t.g, first_row, min(first_row + 32, sh.rowCount[t.g]));
             const long long grow = static_cast<long long>(sh.rowStart[t.g]) + local_row;
             const float *sa_row = p.scale_a + grow * k_steps;
             const float *sw0 = p.scale_w + (static_cast<long long>(t.g) * n_blocks + t.nt * 2 + (tail ? q >> 1 : 0)) * k_steps;
@@ -408,8 +392,8 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
             const int rows_left = sh.rowCount[t.g] - row8;
             __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.d) + (static_cast<long long>(sh.rowStart[t.g]) + row8) * p.N + t.nt * BN +
                 (tail ? (q >> 1) * BNS : 0) + part * 64 + (lane & 7) * 8;
-            ok = tail ? promoteTile<true>(sh, sa_row, valid, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left)
-                      : promoteTile<false>(sh, sa_row, valid, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left);
+            ok = tail ? promoteTile<true>(sh, sa_row, valid, fresh, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left)
+                      : promoteTile<false>(sh, sa_row, valid, fresh, sw0, k_steps, lane_base, full0, lane, it, s2, rdy, out, p.N, rows_left);
         }
     }
 

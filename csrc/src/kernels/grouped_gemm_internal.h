@@ -6,6 +6,9 @@
 #include <cuda_runtime.h>
 
 #include "kernels/nixl_kernels.h"
+#ifdef __CUDACC__
+#include "kernels/tcgen05_ptx.cuh"
+#endif
 
 namespace nixl_gemm {
 
@@ -23,6 +26,36 @@ cudaError_t launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapA64,
 // p.scale_a / p.scale_w point at exponent bytes (uint8 [a_rows][K/128] and [groups][N/128][K/128]);
 // K must be a multiple of 512, N of 256; no dispatch overlap.  The maps of the tokens have boxes of 128, 32 and 64 rows.
 cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
+
+#ifdef __CUDACC__
+// Waits (bounded) until the rows [lo, hi) of group g have arrived: rows of an expert are ordered by source rank, so for the
+// arrival flags of the sources whose rows intersect the range.  On expiry the host sees the status bit and the kernel
+// computes on what is there.
+__device__ __forceinline__ void waitArrivals(const NixlGroupedGemmParams &p, int g, int lo, int hi) {
+    int first = 0;
+    for (int r = 0; r < p.ranks; ++r) {
+        const int c = p.counts[static_cast<long long>(r) * p.experts_total + p.expert_base + g];
+        if (c > 0 && first < hi && first + c > lo) {
+            const uint64_t *flag = p.disp_flag + static_cast<long long>(g) * p.ranks + r;
+            uint64_t t0 = 0;
+            unsigned spins = 0;
+            while (nixl_tc::ldAcquireSys(flag) < p.epoch) {
+                if ((++spins & 63u) == 0) {
+                    const uint64_t now = nixl_tc::nowNs();
+                    if (t0 == 0) t0 = now;
+                    else if (now - t0 > p.timeout_ns) {
+                        atomicOr(p.status, GEMM_ERR_ARRIVAL);
+                        break;
+                    }
+                }
+            }
+        }
+        first += c;
+    }
+}
+// A scale of A: through the read-only path, unless a dispatch may have written it while this kernel was running already.
+__device__ __forceinline__ float ldScale(const float *s, bool fresh) { return fresh ? __ldcg(s) : __ldg(s); }
+#endif
 
 } // namespace nixl_gemm
 

@@ -155,3 +155,33 @@ def test_combine_of_one_rank(tokens, topk, experts, hidden, mode):
         assert bool(((out.double() - want).abs() <= want.abs() * 2.0**-8 + mass * (16 * 2.0**-24)).all())
     assert b.status == 0
     b.destroy()
+
+
+@pytest.mark.parametrize("low_latency", [True, False])
+def test_fused_gemm_takes_the_scales_that_arrive(low_latency):
+    """The GEMM that overlaps a dispatch must read a row's scales after the row's arrival flag, not what the buffer held
+    before: the scale area is filled with another value first, in both halves."""
+    from nixl_b200.ops import grouped_gemm_fp8, quantize_weights
+
+    T, H, E, K, N = 200, 2048, 8, 4, 512
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(3)
+    b = Buffer(0, 1, E, H, T, K, device=dev, low_latency_mode=low_latency)
+    b.connect_ranks()
+    x = torch.randn(T, H, device=dev, generator=g).to(torch.bfloat16)
+    _, idx = torch.topk(torch.softmax(torch.randn(T, E, device=dev, generator=g), -1), K, -1)
+    idx = idx.contiguous()
+    wq, sw = quantize_weights(torch.randn(E, N, H, device=dev, generator=g) * 0.05)
+    rows = b.ll_rows if low_latency else b.compact_rows
+    for _ in range(4):
+        for parity in (0, 1):
+            b._region(parity, "off_recv_scales", rows * (H // 128) * 4).view(torch.float32).fill_(1.0e4)
+        torch.cuda.synchronize()
+        got, h, rx, sc = b.dispatch_gemm(x, idx, wq, sw, low_latency=low_latency)
+        torch.cuda.synchronize()
+        want = grouped_gemm_fp8(rx[:rows], sc[:rows], wq, sw, h.expert_offsets, h.recv_count, tile_mode=1)
+        torch.cuda.synchronize()
+        for e in range(E):
+            s, c = int(h.expert_offsets[e]), int(h.recv_count[e])
+            assert torch.equal(got[s : s + c], want[s : s + c]), (e, c)
+    b.destroy()
