@@ -52,7 +52,7 @@ typedef struct NixlKvXferParams {
     uint64_t *host_flag;       /* may be NULL; host-mapped word that receives host_seq */
     uint64_t host_seq;
     uint32_t *done_counter;    /* device scratch word, zero before the first launch; reset by the kernel */
-    int32_t grid;              /* 0: default (two CTAs per SM) */
+    int32_t grid;              /* 0: default (four CTAs per SM, eight for large requests, never more than there is work for) */
     int32_t *status;           /* may be NULL; device-visible word (device or pinned host memory) that receives 1 when a block id
                                   pointed outside its cache tensor's view entry: that block is skipped, nothing outside is touched */
 } NixlKvXferParams;
@@ -128,7 +128,7 @@ typedef struct NixlEpDispatchParams {
     int32_t rows_per_expert;  /* >0: expert le starts at row le*rows_per_expert; 0: compact (prefix) layout */
     int32_t cap;              /* rows available at every receiver */
     int32_t phases;           /* bit0 send, bit1 receive (wait for arrivals), bit2 publish recv_count/offsets without waiting */
-    int32_t grid;             /* CTAs (cooperative launch); 0 = one per SM */
+    int32_t grid;             /* CTAs; 0: by the number of tokens (at most four per SM) */
     const void *peers;        /* remote memory view */
     NixlEpLayout lay;
     uint64_t epoch;

@@ -1,10 +1,9 @@
 // MoE expert-parallel dispatch / combine for one NVLink domain (contract and algorithm:
 // include/kernels/nixl_kernels.h).
 //
-// Both kernels are persistent, cooperatively launched grids (every CTA resident, so the
-// in-kernel grid barrier cannot deadlock) of 256 threads.  Peer memory is reached through the
-// remote memory view prepared by the agent: plain stores over NVLink, release-ordered flags,
-// and bounded waits that mask a silent peer instead of hanging the GPU.
+// All are persistent grids of 256 threads, launched cooperatively where they contain a grid barrier (every CTA resident,
+// so that it cannot deadlock).  Peer memory is reached through the remote memory view prepared by the agent: plain stores
+// over NVLink, release-ordered flags, and bounded waits that mask a silent peer instead of hanging the GPU.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -1247,9 +1246,15 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
     if (p.topk_weights && (p.K > 8 || p.R > 32 || p.max_tokens < p.T)) return cudaErrorInvalidValue; // a group record holds eight copies
     if (p.rows_per_expert > 0 && static_cast<long long>(p.rows_per_expert) < static_cast<long long>(p.R) * p.T) return cudaErrorInvalidValue;
     const size_t smem = size_t(4) * p.E * sizeof(int) + size_t(kBatch) * p.K * (sizeof(int) + 1) + 16;
-    if (smem > 48 * 1024) { // many experts: the shared-memory limit is a per-device function attribute
-        const cudaError_t e = cudaFuncSetAttribute(epDispatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
+    if (smem > 48 * 1024) { // many experts: the shared-memory limit is a per-device function attribute, raised once to all there is
+        static bool attr_done[64] = {};
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev < 0 || dev >= 64 || !attr_done[dev]) {
+            const cudaError_t e = cudaFuncSetAttribute(epDispatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) attr_done[dev] = true;
+        }
     }
     // With many tokens four CTAs per SM keep enough loads and stores in flight; a few tokens go to one CTA per SM, whose
     // eight warps share them (fewer CTAs at the grid barrier).

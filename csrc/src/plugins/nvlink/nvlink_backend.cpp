@@ -1697,7 +1697,7 @@ nixl_b_params_t nvlinkDefaults() {
         {"copy_path", "vector"},   // kernel for descriptors below ce_threshold: "vector" (SIMT) or "bulk" (TMA 1-D through shared memory); "ce": copy engines for everything
         {"ce_threshold", "100663296"}, // descriptors between GPUs of at least this many bytes (96 MiB) go to the copy engines; 0: never
         {"coalesce", "true"},      // merge descriptors that continue their predecessor on both sides
-        {"grid_ctas", "0"},        // 0: two CTAs per SM
+        {"grid_ctas", "0"},        // 0: by the amount of work (two CTAs per SM, four of the warp-sized kernel, more when there are many chunks)
         {"device_id", "-1"},       // GPU that maps other processes' memory; -1: first registered / current
         {"liveness_ping", "false"},// probe the peer's socket at every post
         {"host_id", ""},           // name of the NVLink box (default: the host name); peers that name another one are left to other backends

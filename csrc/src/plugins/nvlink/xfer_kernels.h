@@ -2,7 +2,8 @@
 //
 // One launch moves a whole batch of descriptors.  Work is cut into power-of-two chunks;
 // chunk c belongs to the descriptor i with chunkStart[i] <= c < chunkStart[i+1].  A
-// persistent grid walks the chunks, so 256 x 4 KiB and 1 x 1 GiB cost one launch each.
+// persistent grid walks the chunks, so 256 x 4 KiB and 1 x 1 GiB cost one launch each.  A chunk is the work of a CTA, or
+// of one warp where a request is small or its descriptors are short (warpChunks).
 // The CTA that finishes last publishes `seq` to a host-mapped completion word, which is
 // what the backend's checkXfer polls - no event, no stream synchronisation.
 #ifndef NIXL_B200_XFER_KERNELS_H

@@ -106,6 +106,34 @@ def test_dispatch_of_several_ranks(n, tokens, topk, hidden, low_latency, kind, n
         b.destroy()
 
 
+def test_dispatch_with_more_experts_than_the_default_shared_memory_holds():
+    n, El, tokens, topk, hidden = 6, 512, 40, 4, 512  # 16 bytes per expert: just above 48 KiB
+    experts = n * El
+    bufs = _ranks(n, experts, hidden, tokens, topk, "er_many", False)
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(5)
+    xs = [torch.randn(tokens, hidden, device=dev, dtype=torch.bfloat16, generator=g) for _ in bufs]
+    idxs = [torch.topk(torch.randn(tokens, experts, device=dev, generator=g), topk, -1)[1].contiguous() for _ in bufs]
+    counts = torch.stack([torch.bincount(i.reshape(-1), minlength=experts) for i in idxs]).int()
+    for b in bufs:
+        b._region(1, "off_counts", n * experts * 4).view(torch.int32).copy_(counts.reshape(-1))
+        b._region(1, "off_counts_flag", n * 8).view(torch.int64).fill_(1)
+    results = [b._dispatch(xs[r], idxs[r], False, False, 0, 5, False) for r, b in enumerate(bufs)]
+    torch.cuda.synchronize()
+    for d, b in enumerate(bufs):
+        assert b.status == 0
+        recv_x, _, h, _, _ = results[d]
+        mine = counts[:, d * El : (d + 1) * El].sum(0).int()
+        assert torch.equal(h.recv_count, mine)
+        for r in range(n):
+            t, k = torch.nonzero(idxs[r] // El == d, as_tuple=True)
+            rows = results[r][2].send_row[t, k].long()
+            assert torch.equal(recv_x[rows], xs[r][t])
+            assert bool((rows >= h.expert_offsets[idxs[r][t, k] - d * El]).all())
+    for b in bufs:
+        b.destroy()
+
+
 @pytest.mark.parametrize("mode", ["push", "pull", "reduced"])
 @pytest.mark.parametrize("tokens,topk,experts,hidden", [(1, 1, 1, 512), (7, 3, 4, 512), (130, 8, 16, 2048), (1300, 4, 8, 1024), (40, 12, 16, 512)])
 def test_combine_of_one_rank(tokens, topk, experts, hidden, mode):
