@@ -80,7 +80,7 @@ struct Shared {
     uint64_t tmemEmpty;          // even CTA: all 16 epilogue warps have read the accumulator
     uint32_t tmemBase;
     int abort;
-    volatile uint32_t chunksIssued; // two issuing threads take turns chunk by chunk: the next chunk whose MMAs may enter the pipe
+    uint32_t chunksIssued;       // two issuing threads take turns chunk by chunk: the next chunk whose MMAs may enter the pipe
     int tilePrefix[kMaxGroups + 1];
     int rowStart[kMaxGroups];
     int rowCount[kMaxGroups];
@@ -270,10 +270,11 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
         // ---------------------------------------------------------------- two MMA issuers (even CTA)
         // The tensor pipe idles whenever its issuing thread does anything but issue (an MMA's issue
         // returns about when its predecessor starts).  Two threads therefore alternate chunk by chunk
-        // (four steps, 32 MMAs): while one is parked in the issue of its chunk, the other waits for its
+        // (four steps, 16 MMAs): while one is parked in the issue of its chunk, the other waits for its
         // next chunk's barriers and sits ready.  A turn counter keeps the chunks entering the pipe in
-        // order (the first step of a tile overwrites the accumulator, and a chunk's scale copy must
-        // precede its MMAs); even chunks use TMEM scale columns of parity 0, odd chunks parity 1.
+        // order (the first step of a tile overwrites the accumulator, and the scale copies of a group of up to eight
+        // chunks, made by the thread that has its first one, must precede the MMAs of both threads that read them);
+        // even groups use one set of TMEM scale columns, odd groups the other.
         const uint32_t me = warp == 1 ? 0u : 1u;
         const uint32_t full_bar0 = smemU32(&sh.full[0]), empty_bar0 = smemU32(&sh.empty[0]), sfempty_bar0 = smemU32(&sh.sfEmpty[0]);
         const uint64_t desc0 = smemDesc(smemU32(tiles));
@@ -296,7 +297,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
             if (!mbarWait(&sh.full[s], full_par, abort_flag)) goto issuer_done;
             {
                 const long long t0 = clock64();
-                while (sh.chunksIssued != cc) {
+                while (ldAcquireCta(&sh.chunksIssued) != cc) {
                     if (*abort_flag) goto issuer_done;
                     if (clock64() - t0 > (1ll << 33)) {
                         *abort_flag = 1;
@@ -333,9 +334,11 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
                 s = ns;
                 full_par = nfull_par;
             }
-            // All of this chunk's MMAs are in the pipe: the other thread's chunk may follow.
-            asm volatile("" ::: "memory");
-            sh.chunksIssued = cc + 1;
+            // All of this chunk's MMAs are in the pipe: the other thread's chunk may follow.  It adds to the accumulator
+            // these MMAs write and may read the scale columns copied here, and tcgen05 operations of two threads are in
+            // order only across a fence on either side of the hand-over (tcFenceAfter: above, with the turn).
+            tcFenceBefore();
+            stReleaseCta(&sh.chunksIssued, cc + 1);
             if (c + 1 == static_cast<uint32_t>(chunks) || c + 2 == static_cast<uint32_t>(chunks)) {
                 // This thread's last chunk of the tile: its share of "accumulator complete" (both shares when
                 // the tile has a single chunk and the other thread never touches it).

@@ -72,6 +72,16 @@ __device__ __forceinline__ void tmaLoad2d(void *smem_dst, const CUtensorMap *map
 }
 __device__ __forceinline__ void tcFenceBefore() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcFenceAfter() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// A word in shared memory by which threads of a CTA hand work to each other (together with the two fences above when the
+// work is tcgen05 operations: these are in order by themselves only within one thread).
+__device__ __forceinline__ void stReleaseCta(uint32_t *p, uint32_t v) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smemU32(p)), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ldAcquireCta(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smemU32(p)) : "memory");
+    return v;
+}
 __device__ __forceinline__ void tcCommit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smemU32(bar)) : "memory");
 }

@@ -1,0 +1,28 @@
+"""The grouped GEMMs with several tiles of different sizes per CTA or CTA pair: what the roles carry from tile to tile (ring
+positions, parities, scale groups, the accumulator's hand-back).  `grid` holds the launch to 2, 4 or 6 CTAs; with the default
+grid the shapes of test_gpu_grouped_gemm_tiles.py give a pair one tile at most."""
+import pytest
+import torch
+
+from nixl_b200.ops import grouped_gemm_mxfp8, to_ue8m0
+from test_gpu_grouped_gemm_tiles import _check, _inputs
+
+pytestmark = pytest.mark.gpu
+
+_MIXED = [1, 300, 32, 0, 129, 513, 64, 255, 257]  # tiles of 32 to 256 tokens in turn
+
+
+def _run(gemm, counts, N, K, grid, seed, mx=False, **kw):
+    a, sa, w, sw, rs, rc = _inputs(counts, N, K, seed)
+    for _ in range(3):  # the bound of _check leaves no room for a tile that was overwritten while it was read
+        out = torch.full((a.shape[0], N), 5.0, dtype=torch.bfloat16, device=a.device)
+        gemm(a, to_ue8m0(sa) if mx else sa, w, to_ue8m0(sw) if mx else sw, rs, rc, out=out, grid=grid, **kw)
+        torch.cuda.synchronize()
+        assert int(out._nixl_status.item()) == 0
+        _check(out, a, sa, w, sw, rs, rc, K)
+
+
+@pytest.mark.parametrize("grid", [2, 4, 6])
+@pytest.mark.parametrize("N,K", [(512, 1024), (768, 1536), (256, 4608), (512, 8704)])  # 2, 3, 9 and 17 chunks of scales: one to three groups
+def test_block_scales_that_one_thread_copies_and_the_other_uses(grid, N, K):
+    _run(grouped_gemm_mxfp8, _MIXED, N, K, grid, 11, mx=True)
