@@ -292,7 +292,6 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
                 known_tile = tile;
             }
             // Everything this chunk depends on, before asking for the turn.
-            if (c == 0 && !mbarWait(&sh.tmemEmpty, (tile & 1u) ^ 1u, abort_flag)) goto issuer_done; // accumulator drained by the previous epilogue
             if (c % kGroupChunks == 0 && !mbarWait(&sh.sfFull[b], (gg >> 1) & 1u, abort_flag)) goto issuer_done;
             if (!mbarWait(&sh.full[s], full_par, abort_flag)) goto issuer_done;
             {
@@ -305,6 +304,11 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
                     }
                 }
             }
+            // Accumulator drained by the previous tile's epilogue.  With the turn in hand, not before: the previous tile is
+            // then issued, so its own wait here has passed and the barrier is at most one phase behind, which is all a parity
+            // can tell.  (With one chunk per tile a thread would otherwise look before the other one issued the tile between,
+            // two phases early, and pass at once.)
+            if (c == 0 && !mbarWait(&sh.tmemEmpty, (tile & 1u) ^ 1u, abort_flag)) goto issuer_done;
             tcFenceAfter();
             const uint32_t sf_base = tmem + kAccCols + b * kSfTmemStride;
             if (c % kGroupChunks == 0) {

@@ -26,3 +26,11 @@ def _run(gemm, counts, N, K, grid, seed, mx=False, **kw):
 @pytest.mark.parametrize("N,K", [(512, 1024), (768, 1536), (256, 4608), (512, 8704)])  # 2, 3, 9 and 17 chunks of scales: one to three groups
 def test_block_scales_that_one_thread_copies_and_the_other_uses(grid, N, K):
     _run(grouped_gemm_mxfp8, _MIXED, N, K, grid, 11, mx=True)
+
+
+@pytest.mark.parametrize("grid", [2, 4, 6])
+@pytest.mark.parametrize("N", [256, 1024])
+def test_block_scales_with_one_chunk_per_tile(grid, N):
+    """K = 512: the two issuing threads take whole tiles in turn, and only the wait for the accumulator keeps them apart."""
+    _run(grouped_gemm_mxfp8, _MIXED, N, 512, grid, 12, mx=True)
+    _run(grouped_gemm_mxfp8, [256] * 24, N, 512, grid, 13, mx=True)
