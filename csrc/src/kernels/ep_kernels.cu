@@ -476,11 +476,13 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         if (tid == 0) {
             __threadfence();
             last = atomicAdd(p.scr.barrier + 2, 1u) == gridDim.x - 1;
-            if (last) p.scr.barrier[2] = 0;
+            if (last) {
+                p.scr.barrier[2] = 0;
+                __threadfence(); // the other CTAs' counts and rows
+            }
         }
         __syncthreads();
         if (last && fixed) {
-            __threadfence(); // the other CTAs' counts
             int *counts = reinterpret_cast<int *>(self + p.lay.off_counts);
             uint64_t *dflag = reinterpret_cast<uint64_t *>(self + p.lay.off_disp_flag);
             for (int e = tid; e < p.E; e += kThreads) {
@@ -491,12 +493,13 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 p.layout_range[e] = static_cast<unsigned>(c);
                 p.expert_offsets[e] = ebase[e];
                 if (e == p.E - 1) p.expert_offsets[p.E] = ebase[e] + p.rows_per_expert;
-                dflag[e] = p.epoch; // (every reader is a later launch)
             }
-            if (tid == 0) {
-                reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
-                *reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag) = p.epoch;
-            }
+            if (tid == 0) reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
+            // The flags go up behind all counts (of every warp) and, through the exit counter, all rows: a GEMM launched on
+            // another stream may look at them while this kernel runs.
+            __syncthreads();
+            for (int e = tid; e < p.E; e += kThreads) stReleaseSys(dflag + e, p.epoch);
+            if (tid == 0) stReleaseSys(reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag), p.epoch);
         }
         if (last)
             for (int e = tid; e < p.E; e += kThreads) {
