@@ -348,27 +348,27 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         }
     }
 
-    const bool alone = p.R == 1;
+    // A group of one rank that sends in this launch has everybody's counts, its own, from the grid barrier, and sends every
+    // row itself.  (A launch that only receives waits for the flags like any other: the caller may have sent on another stream.)
+    const bool own = p.R == 1 && (p.phases & 1);
     // 3. wait for everybody's counts (every CTA looks for itself: 8 flags, no grid barrier needed)
-    //    A group of one rank has them already: its own, from the grid barrier (or from the send phase's launch).
     if (!fixed) {
         const uint64_t *cflag = reinterpret_cast<const uint64_t *>(self + p.lay.off_counts_flag);
         if (tid < p.R) {
             if (masked[tid] == 0 && peer_sh[tid] != nullptr) {
-                if (!alone && !waitFlag(cflag + tid, p.epoch, p.timeout_ns)) {
+                if (!own && !waitFlag(cflag + tid, p.epoch, p.timeout_ns)) {
                     atomicExch(p.scr.mask + tid, 1);
                     atomicOr(p.scr.status, ST_PEER_TIMEOUT);
                 }
             } else if (peer_sh[tid] == nullptr) {
                 atomicExch(p.scr.mask + tid, 1);
             }
-            if (!alone) masked[tid] = ldVolatile(p.scr.mask + tid);
+            if (!own) masked[tid] = ldVolatile(p.scr.mask + tid);
         }
         __syncthreads();
 
         // 4. placement tables.  counts[r][e] is the local copy of the all-gather.
         const int *counts = reinterpret_cast<const int *>(self + p.lay.off_counts);
-        const bool own = alone && (p.phases & 1); // the counts are in shared memory
         for (int e = tid; e < p.E; e += kThreads) {
             int b = 0, all = 0;
             for (int r = 0; r < p.R; ++r) {
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         }
     }
 
-    if ((p.phases & 2) && !alone) { // (alone: every row is this launch's, or an earlier one's on this stream)
+    if ((p.phases & 2) && !own) {
         // 6. arrivals: El x R flags, spread over the grid's threads
         const uint64_t *dflag = reinterpret_cast<const uint64_t *>(self + p.lay.off_disp_flag);
         const int nflags = El * p.R;

@@ -47,3 +47,37 @@ def test_gemm_on_another_stream_takes_this_steps_counts_and_rows(tokens):
         for e, c in enumerate(want_count.tolist()):
             assert torch.equal(got[e * tokens : e * tokens + c], want[e * tokens : e * tokens + c]), (step, e, c)
     b.destroy()
+
+
+def _one_phase(b, handle, phases, use_fp8=False):
+    """The launch that the receive hook makes, on the current stream."""
+    import ctypes
+
+    from nixl_b200.ops import _lib
+
+    p = b._disp_cache[(handle.parity, use_fp8, handle.rows_per_expert, False)][0]
+    p.phases = phases
+    _lib.check(b._dispatch_fn(ctypes.byref(p), _lib.raw_stream(b.device)), "dispatch")
+
+
+def test_receive_phase_waits_for_the_flags():
+    """A receive that runs before its rows are there must end in its bounded wait and say so, not hand out what is there."""
+    T, H, E, K = 20, 512, 4, 2
+    b = Buffer(0, 1, E, H, T, K, device=torch.device("cuda:0"), low_latency_mode=True, timeout_ms=50)
+    b.connect_ranks()
+    x, idx, _ = _routing(T, H, E, K, 2)
+    recv, count, h, _, hook = b.low_latency_dispatch(x, idx, use_fp8=False, return_recv_hook=True)
+    hook()
+    torch.cuda.synchronize()
+    assert b.status == 0 and torch.equal(count, torch.bincount(idx.reshape(-1), minlength=E).int())
+    flags = b._region(h.parity, "off_disp_flag", E * 8).view(torch.int64)
+    flags[1] = 0  # one expert's rows "not yet there"
+    _one_phase(b, h, 2)
+    torch.cuda.synchronize()
+    assert b.status & 1 and int(b.mask[0]) == 1
+    b.clean_mask_buffer()
+    flags[1] = h.epoch
+    _one_phase(b, h, 2)
+    torch.cuda.synchronize()
+    assert b.status == 0
+    b.destroy()
