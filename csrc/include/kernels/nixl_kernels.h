@@ -174,6 +174,9 @@ typedef struct NixlEpCombineParams {
      * expert_rank * max_tokens + token); the home rank adds the rows of the ranks the token went to.  A token
      * whose experts sit on fewer ranks than it has experts crosses NVLink that much less often. */
     int32_t max_tokens;
+    /* Rows of x; 0: not known.  out may overlap x unless x is the exposed region of the pull mode; a group of one rank that is
+     * told the rows, and so sees that they do not overlap, takes a shorter way. */
+    int32_t x_rows;
 } NixlEpCombineParams;
 
 /* Routing statistics of topk_idx [T][K]: tokens per destination rank (a token counts once per rank),

@@ -315,6 +315,7 @@ nixl_status_t nixlEpBuffer::combine(const void *y, const int64_t *topkIdx, const
     p.send_row = h.sendRow;
     p.use_logfmt = 0;
     p.max_tokens = cfg_.maxTokens;
+    p.x_rows = static_cast<int32_t>(rows);
     if (const int e = nixl_ep_combine_launch(&p, stream); e != 0) {
         NIXL_ERROR << "nixlEpBuffer: combine launch failed: " << cudaGetErrorString(static_cast<cudaError_t>(e));
         return NIXL_ERR_BACKEND;

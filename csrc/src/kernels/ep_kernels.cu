@@ -1063,8 +1063,8 @@ __global__ void __launch_bounds__(kThreads) epCombineKernel(const __grid_constan
 }
 
 // Combine when one rank holds every expert (R == 1): nothing has to travel, so whatever the mode the result is the weighted
-// sum of the token's rows of x where they lie.  One kernel without flags, barriers or a landing zone; all of it runs in the
-// send phase, after which the caller may overwrite x.  A warp takes a token or a part of one.  Bound by memory (K rows read,
+// sum of the token's rows of x where they lie.  One kernel without flags, barriers or a landing zone, for calls that send and
+// receive in one launch into an output apart from x (nixl_ep_combine_launch).  A warp takes a token or a part of one.  Bound by memory (K rows read,
 // one written), measured on one B200, 32 experts, top-8: 4096 tokens x 7168 83 us (528 MB, 6.4 TB/s), where the two kernels of
 // the rank-reduced mode took 107 + 34 us; 128 tokens, low-latency layout 4.9 us, where the push mode's copy to the landing zone,
 // barrier and sum took 27.6 us.
@@ -1288,8 +1288,14 @@ extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *s
         p.E / p.R > kMaxRanks * 8 || p.rank < 0 || p.rank >= p.R)
         return cudaErrorInvalidValue;
     void *args[] = {const_cast<NixlEpCombineParams *>(params)};
-    if (p.R == 1 && p.x && p.topk_weights && p.out && (p.pull == 2 || p.send_row)) {
-        if (!(p.phases & 1) || p.T <= 0) return cudaSuccess; // all of it happens in the send phase
+    // A one-rank group sums its rows where they lie, in one pass that writes out while it still reads x: only when both phases
+    // are one launch (a send alone must leave out untouched and x free to be overwritten) and out does not overlap x (the
+    // other paths have read all of x before the first row of out is written).
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(p.x), out0 = reinterpret_cast<uintptr_t>(p.out);
+    const uintptr_t x_bytes = p.x_rows > 0 ? static_cast<uintptr_t>(p.x_rows) * p.H * 2 : 0, out_bytes = static_cast<uintptr_t>(p.T > 0 ? p.T : 0) * p.H * 2;
+    const bool apart = x_bytes > 0 && (out0 + out_bytes <= x0 || x0 + x_bytes <= out0);
+    if (p.R == 1 && (p.phases & 3) == 3 && apart && p.x && p.topk_weights && p.out && (p.pull == 2 || p.send_row)) {
+        if (p.T <= 0) return cudaSuccess;
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -69,6 +69,7 @@ class _CombineParams(ctypes.Structure):
         ("phases", ctypes.c_int32), ("grid", ctypes.c_int32),
         ("peers", ctypes.c_void_p), ("lay", _Layout), ("epoch", ctypes.c_uint64), ("timeout_ns", ctypes.c_uint64), ("scr", _Scratch),
         ("pull", ctypes.c_int32), ("send_row", ctypes.c_void_p), ("use_logfmt", ctypes.c_int32), ("max_tokens", ctypes.c_int32),
+        ("x_rows", ctypes.c_int32),
     ]
 
 
@@ -627,7 +628,10 @@ class Buffer:
         ``use_logfmt=True`` sends the rows in a logarithmic 10-bit format (0.66 of the bf16 bytes on
         the wire, decoded inside the reduction; role of the reference's LogFMT-10,
         examples/device/ep/csrc/kernels/nixl_ep_ll.cu:459-616).  It implies the push path, since the
-        encoding happens on the way out, and needs ``hidden % 512 == 0``."""
+        encoding happens on the way out, and needs ``hidden % 512 == 0``.
+
+        With ``return_recv_hook=True`` ``x`` may be overwritten behind the call (not with ``zero_copy``) and ``out`` is written by
+        the hook.  ``out`` may overlap ``x``, unless ``zero_copy`` is set."""
         if use_logfmt and zero_copy:
             raise ValueError("use_logfmt encodes rows as they are sent; it cannot be combined with zero_copy")
         flat = x.reshape(-1, self.hidden)
@@ -701,7 +705,7 @@ class Buffer:
         p.max_tokens = self.max_tokens
         p.use_logfmt = int(use_logfmt)
         p.send_row = handle.send_row.data_ptr() if handle.send_row is not None else None
-        p.x = x_ptr
+        p.x, p.x_rows = x_ptr, x.shape[0]
         p.recv_info = handle.src_info.data_ptr()
         p.recv_count, p.expert_offsets = handle.recv_count.data_ptr(), handle.expert_offsets.data_ptr()
         p.topk_idx, p.topk_weights, p.out = topk_idx.data_ptr(), topk_weights.data_ptr(), out.data_ptr()

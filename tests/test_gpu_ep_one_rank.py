@@ -81,3 +81,84 @@ def test_receive_phase_waits_for_the_flags():
     torch.cuda.synchronize()
     assert b.status == 0
     b.destroy()
+
+
+def _dispatched(b, x, idx, w, low_latency):
+    """Rows as the experts left them (scaled by expert number + 1) and the sum they must give, with the bound of its rounding."""
+    if low_latency:
+        recv, _, h, _, _ = b.low_latency_dispatch(x, idx, use_fp8=False)
+    else:
+        recv, _, h = b.dispatch(x, idx, use_fp8=False, topk_weights=w)
+    flat = recv.view(-1, x.shape[1])
+    y = flat.clone()
+    for e in range(b.num_experts):
+        s, c = int(h.expert_offsets[e]), int(h.recv_count[e])
+        y[s : s + c] = (flat[s : s + c].float() * (e + 1)).to(torch.bfloat16)
+    want = torch.zeros(x.shape, device=x.device, dtype=torch.float64)
+    mass = torch.zeros_like(want)
+    for k in range(idx.shape[1]):
+        term = (x.float() * (idx[:, k] + 1).unsqueeze(1)).to(torch.bfloat16).double() * w[:, k].double().unsqueeze(1) * (idx[:, k] >= 0).unsqueeze(1)
+        want += term
+        mass += term.abs()
+    # one rounding to bf16 (half a step, 2^-9 of the value) of a sum of up to 8 fp32 products
+    return y, h, want, want.abs() * 2.0**-8 + mass * (16 * 2.0**-24)
+
+
+@pytest.mark.parametrize("mode", ["push", "pull", "reduced", "coded"])
+@pytest.mark.parametrize("at", [None, 0, 3, -2])  # out: elsewhere; at a row of x; two rows in front of x
+@pytest.mark.parametrize("tokens", [1, 130, 900])
+def test_combine_into_the_rows_it_reads(mode, at, tokens):
+    """Only x's own rows may be read before all of x has been: `out` may overlap x where nothing is loaded from x in place."""
+    H, E, K = 1024, 8, 4
+    dev = torch.device("cuda:0")
+    low_latency = mode != "reduced"
+    b = Buffer(0, 1, E, H, tokens, K, device=dev, low_latency_mode=low_latency)
+    b.connect_ranks()
+    for step in range(3):
+        x, idx, w = _routing(tokens, H, E, K, step)
+        idx[::3, 0] = -1
+        y, h, want, bound = _dispatched(b, x, idx, w, low_latency)
+        room = torch.empty(y.shape[0] + tokens + 8, H, device=dev, dtype=torch.bfloat16)
+        rows = room[2 : 2 + y.shape[0]]
+        rows.copy_(y)
+        out = None if at is None else room[2 + at : 2 + at + tokens]
+        if mode == "coded":
+            apart, _, _ = b.low_latency_combine(y, idx, w, h, use_logfmt=True)
+            got, _, _ = b.low_latency_combine(rows, idx, w, h, use_logfmt=True, out=out)
+            assert torch.equal(got, apart)
+            continue
+        if mode == "reduced":
+            got = b.combine(rows, idx, w, h, out=out)
+        else:  # pull: from rows outside the exposed region, which are staged there first
+            b.combine_pull = mode == "pull"
+            got, _, _ = b.low_latency_combine(rows, idx, w, h, out=out)
+        assert out is None or got.data_ptr() == out.data_ptr()
+        assert bool(((got.double() - want).abs() <= bound).all())
+    assert b.status == 0
+    b.destroy()
+
+
+@pytest.mark.parametrize("mode", ["push", "pull", "coded"])
+def test_combine_with_a_hook_writes_out_in_the_hook(mode):
+    T, H, E, K = 50, 1024, 8, 4
+    b = Buffer(0, 1, E, H, T, K, device=torch.device("cuda:0"), low_latency_mode=True)
+    b.connect_ranks()
+    x, idx, w = _routing(T, H, E, K, 5)
+    y, h, want, bound = _dispatched(b, x, idx, w, True)
+    coded = mode == "coded"
+    if mode == "pull":
+        b.get_next_combine_buffer(h).view(-1, H).copy_(y)
+        y = b.get_next_combine_buffer(h).view(-1, H)
+    now, _, _ = b.low_latency_combine(y, idx, w, h, use_logfmt=coded, zero_copy=mode == "pull")
+    out = torch.full((T, H), 7.0, device=x.device, dtype=torch.bfloat16)
+    got, _, hook = b.low_latency_combine(y, idx, w, h, use_logfmt=coded, zero_copy=mode == "pull", return_recv_hook=True, out=out)
+    torch.cuda.synchronize()
+    assert bool((out == 7.0).all())
+    if mode != "pull":
+        y.fill_(float("nan"))  # the send phase has read them
+    hook()
+    torch.cuda.synchronize()
+    assert torch.equal(out, now) and b.status == 0
+    if not coded:
+        assert bool(((out.double() - want).abs() <= bound).all())
+    b.destroy()
