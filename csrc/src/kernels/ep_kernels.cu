@@ -1146,9 +1146,11 @@ __global__ void __launch_bounds__(kThreads, NR <= 8 && !kCoded ? 3 : 2) epCombin
         // Lane k: row and weight of one copy, -1 when there is none.
         int row = -1;
         float weight = 0.f;
-        if (p.pull == 2) { // rank-reduced mode: rows and weights as the dispatch recorded them
+        if (p.pull == 2) { // rank-reduced mode: rows and weights as the dispatch recorded them, for tokens that still have an expert
             const NixlEpGroupRecord *rec = reinterpret_cast<const NixlEpGroupRecord *>(self + p.lay.off_grp) + t;
-            if (lane < 8 && !off && rec->pad[0] == static_cast<int>(p.epoch & 0x7fffffffull) && lane < rec->n) {
+            const long long e = lane < p.K ? p.topk_idx[t * p.K + lane] : -1;
+            const bool wanted = __any_sync(0xffffffffu, e >= 0 && e < p.E);
+            if (wanted && lane < 8 && !off && rec->pad[0] == static_cast<int>(p.epoch & 0x7fffffffull) && lane < rec->n) {
                 row = rec->rows[lane];
                 weight = rec->w[lane];
             }

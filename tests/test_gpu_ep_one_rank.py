@@ -162,3 +162,22 @@ def test_combine_with_a_hook_writes_out_in_the_hook(mode):
     if not coded:
         assert bool(((out.double() - want).abs() <= bound).all())
     b.destroy()
+
+
+def test_rank_reduced_combine_leaves_out_tokens_without_experts():
+    """Tokens whose slots the caller took out after the dispatch come back as zeros."""
+    T, H, E, K = 70, 1024, 8, 3
+    b = Buffer(0, 1, E, H, T, K, device=torch.device("cuda:0"))
+    b.connect_ranks()
+    x, idx, w = _routing(T, H, E, K, 9)
+    y, h, want, bound = _dispatched(b, x, idx, w, False)
+    fewer = idx.clone()
+    fewer[::4] = -1
+    fewer[1::4, 0] = -1  # (one slot: the recorded sum of the token stays)
+    got = b.combine(y, fewer, w, h)
+    assert bool((got[::4] == 0).all())
+    want[::4] = 0
+    assert bool(((got.double() - want).abs() <= bound).all())
+    overlapping = b.combine(y, fewer, w, h, out=y[1 : 1 + T])  # the path of larger groups
+    assert torch.equal(overlapping, got)
+    b.destroy()
