@@ -188,6 +188,14 @@ constexpr int kBatch = 32;  // tokens whose rows are looked up together, and rep
 constexpr int kSlices = 2;  // slices of a token in flight per warp: 2 KiB
 constexpr int kDispatchCtas = 4; // per SM, with many tokens
 
+// Shared memory of the dispatch: `tables` words per expert and the batch's rows.  Where three tables do not fit (above some
+// 19,000 experts) the rank's totals stay in global memory; two tables hold 28,000.
+constexpr size_t kDispatchSmemMax = 226 * 1024;
+__host__ __device__ __forceinline__ size_t dispatchSmem(int E, int K, int tables) {
+    return size_t(tables) * E * sizeof(int) + size_t(kBatch) * K * (sizeof(int) + 1) + 16;
+}
+__host__ __device__ __forceinline__ int dispatchTables(int E, int K) { return dispatchSmem(E, K, 3) <= kDispatchSmemMax ? 3 : 2; }
+
 __host__ __device__ __forceinline__ bool placesAreFixed(const NixlEpDispatchParams &p) { return p.R == 1 && p.rows_per_expert > 0 && p.phases == 3; }
 
 template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpDispatchParams &p, const int *rows, const unsigned char *dests, char *const *peer_sh,
@@ -290,12 +298,14 @@ template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpD
 __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(const __grid_constant__ NixlEpDispatchParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int El = p.E / p.R;
-    // shared: place[E] | ebase[E] | mine[E] | total[E] | rows[kBatch * K] | dests[kBatch * K]
+    // shared: place[E] | mine[E] | total[E] (unless there are too many experts) | rows[kBatch * K] | dests[kBatch * K]
     int *place = reinterpret_cast<int *>(smem); // row of this CTA's next copy to expert e at its receiver
-    int *ebase = place + p.E;
-    int *mine = ebase + p.E;                    // this CTA's copies per expert: of its whole range, then of a batch
+    int *mine = place + p.E;                    // this CTA's copies per expert: of its whole range, then of a batch
+    int *ebase = mine;                          // in between: first row of expert e at its receiver
+    const bool keep_totals = dispatchTables(p.E, p.K) == 3;
     int *total = mine + p.E;                    // the rank's copies per expert (all CTAs')
-    int *rows = total + p.E;
+    int *rows = keep_totals ? total + p.E : total;
+    auto totalOf = [&](int e) { return keep_totals ? total[e] : ldVolatile(p.scr.cnt + e); }; // (behind the grid barrier)
     unsigned char *dests = reinterpret_cast<unsigned char *>(rows + kBatch * p.K);
 
     char *self = peerBase(p.peers, p.rank);
@@ -323,13 +333,13 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         __syncthreads();
         for (int e = tid; e < p.E; e += kThreads) {
             place[e] = mine[e] ? atomicAdd(p.scr.cnt + e, mine[e]) : 0;
-            if (fixed) ebase[e] = e * p.rows_per_expert;
+            if (fixed) place[e] += e * p.rows_per_expert;
         }
         if (fixed) __syncthreads();
     }
     if ((p.phases & 1) && !fixed) {
         gridBarrier(p.scr.barrier, p.scr.status, p.timeout_ns);
-        for (int e = tid; e < p.E; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
+        for (int e = tid; e < p.E && keep_totals; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
         __syncthreads();
 
         // 2. all-gather of counts: CTA b serves destination ranks b, b+grid, ...
@@ -337,14 +347,14 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             char *peer = peer_sh[d];
             if (masked[d] != 0 || peer == nullptr) continue;
             int *dst = reinterpret_cast<int *>(peer + p.lay.off_counts) + static_cast<long long>(p.rank) * p.E;
-            for (int e = tid; e < p.E; e += kThreads) dst[e] = total[e];
+            for (int e = tid; e < p.E; e += kThreads) dst[e] = totalOf(e);
             if (tid == 0) reinterpret_cast<int *>(peer + p.lay.off_grp_tokens)[p.rank] = p.topk_weights != nullptr ? p.T : 0;
             // Experts of that rank that get nothing from us are complete right away.
             uint64_t *dflag = reinterpret_cast<uint64_t *>(peer + p.lay.off_disp_flag);
             __syncthreads(); // the release below covers the whole CTA's stores
             if (tid == 0) stReleaseSys(reinterpret_cast<uint64_t *>(peer + p.lay.off_counts_flag) + p.rank, p.epoch);
             for (int le = tid; le < El; le += kThreads)
-                if (total[d * El + le] == 0) stReleaseSys(dflag + static_cast<long long>(le) * p.R + p.rank, p.epoch);
+                if (totalOf(d * El + le) == 0) stReleaseSys(dflag + static_cast<long long>(le) * p.R + p.rank, p.epoch);
         }
     }
 
@@ -372,7 +382,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         for (int e = tid; e < p.E; e += kThreads) {
             int b = 0, all = 0;
             for (int r = 0; r < p.R; ++r) {
-                const int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e); // (loads of all ranks in flight together)
+                const int c = own ? totalOf(e) : ldVolatile(counts + static_cast<long long>(r) * p.E + e); // (loads of all ranks in flight together)
                 if (masked[r] != 0) continue;
                 if (r < p.rank) b += c;
                 all += c;
@@ -404,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 const int e = p.rank * El + le;
                 int all = 0;
                 for (int r = 0; r < p.R; ++r) {
-                    int c = own ? total[e] : ldVolatile(counts + static_cast<long long>(r) * p.E + e);
+                    int c = own ? totalOf(e) : ldVolatile(counts + static_cast<long long>(r) * p.E + e);
                     if (masked[r] != 0) c = 0;
                     p.layout_range[static_cast<long long>(le) * p.R + r] = (static_cast<long long>(all) << 32) | static_cast<unsigned>(c);
                     all += c;
@@ -414,6 +424,9 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 if (le == El - 1) p.expert_offsets[El] = ebase[e] + (p.rows_per_expert > 0 ? p.rows_per_expert : all);
             }
         }
+        if (p.phases & 1)
+            for (int e = tid; e < p.E; e += kThreads) place[e] += ebase[e];
+        __syncthreads(); // the first batch puts its counts where the first rows are
     }
 
     if (p.phases & 1) {
@@ -432,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 int dest = 0;
                 if (e >= 0 && e < p.E && masked[static_cast<int>(e) / El] == 0) {
                     dest = static_cast<int>(e) / El;
-                    row = static_cast<long long>(ebase[e]) + atomicAdd(place + e, 1);
+                    row = atomicAdd(place + e, 1);
                     if (row >= p.cap) row = -1; // flagged as ST_CAPACITY above
                     atomicAdd(mine + e, 1);     // counted as sent even then
                 }
@@ -450,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 if (c == 0) continue;
                 // One operation releases this CTA's rows and acquires the other CTAs'.
                 const int done = addAcqRelSys(p.scr.sent + e, c) + c;
-                if (done == total[e]) stReleaseSys(reinterpret_cast<uint64_t *>(peer_sh[e / El] + p.lay.off_disp_flag) + static_cast<long long>(e % El) * p.R + p.rank, p.epoch);
+                if (done == totalOf(e)) stReleaseSys(reinterpret_cast<uint64_t *>(peer_sh[e / El] + p.lay.off_disp_flag) + static_cast<long long>(e % El) * p.R + p.rank, p.epoch);
             }
         }
     }
@@ -491,8 +504,8 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 counts[e] = c;
                 p.recv_count[e] = c;
                 p.layout_range[e] = static_cast<unsigned>(c);
-                p.expert_offsets[e] = ebase[e];
-                if (e == p.E - 1) p.expert_offsets[p.E] = ebase[e] + p.rows_per_expert;
+                p.expert_offsets[e] = e * p.rows_per_expert;
+                if (e == p.E - 1) p.expert_offsets[p.E] = p.E * p.rows_per_expert;
             }
             if (tid == 0) reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
             // The flags go up behind all counts (of every warp) and, through the exit counter, all rows: a GEMM launched on
@@ -1250,13 +1263,13 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
     if (p.H % 512) return cudaErrorInvalidValue; // whole warps per pass; scales move as float4
     if (p.topk_weights && (p.K > 8 || p.R > 32 || p.max_tokens < p.T)) return cudaErrorInvalidValue; // a group record holds eight copies
     if (p.rows_per_expert > 0 && static_cast<long long>(p.rows_per_expert) < static_cast<long long>(p.R) * p.T) return cudaErrorInvalidValue;
-    const size_t smem = size_t(4) * p.E * sizeof(int) + size_t(kBatch) * p.K * (sizeof(int) + 1) + 16;
+    const size_t smem = dispatchSmem(p.E, p.K, dispatchTables(p.E, p.K));
     if (smem > 48 * 1024) { // many experts: the shared-memory limit is a per-device function attribute, raised once to all there is
         static bool attr_done[64] = {};
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-            const cudaError_t e = cudaFuncSetAttribute(epDispatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+            const cudaError_t e = cudaFuncSetAttribute(epDispatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDispatchSmemMax));
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 64) attr_done[dev] = true;
         }

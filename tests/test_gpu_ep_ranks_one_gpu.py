@@ -106,10 +106,12 @@ def test_dispatch_of_several_ranks(n, tokens, topk, hidden, low_latency, kind, n
         b.destroy()
 
 
-def test_dispatch_with_more_experts_than_the_default_shared_memory_holds():
-    n, El, tokens, topk, hidden = 6, 512, 40, 4, 512  # 16 bytes per expert: just above 48 KiB
+# 12 bytes per expert: below and just above 48 KiB, more than 16 bytes per expert would leave room for, and (8 bytes) more than 12 would
+@pytest.mark.parametrize("n", [6, 9, 30, 40])
+def test_dispatch_with_more_experts_than_the_default_shared_memory_holds(n):
+    El, tokens, topk, hidden = 512, 40, 4, 512
     experts = n * El
-    bufs = _ranks(n, experts, hidden, tokens, topk, "er_many", False)
+    bufs = _ranks(n, experts, hidden, tokens, topk, f"er_many{n}", False)
     dev = torch.device("cuda:0")
     g = torch.Generator(device=dev).manual_seed(5)
     xs = [torch.randn(tokens, hidden, device=dev, dtype=torch.bfloat16, generator=g) for _ in bufs]
