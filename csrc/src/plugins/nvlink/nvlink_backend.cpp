@@ -84,7 +84,8 @@ bool cudaOk(cudaError_t e, const char *what) {
     return false;
 }
 
-// cuMemGetAddressRange through the runtime's driver entry point (no link against libcuda).
+// cuMemGetAddressRange through the runtime's driver entry point (no link against libcuda): device allocations, and pinned host
+// memory as it was allocated or registered (not rounded to pages).
 bool allocationRange(uintptr_t ptr, uintptr_t &base, size_t &size) {
     using fn_t = int (*)(unsigned long long *, size_t *, unsigned long long);
     static fn_t fn = [] {
@@ -104,21 +105,29 @@ bool allocationRange(uintptr_t ptr, uintptr_t &base, size_t &size) {
     return true;
 }
 
-// Device address of host memory that is pinned from end to end already, 0 otherwise.  Looked at every 2 MiB, so that a
-// range that merely starts and ends in pinned memory is not taken for one.
-uintptr_t pinnedRange(uintptr_t addr, size_t len) {
+// Device address of host memory that is pinned from end to end already, 0 otherwise; `one` says whether a single allocation
+// (or registration) holds all of it.  Walked from allocation to allocation, so a hole of any size between two of them, or a
+// range that goes on behind the last one, is seen.
+uintptr_t pinnedRange(uintptr_t addr, size_t len, bool *one = nullptr) {
     uintptr_t first = 0;
-    for (size_t off = 0;; off = std::min(off + (size_t(2) << 20), len - 1)) {
+    cudaFree(nullptr); // make sure the thread has a context before driver calls
+    for (uintptr_t at = addr; at - addr < len;) {
         cudaPointerAttributes attr{};
-        if (cudaPointerGetAttributes(&attr, reinterpret_cast<void *>(addr + off)) != cudaSuccess || attr.type != cudaMemoryTypeHost || !attr.devicePointer) {
+        uintptr_t base = 0;
+        size_t size = 0;
+        if (cudaPointerGetAttributes(&attr, reinterpret_cast<void *>(at)) != cudaSuccess || attr.type != cudaMemoryTypeHost || !attr.devicePointer ||
+            !allocationRange(at, base, size) || base > at || size <= at - base) {
             cudaGetLastError();
             return 0;
         }
         const uintptr_t dp = reinterpret_cast<uintptr_t>(attr.devicePointer);
-        if (off == 0) first = dp;
-        else if (dp != first + off) return 0;
-        if (off == len - 1) return first;
+        if (at == addr) {
+            first = dp;
+            if (one) *one = size - (at - base) >= len;
+        } else if (dp - first != at - addr) return 0;
+        at = base + size;
     }
+    return first;
 }
 
 // UUID of a local GPU, looked up once per ordinal.
@@ -579,22 +588,19 @@ nixl_status_t Engine::registerMem(const nixlBlobDesc &mem, const nixl_mem_t &nix
             const int dev = primaryDevice_.load() >= 0 ? primaryDevice_.load() : 0;
             DeviceScope ds(dev);
             // Memory that its owner allocated pinned (cudaHostAlloc, torch's pin_memory) cannot be registered again, and need not be.
-            md->devVisible = pinnedRange(mem.addr, mem.len);
-            md->pinnedByOwner = md->devVisible != 0;
-            const cudaError_t e = md->devVisible ? cudaErrorHostMemoryAlreadyRegistered
-                                                 : cudaHostRegister(reinterpret_cast<void *>(mem.addr), mem.len, cudaHostRegisterPortable | cudaHostRegisterMapped);
-            if (e == cudaSuccess) md->pinnedByUs = true;
-            if (md->devVisible) {
-                // found above
-            } else if (e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered) {
-                cudaGetLastError();
+            md->devVisible = pinnedRange(mem.addr, mem.len, &md->pinnedByOwner);
+            if (!md->devVisible) {
+                md->pinnedByOwner = false;
+                const cudaError_t e = cudaHostRegister(reinterpret_cast<void *>(mem.addr), mem.len, cudaHostRegisterPortable | cudaHostRegisterMapped);
                 void *dp = nullptr;
-                if (cudaHostGetDevicePointer(&dp, reinterpret_cast<void *>(mem.addr), 0) == cudaSuccess)
-                    md->devVisible = reinterpret_cast<uintptr_t>(dp);
-                else cudaGetLastError();
-            } else {
-                cudaGetLastError();
-                NIXL_DEBUG << "NVLINK backend: DRAM region not pinned (" << cudaGetErrorString(e) << "); staged copies will be used";
+                if (e == cudaSuccess) {
+                    md->pinnedByUs = true;
+                    if (cudaHostGetDevicePointer(&dp, reinterpret_cast<void *>(mem.addr), 0) == cudaSuccess) md->devVisible = reinterpret_cast<uintptr_t>(dp);
+                    else cudaGetLastError();
+                } else { // "already registered" too: of a part only, or the range would have been found above
+                    cudaGetLastError();
+                    NIXL_DEBUG << "NVLINK backend: DRAM region not pinned (" << cudaGetErrorString(e) << "); staged copies will be used";
+                }
             }
         }
     } else {
@@ -710,10 +716,7 @@ nixl_status_t Engine::loadRemoteMD(const nixlBlobDesc &input, const nixl_mem_t &
             md->devVisible = pub.addr;
             md->ownerLocalDevice = pub.device;
         } else if (cuda_) {
-            void *dp = nullptr; // pinned by its owner? then kernels can touch it
-            if (cudaHostGetDevicePointer(&dp, reinterpret_cast<void *>(pub.addr), 0) == cudaSuccess)
-                md->devVisible = reinterpret_cast<uintptr_t>(dp);
-            else cudaGetLastError();
+            md->devVisible = pinnedRange(pub.addr, pub.len); // pinned by its owner? then kernels can touch it
         }
     } else if (nixl_mem == VRAM_SEG && cuda_ && pub.hasIpc == 1) {
         const std::string key(reinterpret_cast<const char *>(pub.ipc), sizeof(pub.ipc));

@@ -63,7 +63,7 @@ public:
     int device = -1;           // VRAM: CUDA ordinal
     uintptr_t devVisible = 0;  // address usable by kernels (VRAM: addr; pinned DRAM: mapped address; else 0)
     bool pinnedByUs = false;   // we called cudaHostRegister
-    bool pinnedByOwner = false; // DRAM that was pinned before it was registered here
+    bool pinnedByOwner = false; // DRAM that one allocation of its owner holds, pinned before it was registered here
     bool hasIpc = false;
     cudaIpcMemHandle_t ipc{};
     uint64_t ipcOffset = 0;    // addr - base of the enclosing allocation

@@ -141,10 +141,12 @@ struct Runtime {
         if (base) *base = it->first;
         return &it->second;
     }
-    bool isPinned(uintptr_t p) {
+    bool isPinned(uintptr_t p, uintptr_t *base = nullptr, size_t *size = nullptr) {
         auto it = pinned.upper_bound(p);
         if (it == pinned.begin()) return false;
         --it;
+        if (base) *base = it->first;
+        if (size) *size = it->second.size;
         return p < it->first + it->second.size;
     }
 };
@@ -609,10 +611,11 @@ cudaError_t cudaIpcCloseMemHandle(void *ptr) {
 static int fakeGetAddressRange(unsigned long long *base, size_t *size, unsigned long long ptr) {
     std::lock_guard<std::mutex> g(rt().mu);
     uintptr_t b = 0;
-    const Allocation *a = rt().findDevice(static_cast<uintptr_t>(ptr), &b);
-    if (!a) return 1;
+    size_t n = 0;
+    if (const Allocation *a = rt().findDevice(static_cast<uintptr_t>(ptr), &b)) n = a->size;
+    else if (!rt().isPinned(static_cast<uintptr_t>(ptr), &b, &n)) return 1; // (pinned host memory has a range too, as allocated or registered)
     if (base) *base = b;
-    if (size) *size = a->size;
+    if (size) *size = n;
     return 0;
 }
 

@@ -437,6 +437,72 @@ TEST_CASE(host_memory_pinned_and_pageable_to_and_from_a_gpu) {
     }
 }
 
+TEST_CASE(host_memory_counts_as_pinned_only_from_end_to_end) {
+    // Buffers whose owner pinned all of them, in one piece or in two that adjoin, can be seen by kernels; a buffer that
+    // merely starts and ends in pinned memory, or has a pageable tail, must not be handed to one.  A memory view says which.
+    const size_t kPage = 4096;
+    struct Piece { size_t at, len; };
+    struct Case { std::vector<Piece> pinned; bool visible; };
+    const std::vector<Case> cases = {
+        {{{0, 64 * kPage}}, true},                                  // all of it
+        {{{0, 20 * kPage}, {20 * kPage, 44 * kPage}}, true},        // two adjoining pieces
+        {{{0, 8 * kPage}, {56 * kPage, 8 * kPage}}, false},         // a hole
+        {{{0, 63 * kPage + 1}, {63 * kPage + 2, kPage - 2}}, false}, // of one byte
+        {{{0, 32 * kPage}}, false},                                 // a pageable tail
+        {{{32 * kPage, 32 * kPage}}, false},                        // a pageable start
+        {{}, true},                                                 // nobody's: the registration pins it
+    };
+    for (size_t c = 0; c < cases.size(); ++c) {
+        const std::string tag = "hp" + std::to_string(c);
+        void *raw = nullptr;
+        const size_t bytes = 64 * kPage;
+        CHECK_EQ(posix_memalign(&raw, kPage, bytes), 0);
+        auto *host = static_cast<uint8_t *>(raw);
+        for (const Piece &p : cases[c].pinned) CHECK_EQ(cudaHostRegister(host + p.at, p.len, 0), cudaSuccess);
+        nixlAgent a(tag + "_a", nixlAgentConfig(false)), b(tag + "_b", nixlAgentConfig(false));
+        nixlBackendH *ha = nullptr, *hb = nullptr;
+        CHECK_EQ(a.createBackend("NVLINK", {}, ha), NIXL_SUCCESS);
+        CHECK_EQ(b.createBackend("NVLINK", {}, hb), NIXL_SUCCESS);
+        nixl_reg_dlist_t rh(DRAM_SEG), rd(VRAM_SEG);
+        rh.addDesc(nixlBlobDesc(reinterpret_cast<uintptr_t>(host), bytes, 0, ""));
+        CHECK_EQ(b.registerMem(rh), NIXL_SUCCESS);
+        DevBuf dev(0, bytes, 0);
+        rd.addDesc(nixlBlobDesc(reinterpret_cast<uintptr_t>(dev.p), dev.bytes, 0, ""));
+        CHECK_EQ(a.registerMem(rd), NIXL_SUCCESS);
+        nixl_blob_t md;
+        std::string name;
+        b.getLocalMD(md);
+        CHECK_EQ(a.loadRemoteMD(md, name), NIXL_SUCCESS);
+        cudaSetDevice(0);
+        nixlMemViewH view = nullptr;
+        nixl_xfer_dlist_t local(DRAM_SEG); // as its owner sees it
+        local.addDesc(nixlBasicDesc(reinterpret_cast<uintptr_t>(host), bytes, 0));
+        CHECK_EQ(b.prepMemView(local, view) == NIXL_SUCCESS, cases[c].visible);
+        if (view) b.releaseMemView(view);
+        view = nullptr;
+        nixl_remote_dlist_t remote(DRAM_SEG); // and as another agent of the process does
+        remote.addDesc(nixlRemoteDesc(nixlBasicDesc(reinterpret_cast<uintptr_t>(host), bytes, 0), tag + "_b"));
+        CHECK_EQ(a.prepMemView(remote, view) == NIXL_SUCCESS, cases[c].visible);
+        if (view) a.releaseMemView(view);
+        // the bytes arrive either way
+        std::mt19937 rng(static_cast<unsigned>(c));
+        for (size_t i = 0; i < bytes; ++i) dev.p[i] = static_cast<uint8_t>(rng());
+        nixl_xfer_dlist_t l(VRAM_SEG), r(DRAM_SEG);
+        l.addDesc(nixlBasicDesc(reinterpret_cast<uintptr_t>(dev.p), bytes, 0));
+        r.addDesc(nixlBasicDesc(reinterpret_cast<uintptr_t>(host), bytes, 0));
+        nixlXferReqH *req = nullptr;
+        CHECK_EQ(a.createXferReq(NIXL_WRITE, l, r, tag + "_b", req), NIXL_SUCCESS);
+        CHECK(a.postXferReq(req) >= 0);
+        CHECK_EQ(waitDone(a, req), NIXL_SUCCESS);
+        CHECK(std::memcmp(host, dev.p, bytes) == 0);
+        CHECK_EQ(a.releaseXferReq(req), NIXL_SUCCESS);
+        CHECK_EQ(a.deregisterMem(rd), NIXL_SUCCESS);
+        CHECK_EQ(b.deregisterMem(rh), NIXL_SUCCESS);
+        for (const Piece &p : cases[c].pinned) CHECK_EQ(cudaHostUnregister(host + p.at), cudaSuccess);
+        std::free(raw);
+    }
+}
+
 TEST_CASE(a_request_still_running_cannot_be_posted_again) {
     Pair p({}, 4 << 20, 0, 0);
     cudaSetDevice(0);
