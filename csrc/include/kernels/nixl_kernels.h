@@ -229,8 +229,12 @@ typedef struct NixlGroupedGemmParams {
                                     (N % 256 == 0); 3: as 2 with power-of-two scales applied by the tensor core: scale_a and
                                     scale_w then point at biased exponent bytes (UE8M0), uint8 [a_rows][K/128] and
                                     [groups][N/128][K/128], K % 512 == 0 */
+    int32_t expected_rows;       /* about how many rows the groups have together (the counts themselves are on the device), for the
+                                    choice between 1 and 2; 0: as many as a has, which is too many where a is a buffer with room */
 } NixlGroupedGemmParams;
 
+/* The tile mode that a launch with these parameters takes (host only). */
+int nixl_grouped_gemm_fp8_mode(const NixlGroupedGemmParams *params);
 int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params, void *stream);
 
 /* ---------------------------------------------------------------- device API exercisers

@@ -407,6 +407,21 @@ bool nixl_gemm::makeTileMap(CUtensorMap *map, const void *base, uint64_t rows, u
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tile shape: CTA pairs with 256 x 256 tiles when the experts have more rows than one 128-row tile on average and the tiles are
+// enough for the 74 pairs; single CTAs with 128 x 128 tiles otherwise (a decode step, where most tiles hold a handful of rows,
+// and small products, which need every SM).  The rows are those the caller expects: a's own rows are the capacity of
+// the buffer after a dispatch.  Measured back to back, single / pair, us: 32 experts, N = K = 4096: 128 rows each 116 / 122, 200
+// rows 210 / 162, 512 rows 477 / 310; 16 experts, 512 x 2048: 256 rows (32 pair tiles) 14.8 / 18.7, 400 rows (50) 22.8 / 19.0;
+// 1 expert, 4096 x 7168, 512 rows (32) 27.5 / 35.1.  With the weights out of L2 and room for 160 rows each, 32 experts, N = K =
+// 4096: 4 rows each 113 / 125, 32 rows 116 / 123, 64 rows 115 / 125, 128 rows 119 / 125, 160 rows 197 / 152; 2048 x 7168: 32 rows
+// 111 / 121, 128 rows 117 / 123, 160 rows 166 / 149.
+extern "C" int nixl_grouped_gemm_fp8_mode(const NixlGroupedGemmParams *params) {
+    const NixlGroupedGemmParams &p = *params;
+    if (const int asked = p.tile_mode & 0xff) return asked;
+    const long long rows = p.expected_rows > 0 && p.expected_rows < p.a_rows ? p.expected_rows : p.a_rows;
+    return p.rows_per_expert == 0 && !p.counts_flag && p.N % 256 == 0 && rows > 128LL * p.groups && rows * p.N >= 40LL * 256 * 256 ? 2 : 1;
+}
+
 extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params, void *stream) {
     if (!params || !params->a || !params->w || !params->d || !params->scale_a || !params->scale_w || !params->status)
         return cudaErrorInvalidValue;
@@ -422,17 +437,7 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
         std::fprintf(stderr, "nixl_grouped_gemm_fp8_launch: cuTensorMapEncodeTiled failed\n");
         return cudaErrorInvalidValue;
     }
-    // Tile shape: CTA pairs with 256 x 256 tiles when the experts have more rows than one 128-row tile on average and the
-    // tiles are enough for the 74 pairs; single CTAs with 128 x 128 tiles otherwise (the expert-major low-latency layout,
-    // where most tiles hold a handful of rows, and small products, which need every SM).  Measured, single / pair, us:
-    // 32 experts, N = K = 4096: 128 rows each 116 / 122, 200 rows 210 / 162, 512 rows 477 / 310; 16 experts, 512 x 2048:
-    // 256 rows (32 pair tiles) 14.8 / 18.7, 400 rows (50) 22.8 / 19.0; 1 expert, 4096 x 7168, 512 rows (32) 27.5 / 35.1.
-    int mode = p.tile_mode & 0xff;
-    if (mode == 0)
-        mode = (p.rows_per_expert == 0 && !p.counts_flag && p.N % 256 == 0 && p.a_rows > 128LL * p.groups &&
-                static_cast<long long>(p.a_rows) * p.N >= 40LL * 256 * 256)
-            ? 2
-            : 1;
+    const int mode = nixl_grouped_gemm_fp8_mode(&p);
     if (mode == 3) {
         if (p.N % 256 || p.K % 512 || p.counts_flag || p.disp_flag) return cudaErrorInvalidValue;
         if ((reinterpret_cast<uintptr_t>(p.scale_a) | reinterpret_cast<uintptr_t>(p.scale_w)) & 3) return cudaErrorInvalidValue;

@@ -25,6 +25,7 @@ class _Params(ctypes.Structure):
         ("status", ctypes.c_void_p), ("disp_flag", ctypes.c_void_p), ("counts", ctypes.c_void_p),
         ("epoch", ctypes.c_uint64), ("timeout_ns", ctypes.c_uint64),
         ("counts_flag", ctypes.c_void_p), ("rows_per_expert", ctypes.c_int32), ("tile_mode", ctypes.c_int32),
+        ("expected_rows", ctypes.c_int32),
     ]
 
 
@@ -130,6 +131,7 @@ def grouped_gemm_fp8(
     overlapped: bool = False,
     rows_per_expert: int = 0,
     tile_mode: int = 0,
+    expected_rows: int = 0,
 ) -> torch.Tensor:
     """``out[rows of g] = dequant(a[rows]) @ dequant(w[g]).T`` in bf16.
 
@@ -140,7 +142,9 @@ def grouped_gemm_fp8(
     kernel then waits for the count exchange itself (``rows_per_expert`` names the layout) and
     ``grid`` should leave the dispatch's CTAs free (see ``Buffer.dispatch_gemm``).
     ``tile_mode``: 0 lets the library choose, 1 forces 128 x 128 tiles on single CTAs, 2 forces
-    256 x 256 tiles on CTA pairs (``N % 256 == 0``)."""
+    256 x 256 tiles on CTA pairs (``N % 256 == 0``).
+    ``expected_rows``: about how many rows the groups have together, for that choice; 0: what the ``Buffer`` whose dispatch
+    made ``row_count`` expects, else all rows of ``a``.  It does not change the result."""
     rows, K = a.shape
     G, N, K2 = w.shape
     if K != K2 or K % 128 or N % 128:
@@ -166,6 +170,7 @@ def grouped_gemm_fp8(
     p.row_start, p.row_count = row_start.data_ptr(), row_count.data_ptr()
     p.groups, p.N, p.K, p.a_rows, p.grid = G, N, K, rows, grid
     p.tile_mode = tile_mode
+    p.expected_rows = expected_rows or getattr(row_count, "_nixl_expected_rows", 0)
     p.status = status.data_ptr()
     if fused_with is not None:
         buf, handle = fused_with

@@ -528,6 +528,8 @@ class Buffer:
             _lib.launch_on(self.device, fn, ref, stream_ptr, "nixl_ep_dispatch_launch")
 
         launch(phases_now)
+        # What arrives when the ranks send alike; the buffer's rows say only what could.  The expert GEMM chooses its tiles by it.
+        recv_count._nixl_expected_rows = T * K
         hook = (lambda: launch(2)) if hook_later else None
         handle = EPHandle(parity, epoch, recv_count, expert_offsets, layout_range, src_info, self.max_tokens, H, K, send_row[:T], rows_per_expert,
                           has_group_records=topk_weights is not None)
