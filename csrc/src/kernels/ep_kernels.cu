@@ -1162,11 +1162,11 @@ __global__ void __launch_bounds__(kThreads, NR <= 8 && !kCoded ? 3 : 2) epCombin
         if (p.pull == 2) { // rank-reduced mode: rows and weights as the dispatch recorded them, for tokens that still have an expert
             const NixlEpGroupRecord *rec = reinterpret_cast<const NixlEpGroupRecord *>(self + p.lay.off_grp) + t;
             const long long e = lane < p.K ? p.topk_idx[t * p.K + lane] : -1;
-            const bool wanted = __any_sync(0xffffffffu, e >= 0 && e < p.E);
-            if (wanted && lane < 8 && !off && rec->pad[0] == static_cast<int>(p.epoch & 0x7fffffffull) && lane < rec->n) {
+            if (lane < 8 && !off && rec->pad[0] == static_cast<int>(p.epoch & 0x7fffffffull) && lane < rec->n) {
                 row = rec->rows[lane];
                 weight = rec->w[lane];
             }
+            if (!__any_sync(0xffffffffu, e >= 0 && e < p.E)) row = -1; // (looked at last: its load is in flight beside the record's)
         } else if (lane < p.K) {
             const long long e = p.topk_idx[t * p.K + lane];
             if (e >= 0 && e < p.E && !off) row = p.send_row[t * p.K + lane];

@@ -707,7 +707,7 @@ class Buffer:
         p.max_tokens = self.max_tokens
         p.use_logfmt = int(use_logfmt)
         p.send_row = handle.send_row.data_ptr() if handle.send_row is not None else None
-        p.x, p.x_rows = x_ptr, x.shape[0]
+        p.x, p.x_rows = x_ptr, x.size(0)
         p.recv_info = handle.src_info.data_ptr()
         p.recv_count, p.expert_offsets = handle.recv_count.data_ptr(), handle.expert_offsets.data_ptr()
         p.topk_idx, p.topk_weights, p.out = topk_idx.data_ptr(), topk_weights.data_ptr(), out.data_ptr()
