@@ -36,6 +36,14 @@ __device__ __forceinline__ uint64_t ldAcquireSys(const uint64_t *p) {
 __device__ __forceinline__ void stReleaseSys(uint64_t *p, uint64_t v) {
     asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ void stReleaseGpu(uint64_t *p, uint64_t v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned addAcqRelGpu(unsigned *p, unsigned v) {
+    unsigned old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
 __device__ __forceinline__ int addAcqRelSys(int *p, int v) {
     int old;
     asm volatile("atom.add.acq_rel.sys.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
@@ -486,13 +494,9 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
     if (p.phases & 1) {
         __shared__ int last;
         __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            last = atomicAdd(p.scr.barrier + 2, 1u) == gridDim.x - 1;
-            if (last) {
-                p.scr.barrier[2] = 0;
-                __threadfence(); // the other CTAs' counts and rows
-            }
+        if (tid == 0) { // releases this CTA's counts and rows, and acquires the others'
+            last = addAcqRelGpu(p.scr.barrier + 2, 1u) == gridDim.x - 1;
+            if (last) p.scr.barrier[2] = 0;
         }
         __syncthreads();
         if (last && fixed) {
@@ -509,10 +513,11 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             }
             if (tid == 0) reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
             // The flags go up behind all counts (of every warp) and, through the exit counter, all rows: a GEMM launched on
-            // another stream may look at them while this kernel runs.
+            // another stream may look at them while this kernel runs.  It runs on this GPU, the only one of the group, so the
+            // release needs no wider scope.
             __syncthreads();
-            for (int e = tid; e < p.E; e += kThreads) stReleaseSys(dflag + e, p.epoch);
-            if (tid == 0) stReleaseSys(reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag), p.epoch);
+            for (int e = tid; e < p.E; e += kThreads) stReleaseGpu(dflag + e, p.epoch);
+            if (tid == kThreads - 1) stReleaseGpu(reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag), p.epoch); // (beside the others, not behind)
         }
         if (last)
             for (int e = tid; e < p.E; e += kThreads) {
