@@ -303,17 +303,17 @@ template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpD
     }
 }
 
+template<bool kKeepTotals> // the rank's totals fit into shared memory
 __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(const __grid_constant__ NixlEpDispatchParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int El = p.E / p.R;
-    // shared: place[E] | mine[E] | total[E] (unless there are too many experts) | rows[kBatch * K] | dests[kBatch * K]
+    // shared: place[E] | mine[E] | total[E] (kKeepTotals) | rows[kBatch * K] | dests[kBatch * K]
     int *place = reinterpret_cast<int *>(smem); // row of this CTA's next copy to expert e at its receiver
     int *mine = place + p.E;                    // this CTA's copies per expert: of its whole range, then of a batch
     int *ebase = mine;                          // in between: first row of expert e at its receiver
-    const bool keep_totals = dispatchTables(p.E, p.K) == 3;
     int *total = mine + p.E;                    // the rank's copies per expert (all CTAs')
-    int *rows = keep_totals ? total + p.E : total;
-    auto totalOf = [&](int e) { return keep_totals ? total[e] : ldVolatile(p.scr.cnt + e); }; // (behind the grid barrier)
+    int *rows = kKeepTotals ? total + p.E : total;
+    auto totalOf = [&](int e) { return kKeepTotals ? total[e] : ldVolatile(p.scr.cnt + e); }; // (behind the grid barrier)
     unsigned char *dests = reinterpret_cast<unsigned char *>(rows + kBatch * p.K);
 
     char *self = peerBase(p.peers, p.rank);
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
     }
     if ((p.phases & 1) && !fixed) {
         gridBarrier(p.scr.barrier, p.scr.status, p.timeout_ns);
-        for (int e = tid; e < p.E && keep_totals; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
+        for (int e = tid; e < p.E && kKeepTotals; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
         __syncthreads();
 
         // 2. all-gather of counts: CTA b serves destination ranks b, b+grid, ...
@@ -1268,13 +1268,16 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
     if (p.H % 512) return cudaErrorInvalidValue; // whole warps per pass; scales move as float4
     if (p.topk_weights && (p.K > 8 || p.R > 32 || p.max_tokens < p.T)) return cudaErrorInvalidValue; // a group record holds eight copies
     if (p.rows_per_expert > 0 && static_cast<long long>(p.rows_per_expert) < static_cast<long long>(p.R) * p.T) return cudaErrorInvalidValue;
-    const size_t smem = dispatchSmem(p.E, p.K, dispatchTables(p.E, p.K));
+    const int tables = dispatchTables(p.E, p.K);
+    const size_t smem = dispatchSmem(p.E, p.K, tables);
+    const void *kernel = tables == 3 ? reinterpret_cast<const void *>(epDispatchKernel<true>) : reinterpret_cast<const void *>(epDispatchKernel<false>);
     if (smem > 48 * 1024) { // many experts: the shared-memory limit is a per-device function attribute, raised once to all there is
         static bool attr_done[64] = {};
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-            const cudaError_t e = cudaFuncSetAttribute(epDispatchKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDispatchSmemMax));
+            cudaError_t e = cudaFuncSetAttribute(epDispatchKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDispatchSmemMax));
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(epDispatchKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDispatchSmemMax));
             if (e != cudaSuccess) return e;
             if (dev >= 0 && dev < 64) attr_done[dev] = true;
         }
@@ -1290,12 +1293,11 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
         if (p.T >= 4 * sms) requested = kDispatchCtas * sms;
         else if (p.T < sms) requested = p.T > p.R ? p.T : p.R;
     }
-    const int grid = coopGrid(reinterpret_cast<const void *>(epDispatchKernel), requested, smem);
+    const int grid = coopGrid(kernel, requested, smem);
     void *args[] = {const_cast<NixlEpDispatchParams *>(params)};
     if (placesAreFixed(p)) // no CTA waits for another
-        return cudaLaunchKernel(reinterpret_cast<const void *>(epDispatchKernel), dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(epDispatchKernel), dim3(grid), dim3(kThreads), args, smem,
-                                       static_cast<cudaStream_t>(stream));
+        return cudaLaunchKernel(kernel, dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
+    return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *stream) {
