@@ -110,7 +110,11 @@ bool allocationRange(uintptr_t ptr, uintptr_t &base, size_t &size) {
 // range that goes on behind the last one, is seen.
 uintptr_t pinnedRange(uintptr_t addr, size_t len, bool *one = nullptr) {
     uintptr_t first = 0;
-    cudaFree(nullptr); // make sure the thread has a context before driver calls
+    int dev = 0; // make sure the thread has a context before driver calls (by a call that is allowed while a stream is captured)
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     for (uintptr_t at = addr; at - addr < len;) {
         cudaPointerAttributes attr{};
         uintptr_t base = 0;

@@ -36,6 +36,7 @@ def test_gemm_on_another_stream_takes_this_steps_counts_and_rows(tokens):
         side.synchronize()
         flags = b._region(h.parity, "off_disp_flag", E * 8).view(torch.int64)
         assert bool((flags == h.epoch).all()) and int(b._region(h.parity, "off_counts_flag", 8).view(torch.int64)) == h.epoch
+        assert count._nixl_expected_rows == idx.numel()  # by which a GEMM chooses its tiles
         want_count = torch.bincount(idx.reshape(-1), minlength=E).int()
         assert torch.equal(b._region(h.parity, "off_counts", E * 4).view(torch.int32), want_count) and torch.equal(count, want_count)
         a, sa = rx.view(-1, H), sc.view(-1, H // 128)
