@@ -112,7 +112,7 @@ typedef struct NixlEpGroupRecord {
 
 typedef struct NixlEpScratch { /* device memory private to the rank; zero before first use */
     int32_t *cnt;      /* [E] */
-    int32_t *fill;     /* [E] (not used by these kernels) */
+    int32_t *fill;     /* [E] not used; kept so that the record keeps its layout */
     int32_t *sent;     /* [E] */
     uint32_t *barrier; /* [4] grid barrier (two words), CTAs that have left a dispatch */
     int32_t *status;   /* [1] bit0: a peer timed out, bit1: grid barrier timed out, bit2: capacity exceeded */

@@ -10,8 +10,9 @@
 // all of TMEM) are in flight.  (Eight N = 128 instructions, one per slot, read A from shared memory twice and
 // were slower by an eighth.)  A tile with at most 128 rows left runs as M = 128 (tailTile).
 //
-// What bounds this kernel is partly power (the SM clock falls from 1.7 to 1.45 GHz under load) and otherwise not
-// the tensor pipe (four MMAs take 512 cycles, a step about 940) but promotion and the hand-offs around it:
+// What bounds this kernel is not the tensor pipe (four MMAs take 512 cycles, a step about 940) but promotion and the
+// hand-offs around it, since only two steps fit in TMEM; power comes second (the SM clock falls from 1.7 to 1.45 GHz under
+// load, and the block-scaled kernel takes 277 us under the same cap where this one takes 349):
 //  * the issuing thread polls one barrier per step.  full[s] collects the producer's arrival (with
 //    both CTAs' byte count) and one arrival from each of the pair's sixteen promotion warps, sent
 //    when the warp has read the two slots the step will overwrite;
@@ -337,7 +338,7 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
             }
         } else if (warp == 1 && lane == 0 && cta == 0) {
             // ------------------------------------------------------------ MMA issuer (even CTA)
-            // One poll per eight MMAs: full[s] completes when both CTAs' bytes have landed and all
+            // One poll per four MMAs: full[s] completes when both CTAs' bytes have landed and all
             // promotion warps of the pair have read the step's two TMEM slots.
             uint32_t s = 0, full_par = 0, sl = 0; // ring positions as counters: no divisions on this thread
             uint32_t ready = 0;

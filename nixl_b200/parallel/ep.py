@@ -249,7 +249,8 @@ class Buffer:
         self._store = store
 
     def set_num_sms(self, num_sms: int) -> None:
-        """CTAs the dispatch and combine kernels use (0: one per SM), leaving the rest to concurrent compute."""
+        """CTAs the dispatch and combine kernels use (the rank-reduced combine: two per one of these), leaving the rest to
+        concurrent compute.  0: by the number of tokens, up to four per SM."""
         self._num_sms = max(0, int(num_sms))
 
     @property
@@ -258,7 +259,8 @@ class Buffer:
 
     def get_dispatch_config(self, num_ranks: Optional[int] = None) -> dict:
         """Launch configuration in use (the reference returns tuned per-rank-count tables; here the kernels size
-        their per-token thread groups themselves and the only knob is the CTA count)."""
+        their per-token thread groups themselves and the only knob is the CTA count).  ``num_sms`` is what ``set_num_sms`` was
+        given, or the number of SMs, on each of which the kernels may then run several CTAs."""
         return {"num_sms": self._num_sms or torch.cuda.get_device_properties(self.device).multi_processor_count}
 
     get_combine_config = get_dispatch_config
