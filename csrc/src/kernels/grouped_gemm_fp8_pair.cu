@@ -44,6 +44,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels/grouped_gemm_internal.h"
+#include "kernels/programmatic_launch.cuh"
 #include "kernels/tcgen05_ptx.cuh"
 
 namespace {
@@ -241,6 +242,8 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
 
 __global__ void __launch_bounds__(kThreads, 1)
 groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA64, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+    nixl_pdl::allowNextKernel();
+    nixl_pdl::waitForPreviousKernel();
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
     Shared &sh = *reinterpret_cast<Shared *>(tiles + kStages * kStageBytes);
@@ -286,17 +289,13 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
                 next += c;
                 run += ((c + 2 * BM - 1) / (2 * BM)) * n_tiles;
             }
-        } else {
-            for (int g = 0; g < p.groups; ++g) {
-                const int c = p.row_count[g];
-                sh.tilePrefix[g] = run;
-                sh.rowStart[g] = p.row_start[g];
-                sh.rowCount[g] = c;
-                run += ((c + 2 * BM - 1) / (2 * BM)) * n_tiles;
-            }
+            sh.tilePrefix[p.groups] = run;
         }
-        sh.tilePrefix[p.groups] = run;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1 && !p.counts_flag) {
+        int most;
+        nixl_gemm::buildTileTable(p, n_tiles, [](int rows) { return (rows + 2 * BM - 1) / (2 * BM); }, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
     }
     if (warp == 2) {
         // Both CTAs of the pair issue the paired allocation from the same warp and shared offset.
@@ -419,7 +418,7 @@ cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorM
     static bool attr_done[64] = {};
     static int max_pairs[64] = {};
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -427,6 +426,7 @@ cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorM
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
+    attr[1] = nixl_pdl::overlapAttribute();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
@@ -449,5 +449,6 @@ cudaError_t nixl_gemm::launchPairKernel(const CUtensorMap &mapA, const CUtensorM
     const long long max_tiles = (static_cast<long long>(p.a_rows + 2 * BM - 1) / (2 * BM) + p.groups) * (p.N / BN);
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
+    cfg.numAttrs = p.counts_flag || p.disp_flag ? 1 : 2; // (one that waits for a dispatch on another stream: not before the stream's own turn)
     return cudaLaunchKernelEx(&cfg, groupedGemmPairKernel, mapA, mapA64, mapW, p);
 }

@@ -17,6 +17,9 @@ constexpr int kMaxGroups = 512;
 
 // 2-D tensor map over a row-major [rows, k] byte matrix, boxes of box_rows x 128 bytes, 128-byte swizzle.
 bool makeTileMap(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k, uint32_t box_rows = 128);
+// The same matrix as [k / 128][rows][128 bytes], boxes of two neighbouring 128-byte columns x 128 rows: they land one behind the
+// other, each as a box of the map above would.  A second column past the end of k is filled with zeros.
+bool makePairMap(CUtensorMap *map, const void *base, uint64_t rows, uint64_t k);
 
 // 256 x 256 tiles computed by CTA pairs (tcgen05 cta_group::2).  Same contract as the
 // single-CTA kernel; N must be a multiple of 256.  The maps of A have boxes of 128 and 64 rows, that of W 128.
@@ -28,6 +31,33 @@ cudaError_t launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapA64,
 cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
 
 #ifdef __CUDACC__
+// The tile table of a launch, built by one whole warp, 32 groups at a time: prefix[g] tiles come before group g, each of whose
+// tilesOf(rows) row tiles has n_tiles columns of tiles.  One thread that walked the groups took a load's latency for each.
+template<class TilesOf>
+__device__ __forceinline__ void buildTileTable(const NixlGroupedGemmParams &p, int n_tiles, TilesOf tilesOf, int *prefix, int *rowStart, int *rowCount, int &most) {
+    const int lane = threadIdx.x & 31;
+    int run = 0, top = 0;
+    for (int g0 = 0; g0 < p.groups; g0 += 32) {
+        const int g = g0 + lane;
+        const int count = g < p.groups ? p.row_count[g] : 0, start = g < p.groups ? p.row_start[g] : 0;
+        const int here = tilesOf(count) * n_tiles;
+        int upto = here;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += below;
+        }
+        if (g < p.groups) {
+            prefix[g] = run + upto - here;
+            rowStart[g] = start;
+            rowCount[g] = count;
+        }
+        run += __shfl_sync(0xffffffffu, upto, 31);
+        top = max(top, count);
+    }
+    if (lane == 0) prefix[p.groups] = run;
+    most = __reduce_max_sync(0xffffffffu, top);
+}
 // Waits (bounded) until the rows [lo, hi) of group g have arrived: rows of an expert are ordered by source rank, so for the
 // arrival flags of the sources whose rows intersect the range.  On expiry the host sees the status bit and the kernel
 // computes on what is there.
@@ -55,6 +85,21 @@ __device__ __forceinline__ void waitArrivals(const NixlGroupedGemmParams &p, int
 }
 // A scale of A: through the read-only path, unless a dispatch may have written it while this kernel was running already.
 __device__ __forceinline__ float ldScale(const float *s, bool fresh) { return fresh ? __ldcg(s) : __ldg(s); }
+// A row's scales of the four steps from ks on, in one load where they start at a multiple of 16 bytes.  The lanes of a warp read 32
+// rows, that is 32 lines, and each line costs a cycle of the memory that TMA and MMA work on too.
+__device__ __forceinline__ float4 ldScales4(const float *row, int ks, int k_steps, bool fresh) {
+    const float *s = row + ks;
+    if (ks + 4 <= k_steps && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
+        const float4 *v = reinterpret_cast<const float4 *>(s);
+        return fresh ? __ldcg(v) : __ldg(v);
+    }
+    float4 f;
+    f.x = ks < k_steps ? ldScale(s, fresh) : 0.f;
+    f.y = ks + 1 < k_steps ? ldScale(s + 1, fresh) : 0.f;
+    f.z = ks + 2 < k_steps ? ldScale(s + 2, fresh) : 0.f;
+    f.w = ks + 3 < k_steps ? ldScale(s + 3, fresh) : 0.f;
+    return f;
+}
 #endif
 
 } // namespace nixl_gemm

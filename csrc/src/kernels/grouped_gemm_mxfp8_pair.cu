@@ -44,6 +44,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels/grouped_gemm_internal.h"
+#include "kernels/programmatic_launch.cuh"
 #include "kernels/tcgen05_ptx.cuh"
 
 namespace {
@@ -200,6 +201,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     const uint32_t cta = clusterCtaRank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
+    nixl_pdl::allowNextKernel();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbarInit(&sh.full[s], 1);
@@ -213,22 +215,20 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
         mbarInit(&sh.tmemEmpty, 2 * kPromoWarps);
         sh.abort = 0;
         sh.chunksIssued = 0;
-        int run = 0;
-        for (int g = 0; g < p.groups; ++g) {
-            const int c = p.row_count[g];
-            const int tiles_g = (c + BT - 1) / BT; // equal tiles, rounded up to the MMA's granularity
-            sh.tilePrefix[g] = run;
-            sh.rowStart[g] = p.row_start[g];
-            sh.rowCount[g] = c;
-            sh.tileRows[g] = tiles_g > 0 ? ((c + tiles_g - 1) / tiles_g + 31) & ~31 : 32;
-            run += tiles_g * n_tiles;
-        }
-        sh.tilePrefix[p.groups] = run;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemU32(&sh.tmemBase)), "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    nixl_pdl::waitForPreviousKernel();
+    if (warp == 1) {
+        int most;
+        nixl_gemm::buildTileTable(p, n_tiles, [](int rows) { return (rows + BT - 1) / BT; }, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
+        for (int g = lane; g < p.groups; g += 32) { // (each lane wrote its groups' counts itself)
+            const int c = sh.rowCount[g], tiles_g = (c + BT - 1) / BT; // equal tiles, rounded up to the MMA's granularity
+            sh.tileRows[g] = tiles_g > 0 ? ((c + tiles_g - 1) / tiles_g + 31) & ~31 : 32;
+        }
     }
     tcFenceBefore();
     __syncthreads();
@@ -453,7 +453,7 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtenso
     static bool attr_done[64] = {};
     static int max_pairs[64] = {};
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -461,6 +461,7 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtenso
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
+    attr[1] = nixl_pdl::overlapAttribute();
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (dev >= 0 && dev < 64 && !attr_done[dev]) {
@@ -482,5 +483,6 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtenso
     const long long max_tiles = (static_cast<long long>(p.a_rows + BT - 1) / BT + p.groups) * (p.N / (2 * BW));
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapT32, mapT64, mapW, p);
 }

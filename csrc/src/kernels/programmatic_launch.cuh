@@ -1,0 +1,40 @@
+// Launches whose beginning overlaps the end of the kernel in front of them in the stream (programmatic dependent launch).
+//
+// The later kernel's CTAs become resident once every CTA of the earlier one has called allowNextKernel() or has left, and set
+// themselves up; whatever an earlier kernel of the stream may have written is touched only behind waitForPreviousKernel(), which
+// returns when that kernel is complete and its stores are visible.  Every kernel launched this way calls it, in every CTA, so
+// that a kernel that is complete implies that all before it in the stream are.
+#ifndef NIXL_B200_PROGRAMMATIC_LAUNCH_CUH
+#define NIXL_B200_PROGRAMMATIC_LAUNCH_CUH
+
+#include <cuda_runtime.h>
+
+namespace nixl_pdl {
+
+__device__ __forceinline__ void waitForPreviousKernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allowNextKernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+inline cudaLaunchAttribute overlapAttribute() {
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    return a;
+}
+
+// Launches a kernel that calls waitForPreviousKernel().
+template<class... Params, class... Args>
+cudaError_t launch(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Args &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = overlapAttribute();
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
+} // namespace nixl_pdl
+
+#endif

@@ -55,6 +55,7 @@ def test_matches_reference(G, N, K, counts, gap):
         (2, 512, 512, [300, 57], 0),
         (4, 256, 1024, [0, 600, 1, 129], 5),
         (3, 512, 7168, [64, 257, 512], 0),
+        (36, 256, 256, [(11 * i) % 50 for i in range(36)], 0),
     ],
 )
 def test_cta_pair_tiles_match_reference(G, N, K, counts, gap):
@@ -62,9 +63,24 @@ def test_cta_pair_tiles_match_reference(G, N, K, counts, gap):
     _check(G, N, K, counts, gap, tile_mode=2)
 
 
-def _check(G, N, K, counts, gap, tile_mode):
+@pytest.mark.parametrize("expected_rows", [0, 1])  # A on the MMA's M side (the gaps make room for many rows), and W there
+@pytest.mark.parametrize(
+    "G,N,K,counts,grid",
+    [
+        (1, 128, 128, [5], 0),                              # one step: half a stage
+        (2, 256, 384, [33, 20], 1),                         # odd steps, several tiles in turn on one CTA
+        (3, 256, 640, [20, 32, 7], 2),                      # boxes of 32 rows only
+        (5, 384, 896, [64, 130, 33, 65, 16], 2),            # boxes of 32, 64 and 128 rows, several row tiles
+        (40, 128, 256, [(7 * i) % 40 for i in range(40)], 3),   # a tile table of more than one warp's width, with empty groups
+    ],
+)
+def test_stages_of_two_steps(G, N, K, counts, grid, expected_rows):
+    _check(G, N, K, counts, 130, tile_mode=1, grid=grid, expected_rows=expected_rows)
+
+
+def _check(G, N, K, counts, gap, tile_mode, grid=0, expected_rows=0):
     a, sa, wq, sw, rs, rc = _case(G, N, K, counts, gap)
-    out = grouped_gemm_fp8(a, sa, wq, sw, rs, rc, tile_mode=tile_mode)
+    out = grouped_gemm_fp8(a, sa, wq, sw, rs, rc, tile_mode=tile_mode, grid=grid, expected_rows=expected_rows)
     torch.cuda.synchronize()
     assert int(out._nixl_status.item()) == 0
     want = reference_grouped_gemm(a, sa, wq, sw, rs, rc)
@@ -87,6 +103,7 @@ def _check(G, N, K, counts, gap, tile_mode):
         (2, 512, 1536, [300, 57], 0),
         (4, 256, 1024, [0, 600, 1, 129], 3),
         (3, 512, 7168, [64, 257, 512], 0),
+        (36, 256, 512, [(11 * i) % 50 for i in range(36)], 0),
     ],
 )
 def test_block_scaled_tiles_match_reference(G, N, K, counts, gap):
