@@ -11,6 +11,7 @@
 
 #include "device/nixl_device_layout.h"
 #include "kernels/nixl_kernels.h"
+#include "kernels/programmatic_launch.cuh"
 
 namespace {
 
@@ -306,6 +307,8 @@ template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpD
 template<bool kKeepTotals> // the rank's totals fit into shared memory
 __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(const __grid_constant__ NixlEpDispatchParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
+    nixl_pdl::allowNextKernel();
+    nixl_pdl::waitForPreviousKernel();
     const int El = p.E / p.R;
     // shared: place[E] | mine[E] | total[E] (kKeepTotals) | rows[kBatch * K] | dests[kBatch * K]
     int *place = reinterpret_cast<int *>(smem); // row of this CTA's next copy to expert e at its receiver
@@ -1151,6 +1154,8 @@ __device__ __forceinline__ void localRowsCoded(int n, const uint4 *const (&src)[
 
 template <int NR, bool kCoded>
 __global__ void __launch_bounds__(kThreads, NR <= 8 && !kCoded ? 3 : 2) epCombineLocal(const __grid_constant__ NixlEpCombineParams p, int parts) {
+    nixl_pdl::allowNextKernel();
+    nixl_pdl::waitForPreviousKernel();
     const int lane = threadIdx.x & 31;
     const int vecs = p.H / 8;
     const char *self = peerBase(p.peers, p.rank);
@@ -1296,7 +1301,7 @@ extern "C" int nixl_ep_dispatch_launch(const NixlEpDispatchParams *params, void 
     const int grid = coopGrid(kernel, requested, smem);
     void *args[] = {const_cast<NixlEpDispatchParams *>(params)};
     if (placesAreFixed(p)) // no CTA waits for another
-        return cudaLaunchKernel(kernel, dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
+        return nixl_pdl::launch(tables == 3 ? epDispatchKernel<true> : epDispatchKernel<false>, grid, kThreads, smem, static_cast<cudaStream_t>(stream), p);
     return cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), args, smem, static_cast<cudaStream_t>(stream));
 }
 
@@ -1330,15 +1335,9 @@ extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *s
         parts = parts < 1 ? 1 : parts > most ? (most > 0 ? most : 1) : parts;
         const long long want = static_cast<long long>(p.T) * parts;
         const int grid = static_cast<int>(want < ctas ? want : ctas);
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        if (p.K <= 8) {
-            if (p.use_logfmt) epCombineLocal<8, true><<<grid, kThreads, 0, st>>>(p, parts);
-            else epCombineLocal<8, false><<<grid, kThreads, 0, st>>>(p, parts);
-        } else {
-            if (p.use_logfmt) epCombineLocal<kMaxTopk, true><<<grid, kThreads, 0, st>>>(p, parts);
-            else epCombineLocal<kMaxTopk, false><<<grid, kThreads, 0, st>>>(p, parts);
-        }
-        return cudaGetLastError();
+        const auto kernel = p.K <= 8 ? (p.use_logfmt ? epCombineLocal<8, true> : epCombineLocal<8, false>)
+                                     : (p.use_logfmt ? epCombineLocal<kMaxTopk, true> : epCombineLocal<kMaxTopk, false>);
+        return nixl_pdl::launch(kernel, grid, kThreads, 0, static_cast<cudaStream_t>(stream), p, parts);
     }
     if (p.pull == 2) {
         int dev = 0, sms = 0;

@@ -1,10 +1,13 @@
 // Fused paged-KV-cache transfer kernel (see include/kernels/nixl_kernels.h for the contract).
 // The data movement itself is in kv_xfer_body.cuh, shared with the allocation-free entry point.
 #include "kernels/kv_xfer_body.cuh"
+#include "kernels/programmatic_launch.cuh"
 
 namespace {
 
 template<bool kCast, int kVec> __global__ void __launch_bounds__(nixl_kv::kKvThreads, 4) kvXferKernel(const __grid_constant__ nixl_kv::KvPlan k) {
+    nixl_pdl::allowNextKernel();
+    nixl_pdl::waitForPreviousKernel();
     nixl_kv::moveBlocks<kCast, kVec>(k, k.p.src_blocks, k.p.dst_blocks);
     nixl_kv::signalWhenAllDone(k.p, k.p.done_counter);
 }
@@ -21,12 +24,8 @@ extern "C" int nixl_kv_xfer_launch(const NixlKvXferParams *params, void *stream)
     const nixl_kv::KvPlan k = nixl_kv::planFor(p);
     const int grid = nixl_kv::gridFor(k, dev);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (p.cast_fp8) {
-        if (k.vec_bytes == 32) kvXferKernel<true, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
-        else kvXferKernel<true, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
-    } else {
-        if (k.vec_bytes == 32) kvXferKernel<false, 32><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
-        else kvXferKernel<false, 16><<<grid, nixl_kv::kKvThreads, 0, s>>>(k);
-    }
-    return static_cast<int>(cudaGetLastError());
+    const auto kernel = p.cast_fp8 ? (k.vec_bytes == 32 ? kvXferKernel<true, 32> : kvXferKernel<true, 16>)
+                                   : (k.vec_bytes == 32 ? kvXferKernel<false, 32> : kvXferKernel<false, 16>);
+    // Requests posted one behind another: the next one's CTAs move in as this one's leave.
+    return static_cast<int>(nixl_pdl::launch(kernel, grid, nixl_kv::kKvThreads, 0, s, k));
 }
