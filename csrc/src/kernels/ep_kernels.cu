@@ -135,6 +135,26 @@ __device__ __forceinline__ void gridBarrier(unsigned *bar, int *status, uint64_t
     __syncthreads();
 }
 
+// The same for a kernel whose last CTA sets the word back to zero when all have left: one operation to arrive, no generation to read.
+__device__ __forceinline__ void gridBarrierOnce(unsigned *bar, int *status, uint64_t timeout_ns) {
+    __syncthreads();
+    if (threadIdx.x == 0 && addAcqRelGpu(bar, 1u) + 1 < gridDim.x) {
+        uint64_t t0 = 0;
+        unsigned spins = 0;
+        while (ldAcquireGpu(bar) < gridDim.x) {
+            if ((++spins & 63u) == 0) {
+                const uint64_t now = nowNs();
+                if (t0 == 0) t0 = now;
+                else if (now - t0 > timeout_ns) {
+                    atomicOr(status, ST_BARRIER_TIMEOUT);
+                    break;
+                }
+            }
+        }
+    }
+    __syncthreads();
+}
+
 // Threads cooperating on one token / row: as many as keeps the whole grid busy, a power of two
 // between one warp and one CTA.
 __device__ __forceinline__ int threadsPerItem(long long items) {
@@ -193,9 +213,14 @@ __device__ __forceinline__ uint4 quantGroup(const uint4 &lo, const uint4 &hi, bo
 // Measured on one B200, one rank, 32 experts, top-8, before / now: 4096 tokens x 7168 bf16 131 / 113 us (528 MB, 4.7 TB/s; the
 // rows written, 470 MB, are the bound), fp8 97 / 73 us, 4096 x 4096 fp8 74 / 47 us (3.6 TB/s); 128 tokens x 7168 fp8, low-latency
 // layout 21.6 / 13.4 us (8.4 with fixed places); 1 token 20.5 / 11.9 us (7.8).
+// A group of one rank then dropped what only other ranks need (flags early, rows counted as sent), and every group reads the
+// routing once, arrives at the grid barrier with one operation and calls its rows into L2 while it counts.  Compact layout, 32
+// experts, top-8, us before / after: 1 token 17.9 / 11.0, 300 x 4096 bf16 18.1 / 15.5, 700 29.5 / 19.8, 1500 40.3 / 32.0; 4096 x 4096
+// with power-of-two scales 47.2 / 39.8, 4096 x 7168 bf16 116 / 114 (bound by the writes to some 4700 rows that are open at a time).
 constexpr int kBatch = 32;  // tokens whose rows are looked up together, and reported as sent together
 constexpr int kSlices = 2;  // slices of a token in flight per warp: 2 KiB
 constexpr int kDispatchCtas = 4; // per SM, with many tokens
+constexpr int kPrefetch = 8;     // tokens of a CTA that are called into L2 while the copies are counted (58 MB of 4096 x 7168)
 
 // Shared memory of the dispatch: `tables` words per expert and the batch's rows.  Where three tables do not fit (above some
 // 19,000 experts) the rank's totals stay in global memory; two tables hold 28,000.
@@ -332,14 +357,23 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
     // out publishes the counts.  13.4 -> 8.4 us for 128 tokens x 7168, 11.9 -> 7.8 us for one token.
     const bool fixed = placesAreFixed(p);
     const long long t_first = static_cast<long long>(p.T) * blockIdx.x / gridDim.x, t_end = static_cast<long long>(p.T) * (blockIdx.x + 1) / gridDim.x;
+    // A group of one rank that sends in this launch has everybody's counts, its own, from the grid barrier, and sends every
+    // row itself: it waits for no flag and counts no rows as sent, and the last CTA out raises all flags.  (A launch that only
+    // receives waits for the flags like any other: the caller may have sent on another stream.)
+    const bool own = p.R == 1 && (p.phases & 1);
 
     if (p.phases & 1) {
         // 1. this CTA's copies per expert, and its place among the rank's
+        const int n_copies = static_cast<int>(t_end - t_first) * p.K;
+        for (int at = tid * 128; at < min(static_cast<int>(t_end - t_first), kPrefetch) * p.H * 2; at += kThreads * 128)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char *>(p.x) + t_first * p.H * 2 + at));
         for (int e = tid; e < p.E; e += kThreads) mine[e] = 0;
         __syncthreads();
-        for (long long i = t_first * p.K + tid; i < t_end * p.K; i += kThreads) {
-            const long long e = p.topk_idx[i];
-            if (e >= 0 && e < p.E && masked[static_cast<int>(e) / El] == 0) atomicAdd(mine + e, 1);
+        for (int i = tid; i < n_copies; i += kThreads) {
+            const long long e = p.topk_idx[t_first * p.K + i];
+            const bool valid = e >= 0 && e < p.E;
+            if (valid && masked[static_cast<int>(e) / El] == 0) atomicAdd(mine + e, 1);
+            if (i < kBatch * p.K) rows[i] = valid ? static_cast<int>(e) : -1; // (the first batch's experts: read once)
         }
         __syncthreads();
         for (int e = tid; e < p.E; e += kThreads) {
@@ -349,7 +383,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         if (fixed) __syncthreads();
     }
     if ((p.phases & 1) && !fixed) {
-        gridBarrier(p.scr.barrier, p.scr.status, p.timeout_ns);
+        gridBarrierOnce(p.scr.barrier, p.scr.status, p.timeout_ns);
         for (int e = tid; e < p.E && kKeepTotals; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
         __syncthreads();
 
@@ -361,6 +395,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             for (int e = tid; e < p.E; e += kThreads) dst[e] = totalOf(e);
             if (tid == 0) reinterpret_cast<int *>(peer + p.lay.off_grp_tokens)[p.rank] = p.topk_weights != nullptr ? p.T : 0;
             // Experts of that rank that get nothing from us are complete right away.
+            if (own) break; // the flags go up at the end
             uint64_t *dflag = reinterpret_cast<uint64_t *>(peer + p.lay.off_disp_flag);
             __syncthreads(); // the release below covers the whole CTA's stores
             if (tid == 0) stReleaseSys(reinterpret_cast<uint64_t *>(peer + p.lay.off_counts_flag) + p.rank, p.epoch);
@@ -369,9 +404,6 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         }
     }
 
-    // A group of one rank that sends in this launch has everybody's counts, its own, from the grid barrier, and sends every
-    // row itself.  (A launch that only receives waits for the flags like any other: the caller may have sent on another stream.)
-    const bool own = p.R == 1 && (p.phases & 1);
     // 3. wait for everybody's counts (every CTA looks for itself: 8 flags, no grid barrier needed)
     if (!fixed) {
         const uint64_t *cflag = reinterpret_cast<const uint64_t *>(self + p.lay.off_counts_flag);
@@ -407,15 +439,24 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 if (ebase[e] > p.rows_per_expert) atomicOr(p.scr.status, ST_CAPACITY);
             __syncthreads();
             for (int e = tid; e < p.E; e += kThreads) ebase[e] = (e % El) * p.rows_per_expert;
-        } else if (tid < p.R) {
-            // exclusive prefix over the local experts of destination rank `tid`
-            int run = 0;
-            for (int le = 0; le < El; ++le) {
-                const int c = ebase[tid * El + le];
-                ebase[tid * El + le] = run;
-                run += c;
+        } else {
+            // exclusive prefix over the local experts of a destination rank, a warp per rank
+            const int lane = tid & 31;
+            for (int r = tid >> 5; r < p.R; r += kThreads / 32) {
+                int run = 0;
+                for (int l0 = 0; l0 < El; l0 += 32) {
+                    const int c = l0 + lane < El ? ebase[r * El + l0 + lane] : 0;
+                    int upto = c;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                        if (lane >= o) upto += below;
+                    }
+                    if (l0 + lane < El) ebase[r * El + l0 + lane] = run + upto - c;
+                    run += __shfl_sync(0xffffffffu, upto, 31);
+                }
+                if (lane == 0 && run > p.cap) atomicOr(p.scr.status, ST_CAPACITY);
             }
-            if (run > p.cap) atomicOr(p.scr.status, ST_CAPACITY);
         }
         __syncthreads();
 
@@ -451,25 +492,28 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             for (int e = tid; e < p.E; e += kThreads) mine[e] = 0;
             __syncthreads();
             for (int i = tid; i < n * p.K; i += kThreads) {
-                const long long e = p.topk_idx[tb * p.K + i];
-                long long row = -1;
-                int dest = 0;
-                if (e >= 0 && e < p.E && masked[static_cast<int>(e) / El] == 0) {
-                    dest = static_cast<int>(e) / El;
+                int e = rows[i];
+                if (tb != t_first) {
+                    const long long wide = p.topk_idx[tb * p.K + i];
+                    e = wide >= 0 && wide < p.E ? static_cast<int>(wide) : -1;
+                }
+                int row = -1, dest = 0;
+                if (e >= 0 && masked[e / El] == 0) {
+                    dest = e / El;
                     row = atomicAdd(place + e, 1);
                     if (row >= p.cap) row = -1; // flagged as ST_CAPACITY above
                     atomicAdd(mine + e, 1);     // counted as sent even then
                 }
-                rows[i] = static_cast<int>(row);
+                rows[i] = row;
                 dests[i] = static_cast<unsigned char>(dest);
-                if (p.send_row != nullptr) p.send_row[tb * p.K + i] = static_cast<int>(row);
+                if (p.send_row != nullptr) p.send_row[tb * p.K + i] = row;
             }
             __syncthreads();
             if (p.use_fp8) dispatchTokens<true>(p, rows, dests, peer_sh, tb, n, parts);
             else dispatchTokens<false>(p, rows, dests, peer_sh, tb, n, parts);
             __syncthreads(); // all stores of the batch issued (and its tables free for the next one)
             // Count the batch's rows as sent.  Whoever completes an expert's rows raises that expert's arrival flag at its rank.
-            for (int e = tid; e < p.E && !fixed; e += kThreads) {
+            for (int e = tid; e < p.E && !own; e += kThreads) {
                 const int c = mine[e];
                 if (c == 0) continue;
                 // One operation releases this CTA's rows and acquires the other CTAs'.
@@ -499,12 +543,11 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         __syncthreads();
         if (tid == 0) { // releases this CTA's counts and rows, and acquires the others'
             last = addAcqRelGpu(p.scr.barrier + 2, 1u) == gridDim.x - 1;
-            if (last) p.scr.barrier[2] = 0;
+            if (last) p.scr.barrier[0] = p.scr.barrier[2] = 0;
         }
         __syncthreads();
         if (last && fixed) {
             int *counts = reinterpret_cast<int *>(self + p.lay.off_counts);
-            uint64_t *dflag = reinterpret_cast<uint64_t *>(self + p.lay.off_disp_flag);
             for (int e = tid; e < p.E; e += kThreads) {
                 const int c = ldVolatile(p.scr.cnt + e);
                 if (c > p.rows_per_expert) atomicOr(p.scr.status, ST_CAPACITY);
@@ -515,11 +558,13 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
                 if (e == p.E - 1) p.expert_offsets[p.E] = p.E * p.rows_per_expert;
             }
             if (tid == 0) reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
+        }
+        if (last && own && (fixed || masked[0] == 0)) {
             // The flags go up behind all counts (of every warp) and, through the exit counter, all rows: a GEMM launched on
             // another stream may look at them while this kernel runs.  It runs on this GPU, the only one of the group, so the
             // release needs no wider scope.
             __syncthreads();
-            for (int e = tid; e < p.E; e += kThreads) stReleaseGpu(dflag + e, p.epoch);
+            for (int e = tid; e < p.E; e += kThreads) stReleaseGpu(reinterpret_cast<uint64_t *>(self + p.lay.off_disp_flag) + e, p.epoch);
             if (tid == kThreads - 1) stReleaseGpu(reinterpret_cast<uint64_t *>(self + p.lay.off_counts_flag), p.epoch); // (beside the others, not behind)
         }
         if (last)

@@ -182,3 +182,31 @@ def test_rank_reduced_combine_leaves_out_tokens_without_experts():
     overlapping = b.combine(y, fewer, w, h, out=y[1 : 1 + T])  # the path of larger groups
     assert torch.equal(overlapping, got)
     b.destroy()
+
+
+@pytest.mark.parametrize("tokens,experts,topk,sms", [(1, 5, 1, 0), (70, 33, 4, 1), (150, 100, 8, 2), (700, 64, 3, 0), (2500, 32, 8, 0)])
+def test_compact_dispatch_places_every_copy_once(tokens, experts, topk, sms):
+    """Few CTAs (several batches of tokens each), more experts than a warp's width, slots without an expert."""
+    H = 512
+    b = Buffer(0, 1, experts, H, tokens, topk, device=torch.device("cuda:0"), low_latency_mode=False, timeout_ms=1000)
+    b.connect_ranks()
+    b.set_num_sms(sms)
+    for step in range(3):
+        x, idx, w = _routing(tokens, H, experts, topk, 10 + step)
+        idx[step::7] = -1
+        recv, _, h = b.dispatch(x, idx, use_fp8=False, topk_weights=w)
+        torch.cuda.synchronize()
+        assert b.status == 0
+        want = torch.bincount(idx[idx >= 0], minlength=experts)
+        start = torch.cumsum(want, 0) - want
+        assert torch.equal(h.recv_count, want.int()) and torch.equal(h.expert_offsets[:experts], start.int())
+        assert int(h.expert_offsets[experts]) == int(want.sum())
+        flags = b._region(h.parity, "off_disp_flag", experts * 8).view(torch.int64)
+        assert bool((flags == h.epoch).all()) and int(b._region(h.parity, "off_counts_flag", 8).view(torch.int64)) == h.epoch
+        t, k = torch.nonzero(idx >= 0, as_tuple=True)
+        rows = h.send_row[t, k].long()
+        assert torch.equal(torch.sort(rows).values, torch.arange(rows.numel(), device=rows.device))  # each row once
+        assert bool(((rows >= start[idx[t, k]]) & (rows < (start + want)[idx[t, k]])).all())          # among its expert's
+        assert torch.equal(recv[rows], x[t])
+        assert torch.equal(h.src_info[rows, 1].long(), t * topk + k)
+    b.destroy()
