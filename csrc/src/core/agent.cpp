@@ -551,28 +551,39 @@ nixl_status_t nixlAgent::makeXferReq(const nixl_xfer_op_t &operation, const nixl
     req->initiatorDescs->reserve(local_indices.size());
     req->targetDescs->reserve(local_indices.size());
     size_t total = 0;
+    // The run of the previous index is looked at first: a request names many blocks of few runs.
+    const nixlStrideDesc *l_run = nullptr, *r_run = nullptr;
+    auto inRun = [](const nixlStrideDesc *run, size_t i) { return run && i - run->start_idx < run->count; }; // (below its start: wraps around)
+    nixl_meta_dlist_t &ours = *req->initiatorDescs, &theirs = *req->targetDescs;
+    size_t l_prev = 0, r_prev = 0;
     for (size_t k = 0; k < local_indices.size(); ++k) {
-        const nixlMetaDesc l = L.find(local_indices[k]).getMetaDesc(local_indices[k], 1);
-        const nixlMetaDesc r = R.find(remote_indices[k]).getMetaDesc(remote_indices[k], 1);
-        if (l.len != r.len) {
+        const size_t li = static_cast<size_t>(local_indices[k]), ri = static_cast<size_t>(remote_indices[k]);
+        if (!inRun(l_run, li)) l_run = &L.find(li);
+        if (!inRun(r_run, ri)) r_run = &R.find(ri);
+        const size_t len = l_run->len;
+        if (len != r_run->len) {
             data->noteError(NIXL_ERR_INVALID_PARAM);
             return NIXL_ERR_INVALID_PARAM; // nixl_agent.cpp:830
         }
-        total += l.len;
+        total += len;
+        const uintptr_t l_addr = l_run->addr + (li - l_run->start_idx) * l_run->stride, r_addr = r_run->addr + (ri - r_run->start_idx) * r_run->stride;
         // Merge when both index lists advance by one and the new block starts exactly where
         // the previous one ended, on both sides, inside the same registrations.
-        if (merge && k > 0 && local_indices[k] == local_indices[k - 1] + 1 && remote_indices[k] == remote_indices[k - 1] + 1) {
-            nixlMetaDesc &pl = (*req->initiatorDescs)[req->initiatorDescs->descCount() - 1];
-            nixlMetaDesc &pr = (*req->targetDescs)[req->targetDescs->descCount() - 1];
-            if (pl.devId == l.devId && pr.devId == r.devId && pl.metadataP == l.metadataP && pr.metadataP == r.metadataP &&
-                pl.addr + pl.len == l.addr && pr.addr + pr.len == r.addr) {
-                pl.len += l.len;
-                pr.len += r.len;
+        const bool next = merge && k > 0 && li == l_prev + 1 && ri == r_prev + 1;
+        l_prev = li;
+        r_prev = ri;
+        if (next) {
+            nixlMetaDesc &pl = ours[ours.descCount() - 1];
+            nixlMetaDesc &pr = theirs[theirs.descCount() - 1];
+            if (pl.devId == l_run->devId && pr.devId == r_run->devId && pl.metadataP == l_run->metadataP && pr.metadataP == r_run->metadataP &&
+                pl.addr + pl.len == l_addr && pr.addr + pr.len == r_addr) {
+                pl.len += len;
+                pr.len += len;
                 continue;
             }
         }
-        req->initiatorDescs->addDesc(l);
-        req->targetDescs->addDesc(r);
+        ours.emplace(l_addr, len, l_run->devId, l_run->metadataP);
+        theirs.emplace(r_addr, len, r_run->devId, r_run->metadataP);
     }
     req->engine = engine;
     req->remoteAgent = remote_side->remoteAgent;

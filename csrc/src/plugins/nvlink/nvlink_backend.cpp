@@ -897,20 +897,35 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
     req->op = operation;
     req->remoteAgent = remote_agent;
     req->peer = findPeer(remote_agent, &req->peerGen);
-    struct Item {
-        XferDesc d;
-        uint64_t klass; // 1: both ends are VRAM of different GPUs
+    struct Listed { // for the kernel of one GPU
+        std::vector<XferDesc> descs;
+        std::vector<char> cross; // 1: both ends are VRAM of different GPUs
     };
-    std::map<int, std::vector<Item>> perDevice;
+    std::map<int, Listed> perDevice;
 
-    for (int i = 0; i < local.descCount(); ++i) {
-        auto *l = dynamic_cast<LocalMD *>(local[i].metadataP);
-        auto *r = dynamic_cast<RemoteMD *>(remote[i].metadataP);
-        if (!l || !r || local[i].len != remote[i].len) return fail(NIXL_ERR_INVALID_PARAM);
-        const size_t len = local[i].len;
+    // What depends on a descriptor's registrations and not on the descriptor is looked up again only where they change: a request
+    // of 2048 cache blocks has few registrations.
+    const nixlBackendMD *l_seen = nullptr, *r_seen = nullptr;
+    LocalMD *l = nullptr;
+    RemoteMD *r = nullptr;
+    Listed *listed = nullptr; // of `dev`, where peer access has been seen to
+    int dev = -1;
+    char cross = 0;
+    const size_t n_descs = static_cast<size_t>(local.descCount());
+    const nixlMetaDesc *locals = local.data(), *remotes = remote.data();
+    for (size_t i = 0; i < n_descs; ++i) {
+        if (locals[i].metadataP != l_seen || remotes[i].metadataP != r_seen) {
+            l_seen = locals[i].metadataP;
+            r_seen = remotes[i].metadataP;
+            l = dynamic_cast<LocalMD *>(locals[i].metadataP);
+            r = dynamic_cast<RemoteMD *>(remotes[i].metadataP);
+            listed = nullptr;
+        }
+        if (!l || !r || locals[i].len != remotes[i].len) return fail(NIXL_ERR_INVALID_PARAM);
+        const size_t len = locals[i].len;
         if (len == 0) continue;
         req->totalBytes += len;
-        const uintptr_t laddr = local[i].addr, raddr = remote[i].addr;
+        const uintptr_t laddr = locals[i].addr, raddr = remotes[i].addr;
         // Kernel-visible addresses of both ends, when they exist.
         const uintptr_t lvis = l->devVisible ? l->devVisible + (laddr - l->addr) : 0;
         const uintptr_t rvis = r->devVisible ? r->devVisible + (raddr - r->addr) : 0;
@@ -932,18 +947,26 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         // 340 / 378 us; 16 x 4 MiB 1.34 / 1.29 ms; a single 64 KiB 8.5 / 13 us, a single 100 KB 14.4 / 13.5, a single 256 KiB 20 / 17.
         // (Of a handle that is posted again and again.  The first post of a new handle over newly pinned pages gains next to nothing:
         // its table may still be on its way, and the GPU has yet to look up the pages' translations.)
-        const bool by_copy = l->pinnedByOwner && len > (local.descCount() == 1 ? size_t(64) << 10 : size_t(4) << 20);
+        const bool by_copy = l->pinnedByOwner && len > (n_descs == 1 ? size_t(64) << 10 : size_t(4) << 20);
         if (lvis && rvis && !by_copy) { // the copy kernel can see both ends
-            int dev;
-            if (l->mem == VRAM_SEG) dev = l->device;
-            else dev = r->sameProcess ? r->ownerDevice : r->mapDevice;
-            if (dev < 0) return fail(NIXL_ERR_BACKEND);
-            // The launching GPU needs peer access to the GPU that owns the remote memory.  For
-            // another process's memory the IPC mapping enabled it for the device that opened the
-            // handle only; a process driving several GPUs launches from others too.
-            if (r->mem == VRAM_SEG && r->ownerLocalDevice >= 0 && !ensurePeerAccess(dev, r->ownerLocalDevice)) {
-                NIXL_ERROR << "NVLINK backend: GPU " << dev << " cannot access GPU " << r->ownerLocalDevice;
-                return fail(NIXL_ERR_NOT_SUPPORTED);
+            if (!listed) {
+                if (l->mem == VRAM_SEG) dev = l->device;
+                else dev = r->sameProcess ? r->ownerDevice : r->mapDevice;
+                if (dev < 0) return fail(NIXL_ERR_BACKEND);
+                // The launching GPU needs peer access to the GPU that owns the remote memory.  For
+                // another process's memory the IPC mapping enabled it for the device that opened the
+                // handle only; a process driving several GPUs launches from others too.
+                if (r->mem == VRAM_SEG && r->ownerLocalDevice >= 0 && !ensurePeerAccess(dev, r->ownerLocalDevice)) {
+                    NIXL_ERROR << "NVLINK backend: GPU " << dev << " cannot access GPU " << r->ownerLocalDevice;
+                    return fail(NIXL_ERR_NOT_SUPPORTED);
+                }
+                // (A GPU this process cannot name is certainly not the local one.)
+                cross = l->mem == VRAM_SEG && r->mem == VRAM_SEG && r->ownerLocalDevice != l->device ? 1 : 0;
+                listed = &perDevice[dev];
+                if (listed->descs.empty()) {
+                    listed->descs.reserve(n_descs - i);
+                    listed->cross.reserve(n_descs - i);
+                }
             }
             XferDesc d;
             d.src = operation == NIXL_WRITE ? lvis : rvis;
@@ -952,14 +975,15 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
             // Neighbours in the list that continue each other on both sides become one descriptor
             // (a buffer posted as consecutive blocks is one long copy: fewer table entries for
             // the kernel, one copy instead of many for the copy engines).
-            // (A GPU this process cannot name is certainly not the local one.)
-            const bool cross_gpu = l->mem == VRAM_SEG && r->mem == VRAM_SEG && r->ownerLocalDevice != l->device;
-            auto &list = perDevice[dev];
-            const uint64_t klass = cross_gpu ? 1 : 0; // never merge across kinds of path
-            if (coalesce_ && !list.empty() && list.back().d.src + list.back().d.len == d.src && list.back().d.dst + list.back().d.len == d.dst &&
-                list.back().klass == klass)
-                list.back().d.len += d.len;
-            else list.push_back({d, klass});
+            // Never across kinds of path.
+            std::vector<XferDesc> &list = listed->descs;
+            if (coalesce_ && !list.empty() && list.back().src + list.back().len == d.src && list.back().dst + list.back().len == d.dst &&
+                listed->cross.back() == cross) {
+                list.back().len += d.len;
+            } else {
+                list.push_back(d);
+                listed->cross.push_back(cross);
+            }
             continue;
         }
         // One end is pageable host memory, which the runtime stages, or a long piece of pinned memory.
@@ -991,18 +1015,22 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         // 7.5 us to start and drain, the kernel moves a whole batch in one launch at 703 GB/s; they
         // break even near 64 MiB per descriptor.  Inside one GPU's HBM the kernel is faster
         // (moved bytes, 16 x 64 MiB: 3.25 TB/s, the rate of a plain copy, against 2.6 TB/s).
-        for (const Item &it : kv.second) {
-            const bool ce = ceThreshold_ > 0 && it.d.len >= ceThreshold_ && (it.klass == 1 || copyPath_ == CopyPath::COPY_ENGINE);
-            (ce ? b.ceDescs : b.descs).push_back(it.d);
-        }
-        b.stream = c->streams[c->nextStream.fetch_add(1, std::memory_order_relaxed) % c->streams.size()];
         bool local_only = true; // no descriptor reaches another GPU
-        for (const Item &it : kv.second) local_only = local_only && it.klass == 0;
-        uint64_t total = 0, longest = 0;
-        for (auto &d : b.descs) {
+        uint64_t total = 0;
+        b.descs.swap(kv.second.descs);
+        size_t kept = 0;
+        for (size_t i = 0; i < b.descs.size(); ++i) {
+            const XferDesc d = b.descs[i];
+            local_only = local_only && kv.second.cross[i] == 0;
+            if (ceThreshold_ > 0 && d.len >= ceThreshold_ && (kv.second.cross[i] == 1 || copyPath_ == CopyPath::COPY_ENGINE)) {
+                b.ceDescs.push_back(d);
+                continue;
+            }
             total += d.len;
-            longest = std::max<uint64_t>(longest, d.len);
+            b.descs[kept++] = d;
         }
+        b.descs.resize(kept);
+        b.stream = c->streams[c->nextStream.fetch_add(1, std::memory_order_relaxed) % c->streams.size()];
         // Chunk size: aim at ~2 chunks per CTA that can be resident at once (two per SM), between
         // 16 KiB and 256 KiB (128 KiB inside one GPU: 16 x 8 MiB take 45.4 us with 128 KiB, 50.2 us with 256 KiB).  The grid itself may be several times larger (see defaultGridCtas): a
         // large copy then runs as many short-lived CTAs whose tail balances itself.
@@ -1020,18 +1048,20 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
         const bool warp_chunks = copyPath_ == CopyPath::VECTOR && local_only && total <= (uint64_t(64) << 20) && chunkShiftOverride_ <= 15;
         if (warp_chunks) shift = std::min<uint32_t>(15, std::max<uint32_t>(12, log2Ceil(std::max<uint64_t>(1, total / (32 * static_cast<uint64_t>(c->smCount))))));
         if (chunkShiftOverride_ >= 12 && chunkShiftOverride_ <= 22) shift = static_cast<uint32_t>(chunkShiftOverride_);
-        std::vector<uint32_t> starts(n + 1);
         uint64_t chunks = 0;
         uint64_t per = 0; // chunks per descriptor when all descriptors have the same number, else 0
+        auto chunksOf = [&](size_t i) { return (b.descs[i].len + (uint64_t(1) << shift) - 1) >> shift; };
         for (size_t i = 0; i < n; ++i) {
-            starts[i] = static_cast<uint32_t>(chunks);
-            const uint64_t mine = (b.descs[i].len + (uint64_t(1) << shift) - 1) >> shift;
+            const uint64_t mine = chunksOf(i);
             per = i == 0 ? mine : (per == mine ? per : 0);
             chunks += mine;
             if (chunks > 0x7fffffffull) return fail(NIXL_ERR_INVALID_PARAM); // cannot happen below 2^31 * 16 KiB, but stay safe
         }
         b.uniformChunks = per <= kProxyMaxPer ? static_cast<uint32_t>(per) : 0;
-        starts[n] = static_cast<uint32_t>(chunks);
+        auto fillStarts = [&](uint32_t *starts) { // n + 1 of them
+            starts[0] = 0;
+            for (size_t i = 0; i < n; ++i) starts[i + 1] = starts[i] + static_cast<uint32_t>(chunksOf(i));
+        };
         b.launch.nDescs = static_cast<uint32_t>(n);
         b.launch.totalChunks = static_cast<uint32_t>(chunks);
         b.launch.chunkShift = shift;
@@ -1049,7 +1079,7 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
             b.launch.table = nullptr;
             b.launch.chunkStart = nullptr;
             for (size_t i = 0; i < n; ++i) b.launch.inl[i] = b.descs[i];
-            for (size_t i = 0; i <= n; ++i) b.launch.inlStart[i] = starts[i];
+            fillStarts(b.launch.inlStart);
         }
         // A device table for batches too long for the launch parameters, and for any batch of
         // several descriptors that may go through the proxy (a proxy command has room for one).
@@ -1061,11 +1091,15 @@ nixl_status_t Engine::prepXfer(const nixl_xfer_op_t &operation, const nixl_meta_
             if (!b.table) return fail(NIXL_ERR_BACKEND);
             DeviceScope ds(b.device);
             char *base = static_cast<char *>(b.table);
-            std::vector<char> image(soff + sbytes);
-            std::memcpy(image.data(), b.descs.data(), tbytes);
-            if (sbytes) std::memcpy(image.data() + soff, starts.data(), sbytes);
-            // Pageable source: the runtime copies it out before returning, so the vector may die.
-            bool ok = cudaOk(cudaMemcpyAsync(base, image.data(), image.size(), cudaMemcpyHostToDevice, c->prepStream), "table upload");
+            std::vector<char> image; // both arrays; without starts the descriptors go up from where they are
+            if (sbytes) {
+                image.resize(soff + sbytes);
+                std::memcpy(image.data(), b.descs.data(), tbytes);
+                fillStarts(reinterpret_cast<uint32_t *>(image.data() + soff));
+            }
+            // Pageable source: the runtime copies it out before returning, so the vectors may die.
+            bool ok = cudaOk(cudaMemcpyAsync(base, sbytes ? static_cast<const void *>(image.data()) : b.descs.data(), sbytes ? image.size() : tbytes,
+                                             cudaMemcpyHostToDevice, c->prepStream), "table upload");
             ok = ok && cudaOk(cudaEventCreateWithFlags(&b.uploaded, cudaEventDisableTiming), "cudaEventCreate");
             ok = ok && cudaOk(cudaEventRecord(b.uploaded, c->prepStream), "cudaEventRecord");
             if (!ok) return fail(NIXL_ERR_BACKEND);

@@ -70,6 +70,9 @@ class KVBlockTransfer:
                 raise ValueError(f"tensor {t}: a block is {rows[t * self.blocks][1]} bytes here and {theirs[t * self.remote_blocks][1]} bytes at the peer")
         self._local = agent.prep_xfer_dlist("NIXL_INIT_AGENT", agent.get_xfer_descs(rows, mem))
         self._remote = agent.prep_xfer_dlist(remote_agent, theirs)
+        # first entry of every tensor in either list, for requests of many entries
+        self._firsts = {n: (np.arange(self.tensors, dtype=np.int64) * n).astype(np.int32)[:, None] for n in (self.blocks, self.remote_blocks)
+                        if self.tensors * n <= 0x7FFFFFFF}
         self.block_bytes = sum(rows[t * self.blocks][1] for t in range(self.tensors))
 
     def _indices(self, blocks: Sequence[int], per_tensor: int):
@@ -80,8 +83,7 @@ class KVBlockTransfer:
             return [t * per_tensor + int(b) for t in range(self.tensors) for b in blocks]
         # tensor-major, as an array: 64 tensors x 32 blocks take 6 us this way, 100 us as a Python list and half as much again to
         # convert it; up to some 48 entries the list is the cheaper one (2 x 1: 20 against 22.5 us per request)
-        first = np.arange(self.tensors, dtype=np.int32) * per_tensor
-        return (first[:, None] + np.array([int(b) for b in blocks], dtype=np.int32)).reshape(-1)
+        return (self._firsts[per_tensor] + np.array([int(b) for b in blocks], dtype=np.int32)).reshape(-1)
 
     def post(self, local_blocks: Sequence[int], remote_blocks: Sequence[int], op: str = "WRITE", notif: Union[bytes, str] = b""):
         """Starts moving ``local_blocks[i]`` <-> ``remote_blocks[i]`` of every tensor (WRITE: to the peer, READ: from it);
