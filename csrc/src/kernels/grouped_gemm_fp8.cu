@@ -593,8 +593,11 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
     if (mode == 3) {
         if (p.N % 256 || p.K % 512 || p.counts_flag || p.disp_flag) return cudaErrorInvalidValue;
         if ((reinterpret_cast<uintptr_t>(p.scale_a) | reinterpret_cast<uintptr_t>(p.scale_w)) & 3) return cudaErrorInvalidValue;
-        if (!nixl_gemm::makeTileMap(&mapA, p.a, a_rows, k_bytes) || !nixl_gemm::makeTileMap(&mapA32, p.a, a_rows, k_bytes, 32)) return cudaErrorInvalidValue;
-        return nixl_gemm::launchMxPairKernel(mapA, mapA32, mapA64, mapW, p, static_cast<cudaStream_t>(stream));
+        CUtensorMap mapW2;
+        if (!nixl_gemm::makeTileMap(&mapA, p.a, a_rows, k_bytes) || !nixl_gemm::makeTileMap(&mapA32, p.a, a_rows, k_bytes, 32) ||
+            !nixl_gemm::makePairMap(&mapW2, p.w, w_rows, k_bytes))
+            return cudaErrorInvalidValue;
+        return nixl_gemm::launchMxPairKernel(mapA, mapA32, mapA64, mapW, mapW2, p, static_cast<cudaStream_t>(stream));
     }
     if (mode == 2) {
         if (p.N % 256) return cudaErrorInvalidValue;

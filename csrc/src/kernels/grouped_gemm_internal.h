@@ -28,7 +28,9 @@ cudaError_t launchPairKernel(const CUtensorMap &mapA, const CUtensorMap &mapA64,
 // Tiles of 256 columns x up to 256 tokens with power-of-two block scales applied by the tensor core (kind::mxf8f6f4.block_scale):
 // p.scale_a / p.scale_w point at exponent bytes (uint8 [a_rows][K/128] and [groups][N/128][K/128]);
 // K must be a multiple of 512, N of 256; no dispatch overlap.  The maps of the tokens have boxes of 128, 32 and 64 rows.
-cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream);
+// mapW2 is that of makePairMap.
+cudaError_t launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const CUtensorMap &mapW2,
+                               const NixlGroupedGemmParams &p, cudaStream_t stream);
 
 #ifdef __CUDACC__
 // The tile table of a launch, built by one whole warp, 32 groups at a time: prefix[g] tiles come before group g, each of whose

@@ -56,10 +56,11 @@ using nixl_gemm::kMaxGroups;
 constexpr int BW = 128;        // W rows per CTA (256 per pair): the MMA's M side
 constexpr int BT = 256;        // tokens per tile at most: its N side, half of them from either CTA
 constexpr int BK = 128;
-constexpr int kStages = 6;
+constexpr int kMaxStages = 6;
 constexpr int kThreads = 384;
 constexpr int kWTileBytes = BW * BK;
-constexpr int kStageBytes = kWTileBytes + BT / 2 * BK; // 32 KiB per CTA
+constexpr uint32_t kOneStepStage = kWTileBytes + BT / 2 * BK; // 32 KiB
+constexpr int kRingBytes = kMaxStages * kOneStepStage; // 192 KiB per CTA
 constexpr int kChunkSteps = 4;                 // steps whose scale bytes share one 32-bit word
 constexpr int kGroupChunks = 8;                // chunks copied to TMEM in one go
 constexpr int kSfAtomBytes = 512;              // 128 rows x 4 steps
@@ -73,8 +74,8 @@ constexpr int kPromoWarps = 8;
 static_assert(kAccCols + 2 * kSfTmemStride <= kTmemCols, "accumulator and scale columns share TMEM");
 
 struct Shared {
-    uint64_t full[kStages];      // even CTA: both CTAs' operand bytes of a stage have landed
-    uint64_t empty[kStages];     // per CTA: the MMAs that read the stage are done
+    uint64_t full[kMaxStages];   // even CTA: both CTAs' operand bytes of a stage have landed
+    uint64_t empty[kMaxStages];  // per CTA: the MMAs that read the stage are done
     uint64_t sfFull[2];          // even CTA: both CTAs have staged the group's scale layouts (16 warp arrivals)
     uint64_t sfEmpty[2];         // per CTA: the group's buffer has been copied to TMEM
     uint64_t tmemFull;           // per CTA: a tile's accumulator is complete
@@ -86,6 +87,7 @@ struct Shared {
     int rowStart[kMaxGroups];
     int rowCount[kMaxGroups];
     int tileRows[kMaxGroups]; // tokens per tile of the group, a multiple of 32
+    int boxRows;                 // tokens of a CTA that a step has room for: 32, 64 or 128
 };
 
 __device__ __forceinline__ uint32_t clusterCtaRank() {
@@ -113,6 +115,12 @@ __device__ __forceinline__ void tmaLoad2dPair(void *smem_dst, const CUtensorMap 
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
                      smemU32(smem_dst)),
                  "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tmaLoad3dPair(void *smem_dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar_cluster_addr) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
+                     smemU32(smem_dst)),
+                 "l"(map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 __device__ __forceinline__ void mbarArriveClusterRelease(uint32_t cluster_addr) {
@@ -143,6 +151,26 @@ __device__ __forceinline__ uint32_t instrDescMx(uint32_t sf, uint32_t n) {
     return (sf << 4) | ((n >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>((2 * BW) >> 4) << 24) | (sf << 29);
 }
 
+// The first of a stage's two steps: its four MMAs.
+__device__ __forceinline__ void issueFirstStepMx(uint32_t tmem_d, uint64_t dw, uint64_t dt, uint32_t idesc, uint32_t tsfw, uint32_t tsft, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        " .reg .pred pacc, pfirst;\n"
+        " setp.ne.b32 pacc, %7, 0;\n"
+        " setp.ne.b32 pfirst, %6, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], pfirst;\n"
+        " add.u64 %1, %1, 2;\n add.u64 %2, %2, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], pacc;\n"
+        " add.u64 %1, %1, 2;\n add.u64 %2, %2, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], pacc;\n"
+        " add.u64 %1, %1, 2;\n add.u64 %2, %2, 2;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%4], [%5], pacc;\n"
+        "}\n"
+        : "+r"(tmem_d), "+l"(dw), "+l"(dt)
+        : "r"(idesc), "r"(tsfw), "r"(tsft), "r"(accumulate), "r"(1u)
+        : "memory");
+}
+
 // One 128-channel step: four block-scaled MMAs and the commit that frees the stage.  The non-blocking
 // test of the next step's barrier sits between the MMAs: its latency then runs while the others are
 // being issued, and its result is read last.
@@ -169,6 +197,9 @@ __device__ __forceinline__ void issueKStepMx(uint32_t tmem_d, uint64_t dw, uint6
         : "memory");
 }
 
+// Rows of the one TMA box that fetches a CTA's half of a tile: an instruction more per step costs more than the rows it would save.
+__device__ __forceinline__ int boxRows(int half) { return half <= 32 ? 32 : half <= 64 ? 64 : BT / 2; }
+
 struct Tile {
     int g, mt, nt;
 };
@@ -187,12 +218,102 @@ __device__ __forceinline__ bool tileAt(const Shared &sh, int groups, int n_tiles
     return true;
 }
 
+// One issuing thread's share of a pair's chunks.  kTwo: stages of two steps (see the kernel).
+template<bool kTwo>
+__device__ __forceinline__ void issueChunks(Shared &sh, unsigned char *tiles, unsigned char *sf_ring, const NixlGroupedGemmParams &p, int n_tiles, int chunks, int sf_groups, int pair,
+                                            int pairs, int my_tiles, uint32_t me, uint32_t tmem, uint32_t stage_bytes, uint32_t stages) {
+    constexpr uint32_t kSteps = kTwo ? 2 : 1; // of a stage
+    volatile int *abort_flag = &sh.abort;
+    const uint32_t full_bar0 = smemU32(&sh.full[0]), empty_bar0 = smemU32(&sh.empty[0]), sfempty_bar0 = smemU32(&sh.sfEmpty[0]);
+    const uint64_t desc0 = smemDesc(smemU32(tiles));
+    const uint32_t sf_smem0 = smemU32(sf_ring);
+    const uint32_t total_chunks = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(chunks);
+    uint32_t known_tile = 0xffffffffu, n_tokens = 32;
+    for (uint32_t cc = me; cc < total_chunks; cc += 2) {
+        const uint32_t tile = cc / static_cast<uint32_t>(chunks), c = cc - tile * static_cast<uint32_t>(chunks);
+        const uint32_t it0 = cc * (kChunkSteps / kSteps); // the chunk's first use of a stage
+        uint32_t s = it0 % stages, full_par = (it0 / stages) & 1u;
+        const uint32_t gg = tile * static_cast<uint32_t>(sf_groups) + c / kGroupChunks, b = gg & 1u; // scale group
+        if (tile != known_tile) {
+            Tile t;
+            if (tileAt(sh, p.groups, n_tiles, pair + static_cast<int>(tile) * pairs, t)) n_tokens = static_cast<uint32_t>(sh.tileRows[t.g]);
+            known_tile = tile;
+        }
+        // Everything this chunk depends on, before asking for the turn.
+        if (c % kGroupChunks == 0 && !mbarWait(&sh.sfFull[b], (gg >> 1) & 1u, abort_flag)) return;
+        if (!mbarWait(&sh.full[s], full_par, abort_flag)) return;
+        {
+            const long long t0 = clock64();
+            while (ldAcquireCta(&sh.chunksIssued) != cc) {
+                if (*abort_flag) return;
+                if (clock64() - t0 > (1ll << 33)) {
+                    *abort_flag = 1;
+                    return;
+                }
+            }
+        }
+        // Accumulator drained by the previous tile's epilogue.  With the turn in hand, not before: the previous tile is
+        // then issued, so its own wait here has passed and the barrier is at most one phase behind, which is all a parity
+        // can tell.  (With one chunk per tile a thread would otherwise look before the other one issued the tile between,
+        // two phases early, and pass at once.)
+        if (c == 0 && !mbarWait(&sh.tmemEmpty, (tile & 1u) ^ 1u, abort_flag)) return;
+        tcFenceAfter();
+        const uint32_t sf_base = tmem + kAccCols + b * kSfTmemStride;
+        if (c % kGroupChunks == 0) {
+            const uint32_t here = min(static_cast<uint32_t>(kGroupChunks), static_cast<uint32_t>(chunks) - c);
+            for (uint32_t i = 0; i < here; ++i) {
+                const uint32_t src = sf_smem0 + b * kSfBufBytes + i * kSfChunkBytes, dst = sf_base + i * kSfTmemChunk;
+                tmemCpPair(dst, sfDesc(src));
+                if (n_tokens > 128) tmemCpPair(dst + 4, sfDesc(src + kSfAtomBytes));
+                tmemCpPair(dst + 8, sfDesc(src + 2 * kSfAtomBytes));
+            }
+            tcCommitPair(sfempty_bar0 + b * 8u); // the buffer may be refilled once the copies have read it
+        }
+        const uint32_t sfc = sf_base + (c % kGroupChunks) * kSfTmemChunk;
+        uint32_t ready = 1; // the first stage's barrier was waited for above
+#pragma unroll
+        for (uint32_t sub = 0; sub < kChunkSteps; ++sub) {
+            const uint32_t odd = kTwo ? sub & 1u : 0u; // a stage's second step
+            if (!odd) {
+                if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) return;
+                tcFenceAfter();
+            }
+            const uint64_t dw = desc0 + static_cast<uint64_t>((s * stage_bytes + odd * kWTileBytes) >> 4);
+            const uint64_t dt = desc0 + static_cast<uint64_t>((s * stage_bytes + kSteps * kWTileBytes + odd * (stage_bytes / kSteps - kWTileBytes)) >> 4);
+            const uint32_t accumulate = (c | sub) ? 1u : 0u;
+            if (kTwo && !odd) {
+                issueFirstStepMx(tmem, dw, dt, instrDescMx(sub, n_tokens), sfc + 8, sfc, accumulate);
+                continue;
+            }
+            uint32_t ns = s + 1, nfull_par = full_par;
+            if (ns == stages) {
+                ns = 0;
+                nfull_par ^= 1u;
+            }
+            issueKStepMx(tmem, dw, dt, instrDescMx(sub, n_tokens), sfc + 8, sfc, accumulate, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
+            s = ns;
+            full_par = nfull_par;
+        }
+        // All of this chunk's MMAs are in the pipe: the other thread's chunk may follow.  It adds to the accumulator
+        // these MMAs write and may read the scale columns copied here, and tcgen05 operations of two threads are in
+        // order only across a fence on either side of the hand-over (tcFenceAfter: above, with the turn).
+        tcFenceBefore();
+        stReleaseCta(&sh.chunksIssued, cc + 1);
+        if (c + 1 == static_cast<uint32_t>(chunks) || c + 2 == static_cast<uint32_t>(chunks)) {
+            // This thread's last chunk of the tile: its share of "accumulator complete" (both shares when
+            // the tile has a single chunk and the other thread never touches it).
+            tcCommitPair(smemU32(&sh.tmemFull));
+            if (chunks == 1) tcCommitPair(smemU32(&sh.tmemFull));
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_constant__ CUtensorMap mapT32, const __grid_constant__ CUtensorMap mapT64,
-                        const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
+                        const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapW2, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
-    unsigned char *sf_ring = tiles + kStages * kStageBytes; // two buffers of kGroupChunks chunks' layouts
+    unsigned char *sf_ring = tiles + kRingBytes; // two buffers of kGroupChunks chunks' layouts
     Shared &sh = *reinterpret_cast<Shared *>(sf_ring + 2 * kSfBufBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = p.N / (2 * BW), k_steps = p.K / BK;
@@ -203,7 +324,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
 
     nixl_pdl::allowNextKernel();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kMaxStages; ++s) {
             mbarInit(&sh.full[s], 1);
             mbarInit(&sh.empty[s], 1);
         }
@@ -225,10 +346,14 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     if (warp == 1) {
         int most;
         nixl_gemm::buildTileTable(p, n_tiles, [](int rows) { return (rows + BT - 1) / BT; }, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
+        int widest = 32;
         for (int g = lane; g < p.groups; g += 32) { // (each lane wrote its groups' counts itself)
             const int c = sh.rowCount[g], tiles_g = (c + BT - 1) / BT; // equal tiles, rounded up to the MMA's granularity
             sh.tileRows[g] = tiles_g > 0 ? ((c + tiles_g - 1) / tiles_g + 31) & ~31 : 32;
+            widest = max(widest, sh.tileRows[g]);
         }
+        widest = __reduce_max_sync(0xffffffffu, widest);
+        if (lane == 0) sh.boxRows = boxRows(widest / 2);
     }
     tcFenceBefore();
     __syncthreads();
@@ -236,6 +361,15 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     tcFenceAfter();
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
+    // With at most 128 tokens in any tile the kernel is bound by W from HBM: a stage then holds two steps, so that W comes in boxes of
+    // 256 bytes x 128 rows, and the room that wider tiles would take goes to more steps in flight (eight instead of six): 32 experts,
+    // 1024 rows, 2048 x 7168 100 -> 94 us; 40 experts, 9000 rows, 1024 x 3584 60 -> 55 (2 of them by the launch).  Wider tiles keep
+    // stages of one step: with two, 32 experts, 32768 rows, 4096 x 4096 took 558 us instead of 550.
+    const bool two = sh.boxRows <= 64;
+    const uint32_t stage_steps = two ? 2 : 1;
+    const uint32_t t_bytes = static_cast<uint32_t>(sh.boxRows * BK); // of a step
+    const uint32_t stage_bytes = stage_steps * (kWTileBytes + t_bytes);
+    const uint32_t stages = min(static_cast<uint32_t>(kMaxStages), kRingBytes / stage_bytes);
     int my_tiles = 0;
     {
         const int total = sh.tilePrefix[p.groups];
@@ -245,24 +379,32 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     if (warp == 0 && lane == 0) {
         // ---------------------------------------------------------------- TMA producer (both CTAs)
         const uint32_t full0 = mapToCta(smemU32(&sh.full[0]), 0);
-        uint32_t it = 0;
+        uint32_t s = 0, empty_par = 1; // ring position
         Tile t;
         for (int ti = pair; tileAt(sh, p.groups, n_tiles, ti, t); ti += pairs) {
             const int half = sh.tileRows[t.g] / 2; // tokens of this CTA
             const int row0 = sh.rowStart[t.g] + t.mt * (2 * half) + static_cast<int>(cta) * half;
             const int wrow = t.g * p.N + t.nt * (2 * BW) + static_cast<int>(cta) * BW;
-            // One TMA box of 32, 64 or 128 token rows: an instruction more per step costs more than the rows it would save.
-            const int box = half <= 32 ? 32 : half <= 64 ? 64 : BT / 2;
+            const int box = boxRows(half);
             const CUtensorMap *map = box == 32 ? &mapT32 : box == 64 ? &mapT64 : &mapT;
-            const uint32_t bytes = static_cast<uint32_t>(2 * (kWTileBytes + box * BK)); // both CTAs' shares
-            for (int ks = 0; ks < k_steps; ++ks, ++it) {
-                const int s = it % kStages;
-                if (!mbarWait(&sh.empty[s], ((it / kStages) & 1) ^ 1, abort_flag)) goto producer_done;
+            const uint32_t bytes = 2 * stage_steps * static_cast<uint32_t>(kWTileBytes + box * BK); // both CTAs' shares
+            for (int ks = 0; ks < k_steps; ks += static_cast<int>(stage_steps)) {
+                if (!mbarWait(&sh.empty[s], empty_par, abort_flag)) goto producer_done;
                 if (cta == 0) mbarExpectTx(&sh.full[s], bytes);
-                const uint32_t bar = full0 + static_cast<uint32_t>(s) * 8u;
-                unsigned char *st = tiles + s * kStageBytes;
-                tmaLoad2dPair(st, &mapW, ks * BK, wrow, bar);
-                tmaLoad2dPair(st + kWTileBytes, map, ks * BK, row0, bar);
+                const uint32_t bar = full0 + s * 8u;
+                unsigned char *st = tiles + s * stage_bytes;
+                unsigned char *tokens = st + stage_steps * kWTileBytes;
+                if (two) {
+                    tmaLoad3dPair(st, &mapW2, 0, wrow, ks, bar);
+                    tmaLoad2dPair(tokens + t_bytes, map, (ks + 1) * BK, row0, bar);
+                } else {
+                    tmaLoad2dPair(st, &mapW, ks * BK, wrow, bar);
+                }
+                tmaLoad2dPair(tokens, map, ks * BK, row0, bar);
+                if (++s == stages) {
+                    s = 0;
+                    empty_par ^= 1u;
+                }
             }
         }
     producer_done:;
@@ -276,81 +418,8 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
         // chunks, made by the thread that has its first one, must precede the MMAs of both threads that read them);
         // even groups use one set of TMEM scale columns, odd groups the other.
         const uint32_t me = warp == 1 ? 0u : 1u;
-        const uint32_t full_bar0 = smemU32(&sh.full[0]), empty_bar0 = smemU32(&sh.empty[0]), sfempty_bar0 = smemU32(&sh.sfEmpty[0]);
-        const uint64_t desc0 = smemDesc(smemU32(tiles));
-        const uint32_t sf_smem0 = smemU32(sf_ring);
-        const uint32_t total_chunks = static_cast<uint32_t>(my_tiles) * static_cast<uint32_t>(chunks);
-        uint32_t known_tile = 0xffffffffu, n_tokens = 32;
-        for (uint32_t cc = me; cc < total_chunks; cc += 2) {
-            const uint32_t tile = cc / static_cast<uint32_t>(chunks), c = cc - tile * static_cast<uint32_t>(chunks);
-            const uint32_t it0 = cc * kChunkSteps;
-            uint32_t s = it0 % kStages, full_par = (it0 / kStages) & 1u;
-            const uint32_t gg = tile * static_cast<uint32_t>(sf_groups) + c / kGroupChunks, b = gg & 1u; // scale group
-            if (tile != known_tile) {
-                Tile t;
-                if (tileAt(sh, p.groups, n_tiles, pair + static_cast<int>(tile) * pairs, t)) n_tokens = static_cast<uint32_t>(sh.tileRows[t.g]);
-                known_tile = tile;
-            }
-            // Everything this chunk depends on, before asking for the turn.
-            if (c % kGroupChunks == 0 && !mbarWait(&sh.sfFull[b], (gg >> 1) & 1u, abort_flag)) goto issuer_done;
-            if (!mbarWait(&sh.full[s], full_par, abort_flag)) goto issuer_done;
-            {
-                const long long t0 = clock64();
-                while (ldAcquireCta(&sh.chunksIssued) != cc) {
-                    if (*abort_flag) goto issuer_done;
-                    if (clock64() - t0 > (1ll << 33)) {
-                        *abort_flag = 1;
-                        goto issuer_done;
-                    }
-                }
-            }
-            // Accumulator drained by the previous tile's epilogue.  With the turn in hand, not before: the previous tile is
-            // then issued, so its own wait here has passed and the barrier is at most one phase behind, which is all a parity
-            // can tell.  (With one chunk per tile a thread would otherwise look before the other one issued the tile between,
-            // two phases early, and pass at once.)
-            if (c == 0 && !mbarWait(&sh.tmemEmpty, (tile & 1u) ^ 1u, abort_flag)) goto issuer_done;
-            tcFenceAfter();
-            const uint32_t sf_base = tmem + kAccCols + b * kSfTmemStride;
-            if (c % kGroupChunks == 0) {
-                const uint32_t here = min(static_cast<uint32_t>(kGroupChunks), static_cast<uint32_t>(chunks) - c);
-                for (uint32_t i = 0; i < here; ++i) {
-                    const uint32_t src = sf_smem0 + b * kSfBufBytes + i * kSfChunkBytes, dst = sf_base + i * kSfTmemChunk;
-                    tmemCpPair(dst, sfDesc(src));
-                    if (n_tokens > 128) tmemCpPair(dst + 4, sfDesc(src + kSfAtomBytes));
-                    tmemCpPair(dst + 8, sfDesc(src + 2 * kSfAtomBytes));
-                }
-                tcCommitPair(sfempty_bar0 + b * 8u); // the buffer may be refilled once the copies have read it
-            }
-            const uint32_t sfc = sf_base + (c % kGroupChunks) * kSfTmemChunk;
-            uint32_t ready = 1; // the first step's barrier was waited for above
-#pragma unroll
-            for (uint32_t sub = 0; sub < kChunkSteps; ++sub) {
-                if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) goto issuer_done;
-                tcFenceAfter();
-                uint32_t ns = s + 1, nfull_par = full_par;
-                if (ns == kStages) {
-                    ns = 0;
-                    nfull_par ^= 1u;
-                }
-                const uint64_t dw = desc0 + static_cast<uint64_t>((s * kStageBytes) >> 4);
-                const uint64_t dt = dw + static_cast<uint64_t>(kWTileBytes >> 4);
-                issueKStepMx(tmem, dw, dt, instrDescMx(sub, n_tokens), sfc + 8, sfc, (c | sub) ? 1u : 0u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
-                s = ns;
-                full_par = nfull_par;
-            }
-            // All of this chunk's MMAs are in the pipe: the other thread's chunk may follow.  It adds to the accumulator
-            // these MMAs write and may read the scale columns copied here, and tcgen05 operations of two threads are in
-            // order only across a fence on either side of the hand-over (tcFenceAfter: above, with the turn).
-            tcFenceBefore();
-            stReleaseCta(&sh.chunksIssued, cc + 1);
-            if (c + 1 == static_cast<uint32_t>(chunks) || c + 2 == static_cast<uint32_t>(chunks)) {
-                // This thread's last chunk of the tile: its share of "accumulator complete" (both shares when
-                // the tile has a single chunk and the other thread never touches it).
-                tcCommitPair(smemU32(&sh.tmemFull));
-                if (chunks == 1) tcCommitPair(smemU32(&sh.tmemFull));
-            }
-        }
-    issuer_done:;
+        if (two) issueChunks<true>(sh, tiles, sf_ring, p, n_tiles, chunks, sf_groups, pair, pairs, my_tiles, me, tmem, stage_bytes, stages);
+        else issueChunks<false>(sh, tiles, sf_ring, p, n_tiles, chunks, sf_groups, pair, pairs, my_tiles, me, tmem, kOneStepStage, kMaxStages);
     } else if (warp >= 4) {
         // ---------------------------------------------------------------- scale staging, then the epilogue
         const int q = warp & 3;
@@ -446,8 +515,9 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
 
 } // namespace
 
-cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const NixlGroupedGemmParams &p, cudaStream_t stream) {
-    const size_t smem = size_t(kStages) * kStageBytes + size_t(2) * kSfBufBytes + sizeof(Shared) + 1024;
+cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtensorMap &mapT32, const CUtensorMap &mapT64, const CUtensorMap &mapW, const CUtensorMap &mapW2,
+                                          const NixlGroupedGemmParams &p, cudaStream_t stream) {
+    const size_t smem = size_t(kRingBytes) + size_t(2) * kSfBufBytes + sizeof(Shared) + 1024;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     static bool attr_done[64] = {};
@@ -484,5 +554,5 @@ cudaError_t nixl_gemm::launchMxPairKernel(const CUtensorMap &mapT, const CUtenso
     if (pairs > max_tiles) pairs = static_cast<int>(max_tiles);
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapT32, mapT64, mapW, p);
+    return cudaLaunchKernelEx(&cfg, groupedGemmMxPairKernel, mapT, mapT32, mapT64, mapW, mapW2, p);
 }

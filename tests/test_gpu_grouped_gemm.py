@@ -104,6 +104,8 @@ def _check(G, N, K, counts, gap, tile_mode, grid=0, expected_rows=0):
         (4, 256, 1024, [0, 600, 1, 129], 3),
         (3, 512, 7168, [64, 257, 512], 0),
         (36, 256, 512, [(11 * i) % 50 for i in range(36)], 0),
+        (3, 512, 1536, [128, 100, 20], 0),   # stages of two steps, boxes of 64 and 32 rows
+        (3, 512, 2048, [128, 129, 20], 0),   # of one step
     ],
 )
 def test_block_scaled_tiles_match_reference(G, N, K, counts, gap):
