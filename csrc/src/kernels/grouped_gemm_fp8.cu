@@ -229,7 +229,6 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = p.N / BN, k_steps = p.K / BK;
 
-    nixl_pdl::allowNextKernel();
     // The W boxes of this CTA's first tile, if each expert has one row tile, on their way to L2 before the rows are there.  (A hint
     // only: W itself is read behind the wait, as the kernel in front may have written it.)
     if (threadIdx.x == 32 && static_cast<long long>(blockIdx.x) * BN < static_cast<long long>(p.groups) * p.N) {
@@ -250,11 +249,11 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         sh.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    nixl_pdl::waitForPreviousKernel(); // (before TMEM is taken: the kernel in front may be about to)
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemU32(&sh.tmemBase)), "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    nixl_pdl::waitForPreviousKernel();
     // Tile table: group g owns ceil(count/BM) x n_tiles tiles.
     if (p.counts_flag && threadIdx.x == 0) {
         int run = 0, most = 0;
@@ -295,6 +294,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
+    nixl_pdl::allowNextKernel(); // (with TMEM in hand: a kernel that moved in before could take it and then wait for this one)
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
     // A stage holds the W tiles and as many A rows as the fullest expert has: with few rows per expert (a decode step) the kernel

@@ -242,7 +242,6 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
 
 __global__ void __launch_bounds__(kThreads, 1)
 groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA64, const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
-    nixl_pdl::allowNextKernel();
     nixl_pdl::waitForPreviousKernel();
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
@@ -306,6 +305,7 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     __syncthreads();
     clusterSync(); // the partner's barriers exist before anything arrives on them
     tcFenceAfter();
+    nixl_pdl::allowNextKernel(); // (with TMEM in hand: a kernel that moved in before could take it and then wait for this one)
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
     if (warp < 4) {

@@ -322,7 +322,6 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     const uint32_t cta = clusterCtaRank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
-    nixl_pdl::allowNextKernel();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbarInit(&sh.full[s], 1);
@@ -338,11 +337,11 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
         sh.chunksIssued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    nixl_pdl::waitForPreviousKernel(); // (before TMEM is taken: the kernel in front may be about to)
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemU32(&sh.tmemBase)), "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
-    nixl_pdl::waitForPreviousKernel();
     if (warp == 1) {
         int most;
         nixl_gemm::buildTileTable(p, n_tiles, [](int rows) { return (rows + BT - 1) / BT; }, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
@@ -359,6 +358,7 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
     __syncthreads();
     clusterSync();
     tcFenceAfter();
+    nixl_pdl::allowNextKernel(); // (with TMEM in hand: a kernel that moved in before could take it and then wait for this one)
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
     // With at most 128 tokens in any tile the kernel is bound by W from HBM: a stage then holds two steps, so that W comes in boxes of

@@ -141,7 +141,7 @@ def grouped_gemm_fp8(
     ``overlapped``: that dispatch was launched on another stream and may still be running; the
     kernel then waits for the count exchange itself (``rows_per_expert`` names the layout) and
     ``grid`` should leave the dispatch's CTAs free (see ``Buffer.dispatch_gemm``).
-    ``tile_mode``: 0 lets the library choose, 1 forces 128 x 128 tiles on single CTAs, 2 forces
+    ``tile_mode``: 0 lets the library choose, 1 forces tiles of 128 columns on single CTAs, 2 forces
     256 x 256 tiles on CTA pairs (``N % 256 == 0``).
     ``expected_rows``: about how many rows the groups have together, for that choice; 0: what the ``Buffer`` whose dispatch
     made ``row_count`` expects, else all rows of ``a``.  It does not change the result."""
