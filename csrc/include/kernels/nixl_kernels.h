@@ -114,7 +114,7 @@ typedef struct NixlEpScratch { /* device memory private to the rank; zero before
     int32_t *cnt;      /* [E] */
     int32_t *fill;     /* [E] not used; kept so that the record keeps its layout */
     int32_t *sent;     /* [E] */
-    uint32_t *barrier; /* [4] grid barrier (two words), CTAs that have left a dispatch */
+    uint32_t *barrier; /* [4] grid barrier of a combine (two words), CTAs that have left a dispatch, grid barrier of a dispatch */
     int32_t *status;   /* [1] bit0: a peer timed out, bit1: grid barrier timed out, bit2: capacity exceeded */
     int32_t *mask;     /* [R] non-zero: rank excluded */
 } NixlEpScratch;

@@ -136,6 +136,7 @@ __device__ __forceinline__ void gridBarrier(unsigned *bar, int *status, uint64_t
 }
 
 // The same for a kernel whose last CTA sets the word back to zero when all have left: one operation to arrive, no generation to read.
+// The word stays raised until then, so nothing else may use it: a combine of the same buffer may run on another stream meanwhile.
 __device__ __forceinline__ void gridBarrierOnce(unsigned *bar, int *status, uint64_t timeout_ns) {
     __syncthreads();
     if (threadIdx.x == 0 && addAcqRelGpu(bar, 1u) + 1 < gridDim.x) {
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         if (fixed) __syncthreads();
     }
     if ((p.phases & 1) && !fixed) {
-        gridBarrierOnce(p.scr.barrier, p.scr.status, p.timeout_ns);
+        gridBarrierOnce(p.scr.barrier + 3, p.scr.status, p.timeout_ns);
         for (int e = tid; e < p.E && kKeepTotals; e += kThreads) total[e] = ldVolatile(p.scr.cnt + e);
         __syncthreads();
 
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
         __syncthreads();
         if (tid == 0) { // releases this CTA's counts and rows, and acquires the others'
             last = addAcqRelGpu(p.scr.barrier + 2, 1u) == gridDim.x - 1;
-            if (last) p.scr.barrier[0] = p.scr.barrier[2] = 0;
+            if (last) p.scr.barrier[2] = p.scr.barrier[3] = 0;
         }
         __syncthreads();
         if (last && fixed) {

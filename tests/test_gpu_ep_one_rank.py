@@ -210,3 +210,76 @@ def test_compact_dispatch_places_every_copy_once(tokens, experts, topk, sms):
         assert torch.equal(recv[rows], x[t])
         assert torch.equal(h.src_info[rows, 1].long(), t * topk + k)
     b.destroy()
+
+
+def _compact(b, x, idx, w):
+    """A compact dispatch, every copy of which must have arrived in a row of its own among its expert's."""
+    recv, _, h = b.dispatch(x, idx, use_fp8=False, topk_weights=w)
+    t, k = torch.nonzero(idx >= 0, as_tuple=True)
+
+    def check():
+        want = torch.bincount(idx[idx >= 0], minlength=b.num_experts)
+        rows = h.send_row[t, k].long()
+        return (torch.equal(h.recv_count, want.int()) and torch.equal(torch.sort(rows).values, torch.arange(rows.numel(), device=rows.device))
+                and torch.equal(recv[rows], x[t]))
+
+    return recv, h, check
+
+
+def test_dispatch_leaves_the_barrier_of_a_combine_alone():
+    """A combine on another stream may have CTAs at its grid barrier while a dispatch begins and ends: the dispatch must neither
+    count them as its own nor send them away."""
+    H, E, K, T = 512, 32, 4, 700
+    b = Buffer(0, 1, E, H, T, K, device=torch.device("cuda:0"), low_latency_mode=False, timeout_ms=1000)
+    b.connect_ranks()
+    arrivals, generation = 1000, 9  # more than a dispatch has CTAs
+    b._bar[0], b._bar[1] = arrivals, generation
+    for step in range(4):
+        x, idx, w = _routing(T - 50 * step, H, E, K, 30 + step)
+        _, _, check = _compact(b, x, idx, w)
+        torch.cuda.synchronize()
+        assert b.status == 0 and check()
+        assert b._bar.tolist() == [arrivals, generation, 0, 0]
+    b.destroy()
+
+
+@pytest.mark.parametrize("mode", ["push", "reduced"])
+def test_dispatch_beside_a_combine_of_the_same_buffer(mode):
+    """Step n + 1 is dispatched on one stream while step n is combined on another, into memory that overlaps its input (the path of
+    larger groups, with a grid barrier).  Neither waits for the other, and there is room for both at once."""
+    H, E, K, T = 1024, 32, 8, 900
+    dev = torch.device("cuda:0")
+    b = Buffer(0, 1, E, H, T, K, device=dev, low_latency_mode=False, timeout_ms=1000)
+    b.connect_ranks()
+    b.set_num_sms(32)
+    sends, returns = torch.cuda.Stream(dev), torch.cuda.Stream(dev)
+    inputs = [_routing(T - 11 * i, H, E, K, 60 + i) for i in range(4)]
+    alone = []
+    for x, idx, w in inputs:
+        recv, _, h = b.dispatch(x, idx, use_fp8=False, topk_weights=w if mode == "reduced" else None)
+        alone.append(b.combine(recv.clone(), idx, w, h).clone())
+    rooms = [torch.empty(b.compact_rows + T, H, device=dev, dtype=torch.bfloat16) for _ in range(2)]
+    torch.cuda.synchronize()
+    combined = None
+    results, dispatched, keep = [], [], []
+    for step in range(16):
+        x, idx, w = inputs[step % 4]
+        with torch.cuda.stream(sends):
+            if combined is not None and step >= 2:
+                sends.wait_event(combined[step - 2])  # the half of the double buffer that this step takes is free again
+            recv, _, h = b.dispatch(x, idx, use_fp8=False, topk_weights=w if mode == "reduced" else None)
+            dispatched.append((recv, h, sends.record_event()))
+        with torch.cuda.stream(returns):
+            returns.wait_event(dispatched[step][2])
+            y = rooms[step % 2][T:]
+            y.copy_(recv)
+            got = b.combine(y, idx, w, h, out=rooms[step % 2][T - 5 : 2 * T - 5][: x.shape[0]])
+            results.append(got.clone())
+            combined = (combined or []) + [returns.record_event()]
+            keep.append(b._keep_c)
+    torch.cuda.synchronize()
+    assert b.status == 0 and b._bar.tolist()[0] == 0 and b._bar.tolist()[2:] == [0, 0]
+    for step, got in enumerate(results):
+        err = (got.double() - alone[step % 4].double()).norm() / alone[step % 4].double().norm()
+        assert float(err) < 2.0**-8, (step, float(err))  # (rows may come in another order, and with it the sum's; half a bf16 step)
+    b.destroy()
