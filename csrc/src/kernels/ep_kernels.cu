@@ -333,7 +333,8 @@ template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpD
 template<bool kKeepTotals> // the rank's totals fit into shared memory
 __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(const __grid_constant__ NixlEpDispatchParams p) {
     extern __shared__ __align__(16) unsigned char smem[];
-    nixl_pdl::allowNextKernel();
+    // (A launch that waits for peers, or only receives, lets nothing in: see programmatic_launch.cuh.)
+    if (p.R == 1 && (p.phases & 1)) nixl_pdl::allowNextKernel();
     nixl_pdl::waitForPreviousKernel();
     const int El = p.E / p.R;
     // shared: place[E] | mine[E] | total[E] (kKeepTotals) | rows[kBatch * K] | dests[kBatch * K]

@@ -294,7 +294,8 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
     tcFenceBefore();
     __syncthreads();
     tcFenceAfter();
-    nixl_pdl::allowNextKernel(); // (with TMEM in hand: a kernel that moved in before could take it and then wait for this one)
+    // With TMEM in hand: a kernel that moved in before could take it and then wait for this one.  (Not beside a dispatch.)
+    if (!p.counts_flag && !p.disp_flag) nixl_pdl::allowNextKernel();
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
     // A stage holds the W tiles and as many A rows as the fullest expert has: with few rows per expert (a decode step) the kernel

@@ -305,7 +305,8 @@ groupedGemmPairKernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     __syncthreads();
     clusterSync(); // the partner's barriers exist before anything arrives on them
     tcFenceAfter();
-    nixl_pdl::allowNextKernel(); // (with TMEM in hand: a kernel that moved in before could take it and then wait for this one)
+    // With TMEM in hand: a kernel that moved in before could take it and then wait for this one.  (Not beside a dispatch.)
+    if (!p.counts_flag && !p.disp_flag) nixl_pdl::allowNextKernel();
     const uint32_t tmem = sh.tmemBase;
     volatile int *abort_flag = &sh.abort;
     if (warp < 4) {

@@ -4,6 +4,10 @@
 // themselves up; whatever an earlier kernel of the stream may have written is touched only behind waitForPreviousKernel(), which
 // returns when that kernel is complete and its stores are visible.  Every kernel launched this way calls it, in every CTA, so
 // that a kernel that is complete implies that all before it in the stream are.
+//
+// A kernel that waits for something outside its stream (another GPU's flags, a dispatch on another stream) does not call
+// allowNextKernel(): the next kernel's CTAs would hold their SMs' shared memory and registers, idle, for as long as that takes,
+// and keep out the very work of other streams that the wait may depend on.  Its successor then starts when it is complete.
 #ifndef NIXL_B200_PROGRAMMATIC_LAUNCH_CUH
 #define NIXL_B200_PROGRAMMATIC_LAUNCH_CUH
 
