@@ -56,9 +56,11 @@ __device__ __forceinline__ unsigned ldAcquireGpu(const unsigned *p) {
     return v;
 }
 __device__ __forceinline__ int ldVolatile(const int *p) { return *reinterpret_cast<const volatile int *>(p); }
-__device__ __forceinline__ uint4 ldNc(const void *p) {
+// Rows are loaded coherently, past L1: not through the read-only path, which is for data that nobody writes while the kernel runs.
+// The kernel in front of an overlapped launch still writes them then, and so do peers whose flag this kernel waits for.
+__device__ __forceinline__ uint4 ldStream16(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void stPeer16(void *p, const uint4 &v) {
@@ -66,14 +68,14 @@ __device__ __forceinline__ void stPeer16(void *p, const uint4 &v) {
 }
 
 // 32 bytes as two 16-byte halves; one access where the address allows.
-__device__ __forceinline__ void ldNc32(const void *p, bool wide, uint4 &lo, uint4 &hi) {
+__device__ __forceinline__ void ldStream32(const void *p, bool wide, uint4 &lo, uint4 &hi) {
     if (wide) {
-        asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                      : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
                      : "l"(p));
     } else {
-        lo = ldNc(p);
-        hi = ldNc(static_cast<const char *>(p) + 16);
+        lo = ldStream16(p);
+        hi = ldStream16(static_cast<const char *>(p) + 16);
     }
 }
 __device__ __forceinline__ void stPeer32(void *p, bool wide, const uint4 &lo, const uint4 &hi) {
@@ -260,7 +262,7 @@ template<bool kFp8> __device__ __forceinline__ void dispatchTokens(const NixlEpD
         for (int s0 = slices * part / parts; s0 < s_end; s0 += kSlices) {
             uint4 lo[kSlices], hi[kSlices];
 #pragma unroll
-            for (int j = 0; j < kSlices; ++j) ldNc32(src + static_cast<long long>(min(s0 + j, s_end - 1)) * 1024, wide_in, lo[j], hi[j]); // (past the end: the last slice again, not stored)
+            for (int j = 0; j < kSlices; ++j) ldStream32(src + static_cast<long long>(min(s0 + j, s_end - 1)) * 1024, wide_in, lo[j], hi[j]); // (past the end: the last slice again, not stored)
             float4 sc = make_float4(0.f, 0.f, 0.f, 0.f); // lane j: the four scales of slice j
             if constexpr (kFp8) {
 #pragma unroll
@@ -693,7 +695,7 @@ __device__ __forceinline__ void pullReduce(const NixlEpCombineParams &p, int El,
         auto load = [&](uint4(&buf)[KMAX], int v) {
 #pragma unroll
             for (int k = 0; k < KMAX; ++k)
-                if (k < p.K && w[k] == w[k]) buf[k] = ldNc(src[k] + v);
+                if (k < p.K && w[k] == w[k]) buf[k] = ldStream16(src[k] + v);
         };
         auto reduceStore = [&](const uint4(&buf)[KMAX], int v) {
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -994,12 +996,12 @@ __global__ void __launch_bounds__(kThreads) epCombineKernel(const __grid_constan
                 uint32_t *words = reinterpret_cast<uint32_t *>(dst);
                 uint2 *meta = reinterpret_cast<uint2 *>(reinterpret_cast<char *>(dst) + static_cast<long long>(p.H) * 10 / 8);
                 const int blocks = p.H / 512;
-                uint4 lo = ldNc(src + lane * 2), hi = ldNc(src + lane * 2 + 1);
+                uint4 lo = ldStream16(src + lane * 2), hi = ldStream16(src + lane * 2 + 1);
                 for (int b = 0; b < blocks; ++b) {
                     uint4 nlo = lo, nhi = hi;
                     if (b + 1 < blocks) { // next block's loads fly while this one is encoded
-                        nlo = ldNc(src + (b + 1) * 64 + lane * 2);
-                        nhi = ldNc(src + (b + 1) * 64 + lane * 2 + 1);
+                        nlo = ldStream16(src + (b + 1) * 64 + lane * 2);
+                        nhi = ldStream16(src + (b + 1) * 64 + lane * 2 + 1);
                     }
                     uint32_t w[5];
                     uint2 m;
@@ -1016,7 +1018,7 @@ __global__ void __launch_bounds__(kThreads) epCombineKernel(const __grid_constan
                 uint4 val[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    if (v0 + i * 32 < vecs) val[i] = ldNc(src + v0 + i * 32);
+                    if (v0 + i * 32 < vecs) val[i] = ldStream16(src + v0 + i * 32);
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     if (v0 + i * 32 < vecs) stPeer16(dst + v0 + i * 32, val[i]);
@@ -1143,7 +1145,7 @@ __device__ __forceinline__ void localRows(int n, const uint4 *const (&src)[NR], 
 #pragma unroll
         for (int k = 0; k < NR; ++k) {
             raw[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (k < n) raw[k] = ldNc(src[k] + v);
+            if (k < n) raw[k] = ldStream16(src[k] + v);
         }
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1174,14 +1176,14 @@ __device__ __forceinline__ void localRowsCoded(int n, const uint4 *const (&src)[
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] = 0.f;
         const int at = b * 64 + lane * 2;
-        uint4 lo = ldNc(src[0] + at), hi = ldNc(src[0] + at + 1);
+        uint4 lo = ldStream16(src[0] + at), hi = ldStream16(src[0] + at + 1);
 #pragma unroll
         for (int k = 0; k < NR; ++k) {
             if (k >= n) break;
             uint4 nlo = lo, nhi = hi;
             if (k + 1 < NR && k + 1 < n) { // the next row's loads fly while this one is coded
-                nlo = ldNc(src[k + 1 < NR ? k + 1 : k] + at);
-                nhi = ldNc(src[k + 1 < NR ? k + 1 : k] + at + 1);
+                nlo = ldStream16(src[k + 1 < NR ? k + 1 : k] + at);
+                nhi = ldStream16(src[k + 1 < NR ? k + 1 : k] + at + 1);
             }
             uint32_t code[5];
             uint2 meta;

@@ -183,8 +183,8 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
         for (int i = 0; i < 16; ++i) acc[j][i] = 0;
     // Scales are fetched two steps ahead and kept as loaded: multiplying them right away would make the warp
     // wait for the loads it has just issued.  (A loop unrolled over a ring of four made the compiler spill.)
-    float a0 = valid ? ldScale(sa_row, fresh) : 0.f, w00 = __ldg(sw0), w10 = __ldg(sw1);
-    float a1 = valid && k_steps > 1 ? ldScale(sa_row + 1, fresh) : 0.f, w01 = k_steps > 1 ? __ldg(sw0 + 1) : 0.f, w11 = k_steps > 1 ? __ldg(sw1 + 1) : 0.f;
+    float a0 = valid ? ldScale(sa_row, fresh) : 0.f, w00 = ldScale(sw0, false), w10 = ldScale(sw1, false);
+    float a1 = valid && k_steps > 1 ? ldScale(sa_row + 1, fresh) : 0.f, w01 = k_steps > 1 ? ldScale(sw0 + 1, false) : 0.f, w11 = k_steps > 1 ? ldScale(sw1 + 1, false) : 0.f;
 #pragma unroll 1
     for (int ks = 0; ks < k_steps; ++ks, ++it) {
         const float s0 = a0 * w00, s1 = a0 * w10;
@@ -221,8 +221,8 @@ __device__ __forceinline__ bool promoteTile(Shared &sh, const float *sa_row, boo
         // The scale prefetch goes behind the arrive (loads issued before it would hold it up).
         if (nxt < k_steps) {
             a1 = valid ? ldScale(sa_row + nxt, fresh) : 0.f;
-            w01 = __ldg(sw0 + nxt);
-            if (!kTail) w11 = __ldg(sw1 + nxt);
+            w01 = ldScale(sw0 + nxt, false);
+            if (!kTail) w11 = ldScale(sw1 + nxt, false);
         }
         fmaScale32(acc[kBlocks - 2], v0, kTail ? s00 : s11);
         fmaScale32(acc[kBlocks - 1], v1, kTail ? s00 : s11);

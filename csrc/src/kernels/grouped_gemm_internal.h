@@ -85,17 +85,30 @@ __device__ __forceinline__ void waitArrivals(const NixlGroupedGemmParams &p, int
         first += c;
     }
 }
-// A scale of A: through the read-only path, unless a dispatch may have written it while this kernel was running already.
-__device__ __forceinline__ float ldScale(const float *s, bool fresh) { return fresh ? __ldcg(s) : __ldg(s); }
+// A scale, or four exponent bytes.  Not through the read-only path, which is for data that nobody writes while the kernel runs: the
+// kernel in front writes the scales of A, and may write those of W, while this one sets itself up.  `fresh`: a dispatch writes them
+// while this kernel's main loop runs, so L1 may hold lines from before some row's arrival.
+__device__ __forceinline__ float ldScale(const float *s, bool fresh) {
+    float f;
+    if (fresh) asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(f) : "l"(s));
+    else asm volatile("ld.global.f32 %0, [%1];" : "=f"(f) : "l"(s));
+    return f;
+}
+__device__ __forceinline__ uint32_t ldExponents(const uint32_t *s) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(s));
+    return v;
+}
 // A row's scales of the four steps from ks on, in one load where they start at a multiple of 16 bytes.  The lanes of a warp read 32
 // rows, that is 32 lines, and each line costs a cycle of the memory that TMA and MMA work on too.
 __device__ __forceinline__ float4 ldScales4(const float *row, int ks, int k_steps, bool fresh) {
     const float *s = row + ks;
-    if (ks + 4 <= k_steps && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
-        const float4 *v = reinterpret_cast<const float4 *>(s);
-        return fresh ? __ldcg(v) : __ldg(v);
-    }
     float4 f;
+    if (ks + 4 <= k_steps && (reinterpret_cast<uintptr_t>(s) & 15) == 0) {
+        if (fresh) asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(s));
+        else asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "l"(s));
+        return f;
+    }
     f.x = ks < k_steps ? ldScale(s, fresh) : 0.f;
     f.y = ks + 1 < k_steps ? ldScale(s + 1, fresh) : 0.f;
     f.z = ks + 2 < k_steps ? ldScale(s + 2, fresh) : 0.f;

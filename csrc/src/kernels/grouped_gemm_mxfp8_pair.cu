@@ -446,8 +446,8 @@ groupedGemmMxPairKernel(const __grid_constant__ CUtensorMap mapT, const __grid_c
                 if (i >= here) break;
                 uint32_t *layout = buf + i * (kSfChunkBytes / 4);
                 // Token r: word (r % 32) * 4 + r / 32 of its 128 tokens' layout (rows beyond the expert get exponent 127 = 1.0).
-                layout[part * 128 + lane * 4 + q] = valid ? __ldg(sa + i) : 0x7f7f7f7fu;
-                if (part == 0) layout[256 + row] = __ldg(sw + i);
+                layout[part * 128 + lane * 4 + q] = valid ? nixl_gemm::ldExponents(sa + i) : 0x7f7f7f7fu;
+                if (part == 0) layout[256 + row] = nixl_gemm::ldExponents(sw + i);
             }
             asm volatile("fence.proxy.async;" ::: "memory"); // these generic-proxy writes are read by tcgen05.cp
             __syncwarp();

@@ -84,6 +84,13 @@ inline KvPlan planFor(const NixlKvXferParams &p) {
     return k;
 }
 
+// A block id.  Volatile, and not through the read-only path: the kernel in front may write the tables while this one's CTAs wait
+// for it, and nothing else keeps the load behind that wait.
+__device__ __forceinline__ int32_t ldBlock(const int32_t *p) {
+    int32_t b;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(b) : "l"(p));
+    return b;
+}
 __device__ __forceinline__ uint4 ldStream(const void *p) {
     uint4 v;
     asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -129,7 +136,7 @@ struct SlotRef {
     uint32_t vec0;
 };
 
-__device__ __forceinline__ SlotRef lookUp(const KvPlan &k, const int32_t *__restrict__ src_blocks, const int32_t *__restrict__ dst_blocks, long long slot) {
+__device__ __forceinline__ SlotRef lookUp(const KvPlan &k, const int32_t *src_blocks, const int32_t *dst_blocks, long long slot) {
     SlotRef r{nullptr, nullptr, 0};
     if (slot >= k.slots) return r;
     const NixlKvXferParams &p = k.p;
@@ -152,7 +159,7 @@ __device__ __forceinline__ SlotRef lookUp(const KvPlan &k, const int32_t *__rest
     const long long src_extent = (p.tokens - 1LL) * p.src_token_stride + (p.heads - 1LL) * p.src_head_stride + p.head_bytes;
     const long long dst_extent = (p.tokens - 1LL) * p.dst_token_stride + (p.dst_head_offset + p.heads - 1LL) * p.dst_head_stride +
         (p.cast_fp8 ? p.head_bytes / 2 : p.head_bytes);
-    const long long sb = __ldg(src_blocks + i), db = __ldg(dst_blocks + i);
+    const long long sb = ldBlock(src_blocks + i), db = ldBlock(dst_blocks + i);
     const long long soff = sb * p.src_block_stride, doff = db * p.dst_block_stride;
     // The block tables come from device memory that nobody validated: a block must lie inside its tensor's
     // registered range on both sides, or it is skipped and reported.
@@ -171,7 +178,7 @@ __device__ __forceinline__ SlotRef lookUp(const KvPlan &k, const int32_t *__rest
 // Moves every (tensor, block pair) unit of the request.  src_blocks / dst_blocks are the block
 // tables in device memory (wherever the entry point keeps them).
 template<bool kCast, int kVec>
-__device__ __forceinline__ void moveBlocks(const KvPlan &k, const int32_t *__restrict__ src_blocks, const int32_t *__restrict__ dst_blocks) {
+__device__ __forceinline__ void moveBlocks(const KvPlan &k, const int32_t *src_blocks, const int32_t *dst_blocks) {
     constexpr int kDstVec = kCast ? kVec / 2 : kVec;
     const unsigned lane = threadIdx.x & 31u;
     const long long warps = static_cast<long long>(gridDim.x) * (kKvThreads / 32);

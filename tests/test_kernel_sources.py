@@ -1,0 +1,28 @@
+"""Rules that the kernels' sources keep and that no single run can show."""
+import os
+import re
+
+import pytest
+
+KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "src", "kernels")
+
+
+def _overlapped():
+    """The sources of kernels that are launched while the kernel in front of them runs, each with the headers it takes from here."""
+    found = {}
+    for name in sorted(os.listdir(KERNELS)):
+        text = open(os.path.join(KERNELS, name)).read()
+        if name.endswith(".cu") and "kernels/programmatic_launch.cuh" in text:
+            found[name] = [name] + [h for h in re.findall(r'#include "kernels/([^"]+)"', text) if os.path.exists(os.path.join(KERNELS, h))]
+    return found
+
+
+@pytest.mark.parametrize("kernel", sorted(_overlapped()))
+def test_overlapped_kernels_load_coherently(kernel):
+    """The read-only path is for data that stays as it is for as long as the kernel runs.  The kernel in front of an overlapped
+    launch may still write what it loads, and a read-only load is not tied to the wait for that kernel either."""
+    assert len(_overlapped()) >= 5
+    for name in _overlapped()[kernel]:
+        code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(KERNELS, name)).read(), flags=re.S)
+        assert not re.findall(r"__ldg\b|__restrict__|ld\.global(?:\.\w+)*\.nc\b", code), name
+        assert "waitForPreviousKernel" in code or not name.endswith(".cu")
