@@ -362,9 +362,11 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
     const bool fixed = placesAreFixed(p);
     const long long t_first = static_cast<long long>(p.T) * blockIdx.x / gridDim.x, t_end = static_cast<long long>(p.T) * (blockIdx.x + 1) / gridDim.x;
     // A group of one rank that sends in this launch has everybody's counts, its own, from the grid barrier, and sends every
-    // row itself: it waits for no flag and counts no rows as sent, and the last CTA out raises all flags.  (A launch that only
-    // receives waits for the flags like any other: the caller may have sent on another stream.)
+    // row itself, so it waits for no flag.  (A launch that only receives waits for the flags like any other: the caller may have
+    // sent on another stream.)  Unless a GEMM beside this launch takes the rows as they arrive (bit 2 of the phases), it also counts
+    // no rows as sent, and the last CTA out raises all flags.
     const bool own = p.R == 1 && (p.phases & 1);
+    const bool flags_last = own && !(p.phases & 4);
 
     if (p.phases & 1) {
         // 1. this CTA's copies per expert, and its place among the rank's
@@ -399,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             for (int e = tid; e < p.E; e += kThreads) dst[e] = totalOf(e);
             if (tid == 0) reinterpret_cast<int *>(peer + p.lay.off_grp_tokens)[p.rank] = p.topk_weights != nullptr ? p.T : 0;
             // Experts of that rank that get nothing from us are complete right away.
-            if (own) break; // the flags go up at the end
+            if (flags_last) break;
             uint64_t *dflag = reinterpret_cast<uint64_t *>(peer + p.lay.off_disp_flag);
             __syncthreads(); // the release below covers the whole CTA's stores
             if (tid == 0) stReleaseSys(reinterpret_cast<uint64_t *>(peer + p.lay.off_counts_flag) + p.rank, p.epoch);
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             else dispatchTokens<false>(p, rows, dests, peer_sh, tb, n, parts);
             __syncthreads(); // all stores of the batch issued (and its tables free for the next one)
             // Count the batch's rows as sent.  Whoever completes an expert's rows raises that expert's arrival flag at its rank.
-            for (int e = tid; e < p.E && !own; e += kThreads) {
+            for (int e = tid; e < p.E && !flags_last; e += kThreads) {
                 const int c = mine[e];
                 if (c == 0) continue;
                 // One operation releases this CTA's rows and acquires the other CTAs'.
@@ -563,7 +565,7 @@ __global__ void __launch_bounds__(kThreads, kDispatchCtas) epDispatchKernel(cons
             }
             if (tid == 0) reinterpret_cast<int *>(self + p.lay.off_grp_tokens)[0] = p.topk_weights != nullptr ? p.T : 0;
         }
-        if (last && own && (fixed || masked[0] == 0)) {
+        if (last && flags_last && (fixed || masked[0] == 0)) {
             // The flags go up behind all counts (of every warp) and, through the exit counter, all rows: a GEMM launched on
             // another stream may look at them while this kernel runs.  It runs on this GPU, the only one of the group, so the
             // release needs no wider scope.

@@ -140,7 +140,8 @@ def grouped_gemm_fp8(
     ``fused_with``: ``(buffer, handle)`` of the EP dispatch that is filling ``a`` (optional).
     ``overlapped``: that dispatch was launched on another stream and may still be running; the
     kernel then waits for the count exchange itself (``rows_per_expert`` names the layout) and
-    ``grid`` should leave the dispatch's CTAs free (see ``Buffer.dispatch_gemm``).
+    ``grid`` should leave the dispatch's CTAs free (see ``Buffer.dispatch_gemm``; in a group of one rank only that entry point's
+    dispatch announces rows as they arrive, the others announce them all at the end).
     ``tile_mode``: 0 lets the library choose, 1 forces tiles of 128 columns on single CTAs, 2 forces
     256 x 256 tiles on CTA pairs (``N % 256 == 0``).
     ``expected_rows``: about how many rows the groups have together, for that choice; 0: what the ``Buffer`` whose dispatch

@@ -283,3 +283,36 @@ def test_dispatch_beside_a_combine_of_the_same_buffer(mode):
         err = (got.double() - alone[step % 4].double()).norm() / alone[step % 4].double().norm()
         assert float(err) < 2.0**-8, (step, float(err))  # (rows may come in another order, and with it the sum's; half a bf16 step)
     b.destroy()
+
+
+@pytest.mark.parametrize("low_latency", [True, False])
+def test_rows_are_announced_while_the_dispatch_for_a_fused_gemm_runs(low_latency):
+    """``dispatch_gemm``'s GEMM takes an expert's rows as they arrive: counts and flags go up long before the last row is sent."""
+    T, H, E, K = 4096, 4096, 16, 8
+    dev = torch.device("cuda:0")
+    b = Buffer(0, 1, E, H, T, K, device=dev, low_latency_mode=low_latency, timeout_ms=1000)
+    b.connect_ranks()
+    x, _, _ = _routing(T, H, E, K, 1)
+    idx = torch.arange(K, 2 * K, device=dev).repeat(T, 1)
+    idx[:64] -= K  # experts 0 to 7 get the first tokens, 8 to 15 the others
+    looks, seen = torch.cuda.Stream(dev), torch.empty(E + 1, dtype=torch.int64).pin_memory()
+    for step in range(3):
+        parity = (b.epoch + 1) & 1
+        flags, counts_flag = b._region(parity, "off_disp_flag", E * 8).view(torch.int64), b._region(parity, "off_counts_flag", 8).view(torch.int64)
+        torch.cuda.synchronize()
+        _, _, h, _, _ = b._dispatch(x, idx, True, False, T if low_latency else 0, 5, False, grid=1)  # as dispatch_gemm launches it; one CTA: milliseconds
+        done = torch.cuda.Event()
+        done.record()
+        early = torch.zeros(E + 1, dtype=torch.bool)
+        while True:
+            with torch.cuda.stream(looks):
+                seen[:E].copy_(flags, non_blocking=True)
+                seen[E:].copy_(counts_flag, non_blocking=True)
+            looks.synchronize()
+            if done.query():
+                break
+            early |= seen == h.epoch
+        assert step == 0 or (bool(early[:K].all()) and bool(early[E])), early.tolist()  # (the first launch loads the kernel)
+        assert b.status == 0 and bool((flags == h.epoch).all()) and b._cnt.count_nonzero() == 0
+        assert torch.equal(h.recv_count, torch.bincount(idx.reshape(-1), minlength=E).int())
+    b.destroy()
