@@ -48,7 +48,7 @@ constexpr int BM = 128, BN = 128, BK = 128; // tile; BK is also the scale granul
 constexpr int kRingBytes = 200 * 1024;
 constexpr int kMaxStages = 5;
 constexpr int kPrefetchBoxes = 10;         // W boxes per CTA called into L2 ahead of the launch's turn: 45 MB
-constexpr int BMS = 64;                    // rows of a tile whose operands are swapped
+constexpr int kTurned = 64;                // most rows of a tile whose operands are swapped
 constexpr int kStageSteps = 2;             // 128-channel steps per stage (the last one of an odd K has one)
 constexpr int kThreads = 384;              // 4 role warps + 8 promotion warps
 constexpr int kTileBytes = BM * BK;         // 16 KiB (fp8)
@@ -134,7 +134,7 @@ __device__ __forceinline__ void issueStep(uint32_t tmem_d, uint64_t da, uint64_t
 // instruction of a step costs its issuing thread more than the rows it may save (32 experts, 32 rows each, 2048 x 7168: one
 // box of 32 92 us, two of 16 101 us).
 __device__ __forceinline__ int aBoxRows(int rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : BM; }
-template<bool kSwapped> __device__ __forceinline__ int rowTiles(int rows) { return kSwapped ? (rows + BMS - 1) / BMS : (rows + BM - 1) / BM; }
+__device__ __forceinline__ int rowTiles(int rows) { return (rows + BM - 1) / BM; }
 
 // Promotion and store of one tile whose operands are swapped (see groupedGemmKernel): this thread's TMEM lane is column
 // `lane` of the warp's 32 columns of D, the accumulator's columns are the rows of A, kCols of them this warp's.  A row's scale is loaded
@@ -205,22 +205,22 @@ template<bool kSwapped> __device__ __forceinline__ bool tileAt(const Shared &sh,
     }
     const int local = t - sh.tilePrefix[lo];
     out.g = lo;
-    const int m_tiles = kSwapped ? rowTiles<true>(sh.rowCount[lo]) : 0;
+    const int m_tiles = kSwapped ? rowTiles(sh.rowCount[lo]) : 0;
     out.nt = kSwapped ? local / m_tiles : local % n_tiles; // swapped: the row tiles of one W tile side by side
     out.mt = kSwapped ? local - out.nt * m_tiles : local / n_tiles;
     return true;
 }
 
-// kSwapped: W is the MMA's M side (128 rows of it), 32 or 64 rows of A are its N side and the accumulator is transposed; a tile has at
-// most 64 rows, and tiles that share W are neighbours.  With A on the M side every MMA and promotion works on 128 rows however few an
-// expert has, and under a steady load the power that takes lowers the clock.  This form also needs few enough registers (128,
-// the bound of 512 threads) to fit on an SM beside a CTA of the dispatch in front of it: it sets itself up, and calls its first W
-// boxes into L2, while that runs.  Bound by HBM (W is read once: 537 MB in 93 us, 5.8 TB/s, with 4 to 16 rows per expert) and, from 32
-// rows on, by the shared memory that TMA, the MMAs' operands and the scales share.
-// Measured on one B200, 32 experts, N = K = 4096, back to back for half a second, us, one-step stages with A on the M side / this form:
-// 4 rows each 120 / 93, 16 rows 122 / 97, 25 rows 123 / 104, 32 rows 124 / 110; 2048 x 7168, 32 rows 114 / 105.
+// kSwapped: in a tile of at most 64 rows W is the MMA's M side (128 rows of it), 32 or 64 rows of A are its N side and the accumulator
+// is transposed; tiles that share W are neighbours.  With A on the M side every MMA and promotion works on 128 rows however few an
+// expert has, and under a steady load the power that takes lowers the clock.  Bound by HBM (W is read once: 537 MB in 90 us, 6.0 TB/s,
+// with 4 rows per expert) and, from 32 rows on, by the shared memory that TMA, the MMAs' operands and the scales share.  Tiles of more
+// rows keep A on the M side: on the N side they take two tiles, and the same W twice (32 experts of 72 rows 219 us, as now 133), or
+// 64 columns per promotion warp with their scales in shared memory (180).
+// Measured on one B200, 32 experts, N = K = 4096, back to back, us, A on the M side everywhere / this form: 4 rows each 112 / 90, 16 rows
+// 117 / 95, 32 rows 119 / 103, 64 rows 125 / 120, 128 rows 136 / 139; every other expert 70 rows and none between 72 / 73.
 template<bool kSwapped>
-__global__ void __launch_bounds__(kSwapped ? 512 : kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA32, const __grid_constant__ CUtensorMap mapA64,
                   const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p, int prefetch_boxes) {
     extern __shared__ __align__(1024) unsigned char dyn[];
@@ -281,15 +281,15 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             sh.rowCount[g] = c;
             most = max(most, c);
             next += c;
-            run += rowTiles<kSwapped>(c) * n_tiles;
+            run += rowTiles(c) * n_tiles;
         }
         sh.tilePrefix[p.groups] = run;
-        sh.aRows = aBoxRows(kSwapped ? min(most, BMS) : most);
+        sh.aRows = aBoxRows(most);
     }
     if (warp == 1 && !p.counts_flag) {
         int most;
-        nixl_gemm::buildTileTable(p, n_tiles, [](int rows) { return rowTiles<kSwapped>(rows); }, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
-        if (lane == 0) sh.aRows = aBoxRows(kSwapped ? min(most, BMS) : most);
+        nixl_gemm::buildTileTable(p, n_tiles, rowTiles, sh.tilePrefix, sh.rowStart, sh.rowCount, most);
+        if (lane == 0) sh.aRows = aBoxRows(most);
     }
     tcFenceBefore();
     __syncthreads();
@@ -311,13 +311,12 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         uint32_t s = 0, empty_par = 1; // ring position
         Tile t;
         for (int ti = blockIdx.x; tileAt<kSwapped>(sh, p.groups, n_tiles, ti, t); ti += gridDim.x) {
-            constexpr int rows = kSwapped ? BMS : BM; // of a tile
-            const int row0 = sh.rowStart[t.g] + t.mt * rows;
+            const int row0 = sh.rowStart[t.g] + t.mt * BM;
             if (p.disp_flag) {
-                waitArrivals(p, t.g, t.mt * rows, min(t.mt * rows + rows, sh.rowCount[t.g]));
+                waitArrivals(p, t.g, t.mt * BM, min(t.mt * BM + BM, sh.rowCount[t.g]));
                 asm volatile("fence.proxy.async;" ::: "memory"); // peers' generic-proxy stores before our async-proxy reads
             }
-            const int box = aBoxRows(min(sh.rowCount[t.g] - t.mt * rows, rows));
+            const int box = aBoxRows(sh.rowCount[t.g] - t.mt * BM);
             const CUtensorMap *map = box == 32 ? &mapA32 : box == 64 ? &mapA64 : &mapA;
             for (int ks = 0; ks < k_steps; ks += kStageSteps) {
                 const bool two = ks + 1 < k_steps;
@@ -349,10 +348,13 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         const uint64_t desc0 = smemDesc(smemU32(tiles));
         for (int tile = 0; tile < my_tiles; ++tile) {
             uint32_t idesc = instrDesc(BN);
+            bool turned = false;
             if constexpr (kSwapped) {
                 Tile t;
                 tileAt<true>(sh, p.groups, n_tiles, static_cast<int>(blockIdx.x) + tile * static_cast<int>(gridDim.x), t);
-                idesc = instrDesc(aBoxRows(min(sh.rowCount[t.g] - t.mt * BMS, BMS)));
+                const int rows = sh.rowCount[t.g] - t.mt * BM;
+                turned = rows <= kTurned;
+                if (turned) idesc = instrDesc(aBoxRows(rows));
             }
             for (int ks = 0; ks < k_steps; ks += kStageSteps) {
                 if (!ready && !mbarWait(&sh.full[s], full_par, abort_flag)) goto mma_done;
@@ -366,12 +368,12 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
                 uint64_t dw = desc0 + static_cast<uint64_t>((s * stage_bytes) >> 4);
                 uint64_t da = dw + static_cast<uint64_t>((kStageSteps * kTileBytes) >> 4);
                 if (ks + 1 < k_steps) {
-                    issueFirstStep(tmem + buf * BN, kSwapped ? dw : da, kSwapped ? da : dw, idesc, tfull_bar0 + buf * 8u);
+                    issueFirstStep(tmem + buf * BN, turned ? dw : da, turned ? da : dw, idesc, tfull_bar0 + buf * 8u);
                     buf = (buf + 1) & (kAccBufs - 1);
                     dw += kTileBytes >> 4;
                     da += a_bytes >> 4;
                 }
-                issueStep(tmem + buf * BN, kSwapped ? dw : da, kSwapped ? da : dw, idesc, tfull_bar0 + buf * 8u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
+                issueStep(tmem + buf * BN, turned ? dw : da, turned ? da : dw, idesc, tfull_bar0 + buf * 8u, empty_bar0 + s * 8u, full_bar0 + ns * 8u, nfull_par, ready);
                 buf = (buf + 1) & (kAccBufs - 1);
                 s = ns;
                 full_par = nfull_par;
@@ -415,8 +417,10 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
         Tile t;
         const float *scale_a = p.scale_a;
         for (int ti = blockIdx.x; tileAt<kSwapped>(sh, p.groups, n_tiles, ti, t); ti += gridDim.x) {
-            const int cols = aBoxRows(min(sh.rowCount[t.g] - t.mt * BMS, BMS)) / 2; // rows of A that a warp promotes when the operands are swapped
-            const int first = kSwapped ? t.mt * BMS + half * cols : t.mt * BM + q * 32;
+            const int tile_rows = sh.rowCount[t.g] - t.mt * BM;
+            const bool turned = kSwapped && tile_rows <= kTurned;
+            const int cols = aBoxRows(tile_rows) / 2; // rows of A that a warp promotes when the operands are swapped
+            const int first = t.mt * BM + (turned ? half * cols : q * 32);
             if (first >= sh.rowCount[t.g]) { // this warp's rows are padding: it only hands accumulators back
                 bool alive = true;
                 for (int ks = 0; ks < k_steps && alive; ++ks, ++it) {
@@ -428,7 +432,7 @@ groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constan
             }
             const bool fresh = p.disp_flag != nullptr; // the scales travel with the rows
             if (fresh) waitArrivals(p, t.g, first, min(first + 32, sh.rowCount[t.g]));
-            if constexpr (kSwapped) {
+            if (turned) {
                 const int row = first + lane % cols; // whose scales this lane holds
                 const float *sa_row = scale_a + (static_cast<long long>(sh.rowStart[t.g]) + row) * k_steps;
                 const float *sw = p.scale_w + (static_cast<long long>(t.g) * n_tiles + t.nt) * k_steps;
@@ -570,8 +574,9 @@ extern "C" int nixl_grouped_gemm_fp8_mode(const NixlGroupedGemmParams *params) {
     return p.rows_per_expert == 0 && !p.counts_flag && p.N % 256 == 0 && rows > 128LL * p.groups && rows * p.N >= 40LL * 256 * 256 ? 2 : 1;
 }
 
-// Single CTAs with swapped operands (see groupedGemmKernel) up to 40 expected rows per expert: us, A on the M side / W there, for 32
-// experts, N = K = 4096: 32 rows each 122 / 110, 48 rows 126 / 129, 64 rows 129 / 166 (more than 64 rows are two tiles).
+// Single CTAs with swapped operands (see groupedGemmKernel) up to 40 expected rows per expert: us, A on the M side everywhere / swapped,
+// for 32 experts, N = K = 4096: 32 rows each 119 / 103, 48 rows 124 / 118, 64 rows 125 / 120, 72 rows 130 / 133.  Between 40 and 64 rows
+// uneven routing puts more and more experts above 64, where this form gains nothing.
 static bool swappedTiles(const NixlGroupedGemmParams &p) { return expectedRows(p) <= 40LL * p.groups; }
 
 extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params, void *stream) {
@@ -624,7 +629,7 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int grid = p.grid > 0 ? p.grid : sms;
     // Upper bound of tiles (row counts live on the device): never launch more CTAs than that.
-    const long long max_tiles = (static_cast<long long>(p.a_rows) / (swapped ? BMS : BM) + p.groups) * (p.N / BN);
+    const long long max_tiles = (static_cast<long long>(p.a_rows + BM - 1) / BM + p.groups) * (p.N / BN);
     if (grid > max_tiles) grid = static_cast<int>(max_tiles);
     if (p.counts_flag || p.disp_flag) { // waits for a dispatch on another stream: not before the stream's own turn
         kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mapA, mapA32, mapA64, mapW, p, 0);
