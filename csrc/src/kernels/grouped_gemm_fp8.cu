@@ -139,11 +139,13 @@ __device__ __forceinline__ int rowTiles(int rows) { return (rows + BM - 1) / BM;
 // Promotion and store of one tile whose operands are swapped (see groupedGemmKernel): this thread's TMEM lane is column
 // `lane` of the warp's 32 columns of D, the accumulator's columns are the rows of A, kCols of them this warp's.  A row's scale is loaded
 // by the lane of its number and read by all from the warp's own two rows of shared memory, four at a time (shuffles, one per row and
-// step, took as long as HBM took for W).  False when another role gave up.
+// step, took as long as HBM took for W).  Steps take the two rows in turn; a tile's first step may take the one that the last step of
+// the tile before was read from (an odd number of steps), so the warp meets in between.  False when another role gave up.
 template<int kCols>
 __device__ __forceinline__ bool promoteSwapped(Shared &sh, const float *sa_row, bool valid, bool fresh, const float *sw, int k_steps, uint32_t lane_base, int lane, uint32_t &it,
                                                float (*scales)[32], __nv_bfloat16 *out, long long row_stride, int rows_left) {
     volatile int *abort_flag = &sh.abort;
+    __syncwarp();
     uint64_t acc[kCols / 2]; // fp32 pairs
 #pragma unroll
     for (int i = 0; i < kCols / 2; ++i) acc[i] = 0;
@@ -162,7 +164,7 @@ __device__ __forceinline__ bool promoteSwapped(Shared &sh, const float *sa_row, 
             if (ks >= k_steps) break;
             const int buf = it % kAccBufs;
             const float s = s4[j];
-            scales[j & 1][lane] = s; // (a row that this step's predecessor may still be read from is the other one)
+            scales[j & 1][lane] = s; // (the step before may still be read: from the other row)
             __syncwarp();
             if (!mbarWait(&sh.tmemFull[buf], (it / kAccBufs) & 1, abort_flag)) return false;
             tcFenceAfter();

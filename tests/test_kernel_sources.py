@@ -26,3 +26,16 @@ def test_overlapped_kernels_load_coherently(kernel):
         code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(KERNELS, name)).read(), flags=re.S)
         assert not re.findall(r"__ldg\b|__restrict__|ld\.global(?:\.\w+)*\.nc\b", code), name
         assert "waitForPreviousKernel" in code or not name.endswith(".cu")
+
+
+def test_scale_rows_change_hands_between_tiles():
+    """A promotion warp with swapped operands shares its scales through two rows of shared memory, step by step in turn.  With an odd
+    number of steps a tile begins with the row that the tile before ended with: the warp has to meet before that is written."""
+    code = re.sub(r"//[^\n]*", "", open(os.path.join(KERNELS, "grouped_gemm_fp8.cu")).read())
+    body = code[code.index("bool promoteSwapped(") :]
+    body = body[: body.index("\n}\n")]
+    row = re.search(r"scales\[(.*?)\]\[lane\] =", body).group(1)
+    used = [eval(row, {"j": step % 4}) for tile in range(2) for step in range(3)]
+    again = [i for i in range(1, len(used)) if used[i] == used[i - 1]]
+    assert again == [3]  # the second tile's first step, and no other
+    assert "__syncwarp()" in body[: body.index("for (int ks0")]
