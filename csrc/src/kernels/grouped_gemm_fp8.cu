@@ -47,7 +47,6 @@ using namespace nixl_tc;
 constexpr int BM = 128, BN = 128, BK = 128; // tile; BK is also the scale granularity
 constexpr int kRingBytes = 200 * 1024;
 constexpr int kMaxStages = 5;
-constexpr int kPrefetchBoxes = 10;         // W boxes per CTA called into L2 ahead of the launch's turn: 45 MB
 constexpr int kTurned = 64;                // most rows of a tile whose operands are swapped
 constexpr int kStageSteps = 2;             // 128-channel steps per stage (the last one of an odd K has one)
 constexpr int kThreads = 384;              // 4 role warps + 8 promotion warps
@@ -224,21 +223,13 @@ template<bool kSwapped> __device__ __forceinline__ bool tileAt(const Shared &sh,
 template<bool kSwapped>
 __global__ void __launch_bounds__(kThreads, 1)
 groupedGemmKernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapA32, const __grid_constant__ CUtensorMap mapA64,
-                  const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p, int prefetch_boxes) {
+                  const __grid_constant__ CUtensorMap mapW, const NixlGroupedGemmParams p) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     unsigned char *tiles = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(dyn) + 1023) & ~uintptr_t(1023));
     Shared &sh = *reinterpret_cast<Shared *>(tiles + kRingBytes + (kSwapped ? 0 : kTailBytes));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_tiles = p.N / BN, k_steps = p.K / BK;
 
-    // The W boxes of this CTA's first tile, if each expert has one row tile, on their way to L2 before the rows are there.  (A hint
-    // only: W itself is read behind the wait, as the kernel in front may have written it.)
-    if (threadIdx.x == 32 && static_cast<long long>(blockIdx.x) * BN < static_cast<long long>(p.groups) * p.N) {
-        for (int i = 0; i < prefetch_boxes; ++i)
-            if (i * kStageSteps < k_steps)
-                asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(&mapW), "r"(0), "r"(static_cast<int>(blockIdx.x) * BN), "r"(i * kStageSteps)
-                             : "memory");
-    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMaxStages; ++s) {
             mbarInit(&sh.full[s], 2); // producer (with the byte count) + slot watcher
@@ -634,9 +625,8 @@ extern "C" int nixl_grouped_gemm_fp8_launch(const NixlGroupedGemmParams *params,
     const long long max_tiles = (static_cast<long long>(p.a_rows + BM - 1) / BM + p.groups) * (p.N / BN);
     if (grid > max_tiles) grid = static_cast<int>(max_tiles);
     if (p.counts_flag || p.disp_flag) { // waits for a dispatch on another stream: not before the stream's own turn
-        kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mapA, mapA32, mapA64, mapW, p, 0);
+        kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(mapA, mapA32, mapA64, mapW, p);
         return cudaGetLastError();
     }
-    const int prefetch_boxes = expectedRows(p) >= 2LL * p.groups ? kPrefetchBoxes : 0; // (with fewer rows some experts have none)
-    return nixl_pdl::launch(kernel, grid, kThreads, smem, static_cast<cudaStream_t>(stream), mapA, mapA32, mapA64, mapW, p, prefetch_boxes);
+    return nixl_pdl::launch(kernel, grid, kThreads, smem, static_cast<cudaStream_t>(stream), mapA, mapA32, mapA64, mapW, p);
 }

@@ -71,7 +71,7 @@ def test_receive_that_waits_leaves_the_sms_to_other_streams(rows_each):
     b.destroy()
 
 
-# Few rows per expert (W on the MMA's M side, its first boxes called into L2 before the wait), more, CTA pairs, block-scaled.
+# Few rows per expert (W on the MMA's M side), more, CTA pairs, block-scaled.
 @pytest.mark.parametrize("tokens,low_latency,kind", [(24, True, "fp8"), (128, True, "fp8"), (700, False, "fp8"), (24, False, "mx"), (700, False, "mx")])
 def test_dispatch_gemm_combine_without_a_pause(tokens, low_latency, kind):
     """Inputs, routing and the experts' weights are other ones in every step, each written by the kernel in front of the one that

@@ -39,3 +39,14 @@ def test_scale_rows_change_hands_between_tiles():
     again = [i for i in range(1, len(used)) if used[i] == used[i - 1]]
     assert again == [3]  # the second tile's first step, and no other
     assert "__syncwarp()" in body[: body.index("for (int ks0")]
+
+
+@pytest.mark.parametrize("kernel", sorted(_overlapped()))
+def test_overlapped_kernels_fetch_nothing_by_guess(kernel):
+    """In front of the wait for the previous kernel nobody knows what will be read (the routing is what that kernel writes): expert
+    weights that were called into L2 there by their place were read in vain wherever the first experts had no rows."""
+    code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(KERNELS, kernel)).read(), flags=re.S)
+    for begin in re.finditer(r"__global__", code):
+        body = code[begin.start() :].split("__global__", 2)[1]
+        ahead, wait, _ = body.partition("waitForPreviousKernel()")
+        assert not wait or "prefetch" not in ahead
