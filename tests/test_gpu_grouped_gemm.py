@@ -98,6 +98,25 @@ def test_hot_experts_cost_no_second_pass_over_their_weights():
     assert few < 1.25 * many, (few, many)
 
 
+@pytest.mark.parametrize("rows_each", [2, 20, 40, 41])  # expected; the line between the two forms lies behind 40
+@pytest.mark.parametrize("K", [128, 640, 1024])
+def test_only_the_experts_rows_are_written(rows_each, K):
+    """Tiles are padded to 32, 64 or 128 rows; what lies between two experts' rows stays as it is, also before the first."""
+    counts = [1, 31, 33, 63, 0, 65, 17, 128, 129]
+    a, sa, wq, sw, rs, rc = _case(len(counts), 256, K, counts, gap=130)
+    raw = a.view(torch.uint8)
+    a, sa = torch.cat([raw[-130:], raw]).view(a.dtype), torch.cat([sa[-130:], sa])
+    rs = rs + 130
+    out = torch.full((a.shape[0], 256), -7.0, device=a.device, dtype=torch.bfloat16)
+    grouped_gemm_fp8(a, sa, wq, sw, rs, rc, out=out, tile_mode=1, expected_rows=rows_each * len(counts))
+    written = torch.zeros(a.shape[0], dtype=torch.bool, device=a.device)
+    for s, c in zip(rs.tolist(), counts):
+        written[s : s + c] = True
+    assert bool((out[~written] == -7.0).all())
+    many = grouped_gemm_fp8(a, sa, wq, sw, rs, rc, tile_mode=1, expected_rows=10**6)
+    assert torch.equal(out[written], many[written])  # the same products in the same order, whatever the form
+
+
 def _check(G, N, K, counts, gap, tile_mode, grid=0, expected_rows=0):
     a, sa, wq, sw, rs, rc = _case(G, N, K, counts, gap)
     out = grouped_gemm_fp8(a, sa, wq, sw, rs, rc, tile_mode=tile_mode, grid=grid, expected_rows=expected_rows)
