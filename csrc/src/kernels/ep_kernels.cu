@@ -1388,6 +1388,8 @@ extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *s
         const int grid = static_cast<int>(want < ctas ? want : ctas);
         const auto kernel = p.K <= 8 ? (p.use_logfmt ? epCombineLocal<8, true> : epCombineLocal<8, false>)
                                      : (p.use_logfmt ? epCombineLocal<kMaxTopk, true> : epCombineLocal<kMaxTopk, false>);
+        static std::atomic<bool> l1_done[4][64];
+        if (const cudaError_t e = nixl_pdl::preferL1(reinterpret_cast<const void *>(kernel), l1_done[(p.K <= 8) * 2 + (p.use_logfmt != 0)]); e != cudaSuccess) return e;
         return nixl_pdl::launch(kernel, grid, kThreads, 0, static_cast<cudaStream_t>(stream), p, parts);
     }
     if (p.pull == 2) {

@@ -217,3 +217,41 @@ def test_gemms_in_a_graph(rows_each):
         torch.cuda.synchronize()
         assert int(status) == 0 and all(torch.equal(got, ref) for got, ref in zip(outs, want[i]))
     assert not torch.equal(want[0][0], want[0][1])
+
+
+def test_an_sm_that_a_gemm_has_left_is_split_anew():
+    """A GEMM's ring leaves an SM next to no L1.  A kernel that moves in behind it needs L1 for its loads in flight: overlapping the
+    GEMM's end must not cost it more than a launch of its own.  (It cost 6 us more where the SMs stayed as the GEMM had them, and
+    takes 2 us less where they do not; the line lies at half of that cost.)"""
+    T, H, E, K, depth = 4096, 4096, 32, 8, 512
+    dev = torch.device("cuda:0")
+    b = Buffer(0, 1, E, H, T, K, device=dev, low_latency_mode=False, timeout_ms=1000)
+    b.connect_ranks()
+    x, idx, w = _routing(T, H, E, K, 1)
+    recv, scales, h = b.dispatch(x, idx, use_ue8m0=True, topk_weights=w)
+    a, sa = recv[:, :depth].contiguous(), scales.view(torch.int32)[:, : depth // 512].contiguous()
+    wq, sw = quantize_weights_ue8m0(torch.randn(E, H, depth, device=dev) * 0.05)
+    y, out, pad = b.get_next_combine_buffer(h).view(-1, H), torch.empty_like(x), torch.zeros(1, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+
+    def step(apart):
+        grouped_gemm_mxfp8(a, sa, wq, sw, h.expert_offsets, h.recv_count, out=y, status=status)
+        if apart:
+            pad.zero_()  # a kernel that neither lets another in nor moves in early
+        b.combine(y, idx, w, h, out=out)
+
+    times = {False: [], True: []}
+    for i in range(42):
+        for apart in times:
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(200000)  # all launches are queued when the first one starts
+            begin.record()
+            step(apart)
+            end.record()
+            end.synchronize()
+            if i > 1:
+                times[apart].append(begin.elapsed_time(end) * 1e3)
+    chained, separate = (sorted(times[apart])[20] for apart in (False, True))
+    assert b.status == 0 and int(status) == 0
+    assert chained < separate + 3, (chained, separate)
+    b.destroy()

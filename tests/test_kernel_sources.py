@@ -50,3 +50,11 @@ def test_overlapped_kernels_fetch_nothing_by_guess(kernel):
         body = code[begin.start() :].split("__global__", 2)[1]
         ahead, wait, _ = body.partition("waitForPreviousKernel()")
         assert not wait or "prefetch" not in ahead
+
+
+@pytest.mark.parametrize("kernel", sorted(_overlapped()))
+def test_overlapped_kernels_without_shared_memory_ask_for_l1(kernel):
+    """An SM that a GEMM has just left has hardly any L1 unless the kernel that moves in asks for it."""
+    code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(KERNELS, kernel)).read(), flags=re.S)
+    for begin in re.finditer(r"nixl_pdl::launch\(kernel, [^;]*?, 0, ", code):
+        assert "nixl_pdl::preferL1(" in code[code.rindex("const auto kernel", 0, begin.start()) : begin.start()]
