@@ -216,10 +216,11 @@ __device__ __forceinline__ uint4 quantGroup(const uint4 &lo, const uint4 &hi, bo
 // Measured on one B200, one rank, 32 experts, top-8, before / now: 4096 tokens x 7168 bf16 131 / 113 us (528 MB, 4.7 TB/s; the
 // rows written, 470 MB, are the bound), fp8 97 / 73 us, 4096 x 4096 fp8 74 / 47 us (3.6 TB/s); 128 tokens x 7168 fp8, low-latency
 // layout 21.6 / 13.4 us (8.4 with fixed places); 1 token 20.5 / 11.9 us (7.8).
-// A group of one rank then dropped what only other ranks need (flags early, rows counted as sent), and every group reads the
-// routing once, arrives at the grid barrier with one operation and calls its rows into L2 while it counts.  Compact layout, 32
-// experts, top-8, us before / after: 1 token 17.9 / 11.0, 300 x 4096 bf16 18.1 / 15.5, 700 29.5 / 19.8, 1500 40.3 / 32.0; 4096 x 4096
-// with power-of-two scales 47.2 / 39.8, 4096 x 7168 bf16 116 / 114 (bound by the writes to some 4700 rows that are open at a time).
+// A group of one rank then dropped what only others need (flags early, rows counted as sent), except in the launch that a GEMM
+// beside it follows row by row; every group reads the routing once, arrives at the grid barrier with one operation and calls its
+// rows into L2 while it counts.  Compact layout, 32 experts, top-8, us before / after: 1 token 17.9 / 11.0, 300 x 4096 bf16 18.1 /
+// 15.5, 700 29.5 / 19.8, 1500 40.3 / 32.0; 4096 x 4096 with power-of-two scales 47.2 / 39.8, 4096 x 7168 bf16 116 / 114 (bound by
+// the writes to some 4700 rows that are open at a time).
 constexpr int kBatch = 32;  // tokens whose rows are looked up together, and reported as sent together
 constexpr int kSlices = 2;  // slices of a token in flight per warp: 2 KiB
 constexpr int kDispatchCtas = 4; // per SM, with many tokens
@@ -1389,7 +1390,7 @@ extern "C" int nixl_ep_combine_launch(const NixlEpCombineParams *params, void *s
         const auto kernel = p.K <= 8 ? (p.use_logfmt ? epCombineLocal<8, true> : epCombineLocal<8, false>)
                                      : (p.use_logfmt ? epCombineLocal<kMaxTopk, true> : epCombineLocal<kMaxTopk, false>);
         static std::atomic<bool> l1_done[4][64];
-        if (const cudaError_t e = nixl_pdl::preferL1(reinterpret_cast<const void *>(kernel), l1_done[(p.K <= 8) * 2 + (p.use_logfmt != 0)]); e != cudaSuccess) return e;
+        if (const cudaError_t e = nixl_pdl::preferL1(reinterpret_cast<const void *>(kernel), dev, l1_done[(p.K <= 8) * 2 + (p.use_logfmt != 0)]); e != cudaSuccess) return e;
         return nixl_pdl::launch(kernel, grid, kThreads, 0, static_cast<cudaStream_t>(stream), p, parts);
     }
     if (p.pull == 2) {

@@ -10,9 +10,12 @@
 // all of TMEM) are in flight.  (Eight N = 128 instructions, one per slot, read A from shared memory twice and
 // were slower by an eighth.)  A tile with at most 128 rows left runs as M = 128 (tailTile).
 //
-// What bounds this kernel is not the tensor pipe (four MMAs take 512 cycles, a step about 940) but promotion and the
-// hand-offs around it, since only two steps fit in TMEM; power comes second (the SM clock falls from 1.7 to 1.45 GHz under
-// load, and the block-scaled kernel takes 277 us under the same cap where this one takes 349):
+// What bounds this kernel is not the tensor pipe: four MMAs take 512 cycles, a step some 1100 (37 experts of 512 rows each, 2048 x
+// 7168: 592 whole tiles, eight per pair; 350 us at 1.44 GHz under the power cap, tile ends counted in).  The promotion's own
+// instructions are less than the MMAs' cycles too (128 two-wide FMAs per scheduler and step, and the TMEM reads), so what is not
+// reached is their overlap: only two steps fit in TMEM and a slot is handed back late.  Uneven experts come on top: 16384 rows of 32
+// experts take 305 us when all have 512 and 364 when they vary by an eighth.  Power is a bound beside these, not in front of them: the
+// block-scaled kernel takes 246 and 281 us for the same products under the same cap.  What was done about the hand-offs:
 //  * the issuing thread polls one barrier per step.  full[s] collects the producer's arrival (with
 //    both CTAs' byte count) and one arrival from each of the pair's sixteen promotion warps, sent
 //    when the warp has read the two slots the step will overwrite;

@@ -33,7 +33,10 @@
 //
 // Bound by power: the SM clock is 1.55 GHz at the first launch and 1.25 to 1.4 GHz after half a second; a full step takes
 // 697 cycles of which the MMAs need 512.  What is left is mostly the traffic into shared memory (64 of 128 bytes per cycle
-// at full rate, beside the operands' reads).  Measured on one B200 back to back for half a second, before (tokens on the
+// at full rate, beside the operands' reads).  The cap by itself would allow more: a library's plain fp8 product (8192 cubed, no block
+// scales, the same random inputs) settles at 2.65 PFLOP/s and 1.34 GHz (3.08 as a burst), this kernel, with experts of whole
+// tiles, at 1.97 (2048 x 7168) to 2.10 (4096 x 4096) and 1.06 to 1.24 GHz (2.36 to 2.43): it spends more energy per operation,
+// where is not known.  Measured on one B200 back to back for half a second, before (tokens on the
 // M side, eight N = 128 MMAs per step, scale copies every 512 channels) / now: 31 experts that share 16384 rows unevenly,
 // 2048 x 7168: 335 / 277 us (1.74 PFLOP/s); 32 experts, 32768 rows, 4096 x 4096: 659 / 562 us (1.96 PFLOP/s); one
 // expert, 8192 rows, 4096 x 7168: 239 / 200 us (2.41 PFLOP/s); 32 experts, 1024 rows, 2048 x 7168: 130 / 97 us.

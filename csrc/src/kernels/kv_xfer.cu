@@ -27,7 +27,7 @@ extern "C" int nixl_kv_xfer_launch(const NixlKvXferParams *params, void *stream)
     const auto kernel = p.cast_fp8 ? (k.vec_bytes == 32 ? kvXferKernel<true, 32> : kvXferKernel<true, 16>)
                                    : (k.vec_bytes == 32 ? kvXferKernel<false, 32> : kvXferKernel<false, 16>);
     static std::atomic<bool> l1_done[4][64];
-    if (const cudaError_t e = nixl_pdl::preferL1(reinterpret_cast<const void *>(kernel), l1_done[(p.cast_fp8 != 0) * 2 + (k.vec_bytes == 32)]); e != cudaSuccess) return e;
+    if (const cudaError_t e = nixl_pdl::preferL1(reinterpret_cast<const void *>(kernel), dev, l1_done[(p.cast_fp8 != 0) * 2 + (k.vec_bytes == 32)]); e != cudaSuccess) return e;
     // Requests posted one behind another: the next one's CTAs move in as this one's leave.
     return static_cast<int>(nixl_pdl::launch(kernel, grid, nixl_kv::kKvThreads, 0, s, k));
 }

@@ -14,7 +14,8 @@
 //     slots up while the loads of this one are in flight.
 //   - Rows that are contiguous on both sides are merged on the host, and indexes divide by multiplication.
 // Measured on one B200 (bytes read + written, before / now): 64 tensors x 256 blocks of 8 KiB, bf16, 268 MB: 54.2 / 51.6 us
-// (5.2 TB/s); 48 tensors x 61 blocks of 16 KiB, fp8 cast and token-major to head-major, 72 MB: 22.4 / 18.9 us (3.8 TB/s).
+// (5.2 TB/s); 48 tensors x 61 blocks of 16 KiB, fp8 cast and token-major to head-major, 72 MB: 22.4 / 18.9 us (3.8 TB/s), with the one
+// in front overlapped; each kilobyte read is then stored as eight pieces of 64 bytes, as blocks are walked in the source's order.
 #ifndef NIXL_B200_KV_XFER_BODY_CUH
 #define NIXL_B200_KV_XFER_BODY_CUH
 

@@ -42,14 +42,12 @@ cudaError_t launch(void (*kernel)(Params...), unsigned grid, unsigned threads, s
 }
 
 // For an overlapped kernel that has loads in flight rather than shared memory: asks for the whole of an SM's L1, once per device
-// (`done` belongs to the kernel).  Without it the kernel's CTAs take an SM over as the kernel in front has split it, and behind a
+// (`dev` is the current one, `done` belongs to the kernel).  Without it the kernel's CTAs take an SM over as the kernel in front has split it, and behind a
 // GEMM, whose ring leaves some 28 KB to L1, that bounds the bytes in flight: combine of 4096 tokens x 4096 behind its expert GEMM,
 // whole step 562 -> 550 us (2048 channels 218 -> 212, 1024 channels 116 -> 112); with all of it asked for as shared memory and no
-// overlap 562 as well.
-inline cudaError_t preferL1(const void *kernel, std::atomic<bool> (&done)[64]) {
-    int dev = 0;
-    if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
-    if (dev >= 64 || done[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+// overlap 562 as well.  Asking for 8, 14, 17 or 25 percent of shared memory instead gives the same times.
+inline cudaError_t preferL1(const void *kernel, int dev, std::atomic<bool> (&done)[64]) {
+    if (dev < 0 || dev >= 64 || done[dev].load(std::memory_order_relaxed)) return cudaSuccess;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
     if (e == cudaSuccess) done[dev].store(true, std::memory_order_relaxed);
     return e;
