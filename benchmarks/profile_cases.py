@@ -4,7 +4,7 @@
 Inputs are larger than L2 (126 MB) where DRAM figures matter, hold at most a few GB and launch
 the kernel of interest a handful of times.  One GPU only.
 
-    python benchmarks/profile_cases.py copy|kv|ep|ep_push|ep_rr|gemm|gemm_pair|gemm_mx
+    python benchmarks/profile_cases.py copy|kv|ep|ep_push|ep_rr|gemm|gemm_pair|gemm_mx|gemm_few|gemm_mx_few
 """
 import os
 import sys
@@ -131,6 +131,41 @@ def case_gemm_mx():
     assert int(out._nixl_status.item()) == 0
 
 
+def _few_rows(rows_per, pow2):
+    """A decode step's product: 16 experts whose weights (235 MB) are what is read."""
+    from nixl_b200.ops import quantize_weights, quantize_weights_ue8m0
+
+    G, N, K = 16, 2048, 7168
+    quantize = quantize_weights_ue8m0 if pow2 else quantize_weights
+    parts = [quantize(torch.randn(1, N, K, device="cuda:0") * 0.02) for _ in range(G)]
+    wq = torch.cat([q.view(torch.uint8) for q, _ in parts]).view(torch.float8_e4m3fn)
+    return (*_gemm_inputs(G, N, K, rows_per, pow2), wq, torch.cat([s for _, s in parts]))
+
+
+def case_gemm_few():
+    """Eight rows per expert, swapped operands on single CTAs (groupedGemmKernel<true>)."""
+    from nixl_b200.ops import grouped_gemm_fp8
+
+    a, sa, rs, rc, wq, sw = _few_rows(8, False)
+    for _ in range(3):
+        out = grouped_gemm_fp8(a, sa, wq, sw, rs, rc)
+    torch.cuda.synchronize()
+    assert int(out._nixl_status.item()) == 0
+
+
+def case_gemm_mx_few():
+    """32 rows per expert, stages of two steps on CTA pairs (groupedGemmMxPairKernel)."""
+    from nixl_b200.ops import grouped_gemm_mxfp8, to_ue8m0
+
+    a, sa, rs, rc, wq, sw = _few_rows(32, True)
+    sab = to_ue8m0(sa)
+    for _ in range(3):
+        out = grouped_gemm_mxfp8(a, sab, wq, sw, rs, rc)
+    torch.cuda.synchronize()
+    assert int(out._nixl_status.item()) == 0
+
+
 if __name__ == "__main__":
-    {"copy": case_copy, "kv": case_kv, "ep": case_ep, "ep_push": case_ep_push, "ep_rr": case_ep_rr, "gemm": case_gemm, "gemm_pair": case_gemm_pair, "gemm_mx": case_gemm_mx}[sys.argv[1]]()
+    {"copy": case_copy, "kv": case_kv, "ep": case_ep, "ep_push": case_ep_push, "ep_rr": case_ep_rr, "gemm": case_gemm, "gemm_pair": case_gemm_pair, "gemm_mx": case_gemm_mx,
+     "gemm_few": case_gemm_few, "gemm_mx_few": case_gemm_mx_few}[sys.argv[1]]()
     print("ok", sys.argv[1])
